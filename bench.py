@@ -45,8 +45,8 @@ sys.path.insert(0, str(ROOT))
 PKG = "cudaraster-linux_gb300"
 
 # The library's kernels in one blocking draw of the soup: the draw-block write,
-# setup, bin count / scan / scatter, coarse count / scan / scatter and fine.
-KERNELS_PER_DRAW = 9
+# setup, pairs and items (bin stage), list scan and scatter (coarse stage), fine.
+KERNELS_PER_DRAW = 7
 METRIC = "frames/s & Mtri/s on 1 GB300: batched+predicted vs plain, bit-exact framebuffers"
 WORKLOAD = {"workload": "plain path at scale: 1M-triangle random soup, 1920x1080, 1 spp, Gouraud, depth LESS, opaque",
             "num_tris": 1_000_000, "width": 1920, "height": 1080, "samples": 1, "pipe": "PixelPipe_gouraud",
@@ -450,14 +450,14 @@ def main():
     V = sc["vertices"].shape[0]
     # Algorithmic bytes per launch of each stage (one frame), each byte counted once:
     #   setup : index 12 B per triangle, each clip position 16 B once; subtri byte + header 16 B + data 64 B written
-    #   bin   : subtri byte + header per triangle read, 4 B per bin entry written
-    #   coarse: 4 B entry + 16 B header per bin entry read, 4 B per tile entry written
+    #   bin   : subtri byte + header per triangle read, an 8 B (tile, triangle) pair per tile entry written
+    #   coarse: the pairs read, 4 B per tile entry written
     #   fine  : 4 B per tile entry, header + data once per bin entry, colour + depth of every sample written
     N = ((W + 7) // 8 * 8) * ((H + 7) // 8 * 8)
     alg = {
         "setup": T * (12 + 1 + 16 + 64) + V * 16,
-        "bin": T * 17 + counters["bin_entries"] * 4,
-        "coarse": counters["bin_entries"] * 20 + counters["tile_entries"] * 4,
+        "bin": T * 17 + counters["tile_entries"] * 8,
+        "coarse": counters["tile_entries"] * 12,
         "fine": counters["tile_entries"] * 4 + counters["bin_entries"] * 80 + N * 8,
     }
     achieved = alg[names[dom]] / (stage_ms[dom] / 1e3) / 1e9

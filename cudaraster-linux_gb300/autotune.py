@@ -1,5 +1,5 @@
-"""Autotuner for the run-time pipeline parameters (bin size, coarse unit size,
-bin chunk size, fine warps per CTA) -- the reference's compile-time CR_*
+"""Autotuner for the run-time pipeline parameters (bin size, bin chunk size, fine
+warps per CTA) -- the reference's compile-time CR_*
 constants (Constants.hpp:24-46) made tunable. Output bits never depend on
 them (tests/test_gpu_batch.py::test_tuning_does_not_change_bits), so the
 tuner only measures time.
@@ -37,10 +37,9 @@ SELF_PIXELS = (4, 8, 12, 16, 24, 32, 48, 64)
 def candidates(quick: bool = False, medium: bool = False):
     bins = (3, 4, 5)
     warps = (4, 8)
-    units = (0,) if quick else ((0, 64, 256) if medium else (0, 64, 128, 256, 512, 1024))
-    chunks = (0,) if quick or medium else (0, 256, 1024, 4096)
-    for b, w, u, c in itertools.product(bins, warps, units, chunks):
-        yield {"bin_log2": b, "fine_warps": w, "coarse_unit_entries": u, "bin_chunk_tris": c}
+    chunks = (0,) if quick else ((0, 256) if medium else (0, 128, 256, 512))
+    for b, w, c in itertools.product(bins, warps, chunks):
+        yield {"bin_log2": b, "fine_warps": w, "bin_chunk_tris": c}
 
 
 def tune_single(scene: dict, pipe: str, cands, steps: int = 6, samples: int = 1) -> dict:

@@ -1,797 +1,990 @@
-// binning.cu -- bin and coarse stages (stages 2 and 3 of 4).
+// binning.cu -- bin and coarse stages (stages 2 and 3 of 4): the tile lists.
 //
 // The reference bins with 16 persistent CTAs writing segmented linked lists
-// per (bin, stream) and then merges the 16 streams per bin in triangle order
-// (BinRaster.inl:19-469, CoarseRaster.inl:28-809). On GB300 both stages are
-// count -> scan -> scatter passes over all SMs instead:
+// per (bin, stream), merges the 16 streams per bin in triangle order
+// (BinRaster.inl:19-469) and rasterizes each bin's list into per-tile lists
+// (CoarseRaster.inl:28-809). On GB300 the tile lists are built directly, with
+// one device-wide atomic counter per tile (they live in L2, 4 bytes a tile):
 //
-//   bin:    chunks of consecutive triangles, each taken by one warp (in
-//           order, as warps free up). binCount counts (bin, chunk) entries,
-//           binScan turns the counts into per-bin offsets in chunk order and
-//           allocates each bin's contiguous list, binScatter writes the
-//           entries. Every bin list comes out in submission order, with no
-//           merge.
-//   coarse: units of consecutive bin-list entries of one bin (sized on the
-//           device once the bin lists are known), each taken by one warp,
-//           with the same three passes over the tiles of the bin.
+//   pairs:   records the (tile, triangle) pairs of the subtriangles in at most
+//            2x2 tiles, each with its place in the tile's list, and counts
+//            their bins; queues the others as items.
+//   items:   records the pairs of the items and counts their tiles and bins.
+//   scan:    allocates each tile's list from the counts.
+//   scatter: writes the recorded pairs at their places, those of the items
+//            behind the others.
+//   sort:    puts the lists of order-dependent pipes in submission order.
 //
-// Both stages walk their items 32 at a time (a group) and expand a group into
-// (item, cell) pairs -- every cell of each item's bounding box -- dealt
-// evenly over the lanes, so an item covering many cells costs its cell count
-// / 32 iterations instead of holding up the whole warp. Pairs are taken 32 at
-// a time in item order; the rank of a pair in its cell's list is the cell's
-// running index plus the number of lower lanes on the same cell (a match on
-// the cell index).
+// The counters' atomics give a list's entries in no particular order. Pipes
+// whose fine stage resolves visibility by keys (fine.cuh) do not depend on it;
+// for the others the lists are sorted. A count -> scan -> scatter pass per
+// level, bins then tiles, with every list in order (the design before) took
+// for its six kernels, against these, in us: 101 / 74 on 1M small triangles at
+// 1080p, 309 / 190 on an 8.4M-triangle 4x MSAA heightfield at 4K, 276 / 86 on
+// 20,000 triangles of 60 pixels, 85 / 63 with the sort (11) on 300k blended
+// ones.
+//
+// None of these kernels lets its dependent launch early (launch.h): CTAs that
+// wait for it would hold slots that its own need (32-scene batch 1010 us with,
+// 959 without).
 //
 // List entries are triangle << 3 | subtriangle (7 = the triangle's own slot),
-// as in the reference. Placement of a list in memory depends on atomics,
-// its content and order do not.
+// as in the reference. Which cells an entry goes to: its box's cells, and of
+// a box larger than 2x2 cells those that the triangle may touch
+// (triTouchesCell) -- for tiles, the box within each bin counts, and the bin
+// must hold the entry too.
 #include "cudaraster/detail/binning.cuh"
 #include "cudaraster/detail/launch.h"
 #include "cudaraster/detail/per_device.h"
 
+#include <algorithm>
+
 namespace cr {
 
-constexpr int kBinThreads = 512;
-constexpr int kBinWarps = kBinThreads / 32;
+constexpr int kListThreads = 256;
+constexpr int kListWarps = kListThreads / 32;
 
-// Exclusive block scan over kBinThreads values; returns the exclusive prefix,
-// total in *total. scratch >= kBinWarps + 1 ints.
-__device__ __forceinline__ S32 blockExclusiveScan(S32 v, S32* scratch, S32* total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    S32 inc = warpInclusiveScan(v);
-    if (lane == 31) scratch[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-        S32 w = (lane < kBinWarps) ? scratch[lane] : 0;
-        S32 wi = warpInclusiveScan(w);
-        if (lane < kBinWarps) scratch[lane] = wi - w;
-        if (lane == kBinWarps - 1) scratch[kBinWarps] = wi;
+// Warp-level inclusive scan.
+__device__ __forceinline__ S32 warpInclusiveScan(S32 v) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        S32 t = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        if (lane >= o) v += t;
     }
-    __syncthreads();
-    S32 r = scratch[warp] + inc - v;
-    *total = scratch[kBinWarps];
-    __syncthreads();
-    return r;
+    return v;
 }
 
-// Geometry of a cell grid (bins of the viewport, or tiles inside one bin).
-struct Grid {
-    S32 halfW, halfH, cellLog2;
-    bool centerOnly;          // one sample per pixel: boxes of pixel centres (cellBox)
-    S32 cx0, cy0, cx1, cy1;   // clamp window (inclusive)
-    S32 stride;               // cells per row of the local index space
-};
+// Queues list entry `entry` as a large or huge item.
+__device__ __forceinline__ void queueLarge(const DrawDev& d, U32 entry, bool huge) {
+    const S32 k = atomicAdd(&d.counters->largeItems[huge ? 1 : 0], 1);
+    d.largeItems[huge ? d.maxSubtris - 1 - k : (S64)k] = entry;
+}
 
-// The current group of a warp, one word per list item (lane).
-struct GroupSmem {
-    S32 incl[32];   // inclusive prefix of the entries' box tile counts
+// Up to 32 items (subtriangles) of a warp, one word per lane, to be expanded
+// into (item, cell) pairs dealt evenly over the lanes.
+struct ItemSmem {
+    S32 incl[32];   // inclusive prefix of the items' cell counts
     U32 v[3][32];   // vertices, packed as in the triangle header
-    U32 box[32];    // lx | ly << 9 | (w - 1) << 18 (local cells, < 512 each), bit 31: box of at most 2x2 cells
+    U32 box[32];    // tile box: lx | ly << 9 | (w - 1) << 18
+    U32 ext[32];    // h - 1 | (bin box of at most 2x2 bins) << 9 | first cell of the slice << 10
     U32 mul[32];    // ceil(2^32 / w) (0 for w = 1): cell k of the box is in row umulhi(k, mul)
-    U32 entry[32];
+    S32 tile0[32];  // global tile of the box's first tile
+    S32 wt[32];     // tiles per row of the viewport
+    S32 inst[32];
+    S32 F[3][32], dx[3][32], dy[3][32];   // tile edges
 };
 
-// Publishes a group of up to 32 list items (lane i: item entry, if valid)
-// with their cell boxes; returns the group's number of (item, cell) pairs
-// and the lane's inclusive prefix of them in incl -- or -1 when no item has
-// more than one cell, with the lane's own cell (or -1) in cell1.
-__device__ __forceinline__ S32 stageItems(const DrawDev& d, const Grid& gr, bool valid, U32 entry, GroupSmem& gs,
-                                          S32& incl, int& cell1) {
+// Edge k of a triangle over the viewport's tiles: tile (cx, cy) may be touched
+// iff F + dx * cy - dy * cx >= 0 for all three. This is edgeTouchesRect on the
+// tile's rectangle, whose value E + 128 (dx * cy - dy * cx) is not negative
+// iff floor(E / 128) + dx * cy - dy * cx is not; |F| stays below 2^27 and the
+// products below 2^26, so 32 bits hold it (20,000 triangles of 60 pixels: 57 us
+// for this kernel with the 64-bit test per pair, 43 so).
+__device__ __forceinline__ void tileEdge(S32 ox, S32 oy, S32 dx, S32 dy, S32 halfW, S32 halfH, S32& F) {
+    const S32 side = 1 << (kTileLog2 + kSubpixelLog2);
+    const S32 px = (dy > 0 ? 0 : side - 1) - halfW, py = (dx > 0 ? side - 1 : 0) - halfH;
+    F = (S32)(((S64)(ox - px) * dy - (S64)(oy - py) * dx) >> (kTileLog2 + kSubpixelLog2));
+}
+
+__device__ __forceinline__ void stageItem(ItemSmem& sm, int lane, uint4 h, const TriGeom& g, const CellBox& b,
+                                          bool binsSmall, U32 cell0, S32 inst, const InstanceDev* in) {
+    const U32 w = (U32)(b.hx - b.lx + 1);
+    sm.v[0][lane] = h.x;
+    sm.v[1][lane] = h.y;
+    sm.v[2][lane] = h.z;
+    sm.box[lane] = (U32)b.lx | (U32)b.ly << 9 | (w - 1u) << 18;
+    sm.ext[lane] = (U32)(b.hy - b.ly) | (binsSmall ? 1u << 9 : 0u) | cell0 << 10;
+    sm.mul[lane] = w > 1u ? 0xFFFFFFFFu / w + 1u : 0u;
+    const S32 wt = __ldg(&in->widthTiles);
+    sm.tile0[lane] = __ldg(&in->tileBase) + b.ly * wt + b.lx;
+    sm.wt[lane] = wt;
+    sm.inst[lane] = inst;
+    const S32 halfW = __ldg(&in->width) << (kSubpixelLog2 - 1), halfH = __ldg(&in->height) << (kSubpixelLog2 - 1);
+    const S32 ox[3] = {g.x0, g.x1, g.x2}, oy[3] = {g.y0, g.y1, g.y2};
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int n = k == 2 ? 0 : k + 1;
+        const S32 dx = ox[n] - ox[k], dy = oy[n] - oy[k];
+        sm.dx[k][lane] = dx;
+        sm.dy[k][lane] = dy;
+        S32 F;
+        tileEdge(ox[k], oy[k], dx, dy, halfW, halfH, F);
+        sm.F[k][lane] = F;
+    }
+}
+
+// Pair p of the `items` staged items (p below their pair count): its item j
+// and global tile; returns whether the tile's list takes the entry. The
+// quotient k / w = umulhi(k, ceil(2^32 / w)) is exact for k * w < 2^32 (boxes
+// have at most 512 x 512 tiles).
+__device__ __forceinline__ bool pairTile(const DrawDev& d, const ItemSmem& sm, S32 items, S32 p, int& j, S32& tile) {
+    int jj = 0;
+    if (items > 1) {
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1)
+            if (sm.incl[jj + s - 1] <= p) jj += s;
+    }
+    const U32 box = sm.box[jj], ext = sm.ext[jj], mul = sm.mul[jj];
+    const U32 k = (U32)(p - (jj ? sm.incl[jj - 1] : 0)) + (ext >> 10);
+    const S32 w = (S32)(box >> 18) + 1;
+    const S32 q = (S32)(mul ? __umulhi(k, mul) : k);
+    const S32 r = (S32)k - q * w;
+    const S32 lx = (S32)(box & 0x1FFu), ly = (S32)((box >> 9) & 0x1FFu);
+    const S32 hx = lx + w - 1, hy = ly + (S32)(ext & 0x1FFu);
+    const S32 cx = lx + r, cy = ly + q;
+    j = jj;
+    tile = sm.tile0[jj] + q * sm.wt[jj] + r;
+    // The box within the tile's bin; of at most 2x2 tiles, all its tiles take
+    // the entry if the bin does. A tile that the triangle may touch lies in a
+    // bin that it may touch.
+    const S32 side = 1 << d.binLog2;
+    const S32 bx0 = cx & -side, by0 = cy & -side;
+    const bool few = min(hx, bx0 + side - 1) - max(lx, bx0) <= 1 && min(hy, by0 + side - 1) - max(ly, by0) <= 1;
+    if (!few) {
+        const S32 e0 = sm.F[0][jj] + sm.dx[0][jj] * cy - sm.dy[0][jj] * cx;
+        const S32 e1 = sm.F[1][jj] + sm.dx[1][jj] * cy - sm.dy[1][jj] * cx;
+        const S32 e2 = sm.F[2][jj] + sm.dx[2][jj] * cy - sm.dy[2][jj] * cx;
+        return (e0 | e1 | e2) >= 0;
+    }
+    if (ext >> 9 & 1u) return true;
+    const InstanceDev* in = &d.inst[sm.inst[jj]];
+    return triTouchesCell(geomFromHeader(make_uint4(sm.v[0][jj], sm.v[1][jj], sm.v[2][jj], 0u)), cx >> d.binLog2,
+                          cy >> d.binLog2, d.binLog2, __ldg(&in->width), __ldg(&in->height));
+}
+
+__device__ __forceinline__ CellBox headerBox(const TriGeom& g, const InstanceDev* in) {
+    return tileBox(min3i(g.x0, g.x1, g.x2), min3i(g.y0, g.y1, g.y2), max3i(g.x0, g.x1, g.x2), max3i(g.y0, g.y1, g.y2),
+                   __ldg(&in->width), __ldg(&in->height), __ldg(&in->widthTiles), __ldg(&in->heightTiles),
+                   __ldg(&in->samplesLog2) == 0);
+}
+
+// Instance of a triangle slot (no search for a single scene).
+__device__ __forceinline__ int instanceOf(const DrawDev& d, U32 tri) {
+    return d.numInstances == 1 ? 0 : findInstance64(d.triPrefix, d.numInstances, (S64)tri);
+}
+
+// ----------------------------------------------------------------- pairs
+//
+// A warp takes a chunk of triangles: its live subtriangles stream through a
+// ring in shared memory 32 at a time, their (tile, triangle) pairs through a
+// second one, so that both steps work with all lanes however many triangles
+// setup culled and however many tiles each covers.
+
+constexpr int kRing = 256;
+constexpr int kSharedBins = 2048;
+
+struct PairSmem {
+    U64 pairs[kRing];    // global tile << 10 | triangle of the chunk
+    U32 live[kRing];     // list entries
+    U32 medium[64];      // medium items not yet queued
+};
+
+// The grid that a triangle's boxes are formed on.
+struct SceneGrid {
+    S32 width, height, widthTiles, heightTiles, widthBins, tileBase, binBase;
+    bool centerOnly;
+};
+__device__ __forceinline__ SceneGrid loadGrid(const InstanceDev* in) {
+    return SceneGrid{__ldg(&in->width),     __ldg(&in->height),   __ldg(&in->widthTiles), __ldg(&in->heightTiles),
+                     __ldg(&in->widthBins), __ldg(&in->tileBase), __ldg(&in->binBase),    __ldg(&in->samplesLog2) == 0};
+}
+
+// Appends the list entries of triangles [next, next + 128) below end to the
+// ring (which holds fewer than 32): lane l takes triangles 4 l to 4 l + 3
+// (chunks start at multiples of four; the buffer is padded to whole words).
+// `ahead` holds their counts, loaded since the last call, and then the next
+// 128's.
+__device__ __forceinline__ U32 loadCounts(const DrawDev& d, S64 first, S64 end) {
+    U32 counts = first < end ? __ldg((const U32*)(d.triSubtris + first)) : 0u;
+    if (first + 4 > end && first < end) counts &= (1u << (8 * (U32)(end - first))) - 1u;
+    return counts;
+}
+__device__ __forceinline__ void refillRing(const DrawDev& d, S64 next, S64 end, U32& ahead, U32* ring, S32 head,
+                                           S32& fill) {
     const int lane = threadIdx.x & 31;
-    S32 n = 0;
-    CellBox b{};
-    uint4 h = make_uint4(0u, 0u, 0u, 0u);
-    if (valid) {
-        h = __ldg(&d.triHeader[entrySlot(entry, d.triHeader)]);
-        b = cellBox(geomFromHeader(h), gr.halfW, gr.halfH, gr.cellLog2, gr.cx0, gr.cy0, gr.cx1, gr.cy1, gr.centerOnly);
-        n = b.count();
-    }
-    gs.entry[lane] = entry;
-    // Every item in at most one cell (the common case for small triangles):
-    // the pairs are the items themselves, no expansion needed.
-    if (__all_sync(0xFFFFFFFFu, n <= 1)) {
-        cell1 = n == 1 ? (b.ly - gr.cy0) * gr.stride + (b.lx - gr.cx0) : -1;
+    const U32 ltMask = (1u << lane) - 1u;
+    const S64 first = next + 4 * lane;
+    U32 counts = ahead;
+    ahead = loadCounts(d, first + 128, end);
+    if (__any_sync(0xFFFFFFFFu, counts & 0xFEFEFEFEu)) {
+        // Clipped triangles with several subtriangles (rare): straight to
+        // the large items, which have room for every subtriangle.
+        for (int j = 0; j < 4; j++) {
+            const U32 n = counts >> (8 * j) & 0xFFu;
+            if (n < 2u) continue;
+            for (U32 s = 0; s < n; s++) {
+                const U32 e = (U32)(first + j) << 3 | s;
+                const TriGeom g = geomFromHeader(__ldg(&d.triHeader[entrySlot(e, d.triHeader)]));
+                queueLarge(d, e, headerBox(g, &d.inst[instanceOf(d, e >> 3)]).count() > kHugeCells);
+            }
+            counts &= ~(0xFFu << (8 * j));
+        }
         __syncwarp();
-        return -1;
     }
-    U32 box = 0, mul = 0;
-    if (n > 0) {
-        const U32 w = (U32)(b.hx - b.lx + 1);
-        box = (U32)(b.lx - gr.cx0) | (U32)(b.ly - gr.cy0) << 9 | (w - 1u) << 18 | (b.small() ? 1u << 31 : 0u);
-        mul = w > 1u ? 0xFFFFFFFFu / w + 1u : 0u;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const bool live = counts >> (8 * j) & 1u;
+        const U32 mask = __ballot_sync(0xFFFFFFFFu, live);
+        if (live) ring[(head + fill + __popc(mask & ltMask)) & (kRing - 1)] = (U32)(first + j) << 3 | 7u;
+        fill += __popc(mask);
     }
-    incl = warpInclusiveScan(n);
-    gs.incl[lane] = incl;
-    gs.v[0][lane] = h.x;
-    gs.v[1][lane] = h.y;
-    gs.v[2][lane] = h.z;
-    gs.box[lane] = box;
-    gs.mul[lane] = mul;
     __syncwarp();
+}
+
+// 32 pairs (or the chunk's last ones) between the update of their tiles'
+// counters and the write of their records.
+struct PairBatch {
+    U64 pair;
+    S32 first;     // in the head lanes of the runs of pairs on one tile: the counter before the run
+    U32 heads;
+    S32 n, at;     // pairs, index of the first one in the chunk
+};
+
+// Neighbouring triangles of a mesh mostly share their tile: a run of pairs on
+// one tile moves its counter once.
+__device__ __forceinline__ PairBatch countPairs(const DrawDev& d, const U64* ring, S32 head, S32 n, S32 at) {
+    const int lane = threadIdx.x & 31;
+    const U32 ltMask = (1u << lane) - 1u;
+    PairBatch b;
+    b.pair = lane < n ? ring[(head + lane) & (kRing - 1)] : 0ull;
+    const U32 tile = (U32)(b.pair >> 10);
+    const U32 before = __shfl_up_sync(0xFFFFFFFFu, tile, 1);
+    const bool first = lane < n && (lane == 0 || before != tile);
+    b.heads = __ballot_sync(0xFFFFFFFFu, first);
+    b.first = 0;
+    if (first) {
+        const U32 later = b.heads & ~(ltMask | 1u << lane);
+        b.first = atomicAdd(d.tileWork + ((S64)tile << d.tileWorkLog2), (later ? __ffs(later) - 1 : n) - lane);
+    }
+    b.n = n;
+    b.at = at;
+    return b;
+}
+
+__device__ __forceinline__ void writePairs(U64* pairs, const PairBatch& b) {
+    const int lane = threadIdx.x & 31;
+    const U32 upTo = b.heads & ((2u << lane) - 1u);
+    const int head = upTo ? 31 - __clz(upTo) : 0;
+    const S32 place = __shfl_sync(0xFFFFFFFFu, b.first, head) + lane - head;
+    if (lane < b.n) pairs[b.at + lane] = (U64)(U32)place << 37 | b.pair;
+}
+
+// Moves up to 32 of the warp's medium items to the queue.
+__device__ __forceinline__ void flushMedium(const DrawDev& d, const U32* medium, S32& fill) {
+    const int lane = threadIdx.x & 31;
+    const S32 n = min(fill, 32);
+    S32 base = 0;
+    if (lane == 0) base = atomicAdd(&d.counters->mediumItems, n);
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    if (lane < n) d.mediumItems[base + lane] = medium[fill - n + lane];
+    fill -= n;
+    __syncwarp();
+}
+
+// Persistent warps over chunks, taken in order as warps free up. Bound by
+// latency (flags, headers and counters are three trips to L2 or beyond): a
+// group's headers load while the one before it is worked on, a batch's records
+// are written after the next one's counters have been issued.
+__global__ void __launch_bounds__(kListThreads) pairKernel(const __grid_constant__ DrawDev d) {
+    pdlWait();
+    __shared__ PairSmem s_pair[kListWarps];
+    __shared__ S32 s_bins[kSharedBins];
+    if (__ldcg(&d.counters->overflow) & kOverflowSubtris) return;
+    // Bins are counted in shared memory and handed over at the end, where the
+    // draw's fit.
+    const bool sharedBins = d.totalBins <= kSharedBins;
+    if (sharedBins) {
+        for (int b = threadIdx.x; b < d.totalBins; b += kListThreads) s_bins[b] = 0;
+        __syncthreads();
+    }
+    auto countBin = [&](S32 b) {
+        if (sharedBins) atomicAdd(&s_bins[b], 1); else atomicAdd(&d.binWork[b * kBinWorkStride], 1);
+    };
+    PairSmem& sm = s_pair[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const U32 ltMask = (1u << lane) - 1u;
+    const bool recordable = d.totalTiles <= kMaxRecord && d.totalTris <= kMaxRecord;
+    S32 mediumFill = 0;
+    // A warp's first chunk is its own, the others come from a counter (one
+    // address passes 1.4 atomics per ns: 5,000 warps asking at once wait 3.5 us).
+    const S32 warps = gridDim.x * kListWarps;
+    S32 chunk = blockIdx.x * kListWarps + (threadIdx.x >> 5);
+    while (chunk < d.numChunks) {
+        S32 nextChunk = 0;   // taken now, needed at the end
+        if (lane == 0 && d.numChunks > warps) nextChunk = atomicAdd(&d.counters->chunkWork, 1);
+        const S64 t0 = (S64)chunk * d.chunkTris, end = min(t0 + d.chunkTris, d.totalTris);
+        U64* out = d.pairs + (S64)chunk * 2 * d.chunkTris;
+        // Mostly all of a chunk's triangles belong to one scene.
+        const int inst0 = instanceOf(d, (U32)t0);
+        const bool oneScene = inst0 == instanceOf(d, (U32)end - 1u);
+        SceneGrid grid = loadGrid(&d.inst[inst0]);
+        S64 next = t0;
+        U32 ahead = loadCounts(d, next + 4 * lane, end);
+        S32 head = 0, fill = 0;                   // live subtriangles in the ring
+        S32 pairHead = 0, pairFill = 0, done = 0; // pairs in their ring, pairs taken from it
+        PairBatch prev{};
+        U32 entry = 0;
+        uint4 h = make_uint4(0u, 0u, 0u, 0u);
+        auto fetch = [&]() {   // the next group's size, its entries and headers
+            while (fill < 32 && next < end) {
+                refillRing(d, next, end, ahead, sm.live, head, fill);
+                next += 128;
+            }
+            const int g = min(fill, 32);
+            if (lane < g) {
+                entry = sm.live[(head + lane) & (kRing - 1)];
+                h = __ldg(&d.triHeader[entry >> 3]);
+            }
+            __syncwarp();
+            head += g;
+            fill -= g;
+            return g;
+        };
+        int g = fetch();
+        while (g > 0) {
+            const U32 e = entry;
+            const TriGeom tg = geomFromHeader(h);
+            const bool valid = lane < g;
+            g = fetch();
+            if (!oneScene && valid) grid = loadGrid(&d.inst[instanceOf(d, e >> 3)]);
+            const CellBox t = tileBox(min3i(tg.x0, tg.x1, tg.x2), min3i(tg.y0, tg.y1, tg.y2), max3i(tg.x0, tg.x1, tg.x2),
+                                      max3i(tg.y0, tg.y1, tg.y2), grid.width, grid.height, grid.widthTiles,
+                                      grid.heightTiles, grid.centerOnly);
+            const CellBox b = t.coarser(d.binLog2);
+            const bool live = valid && !b.empty();
+            bool small = live && t.small() && recordable;
+            bool one = small && !t.empty();
+            U32 m0 = __ballot_sync(0xFFFFFFFFu, one);
+            U32 mR = __ballot_sync(0xFFFFFFFFu, one && t.hx > t.lx), mD = __ballot_sync(0xFFFFFFFFu, one && t.hy > t.ly);
+            S32 nR = __popc(m0), nD = nR + __popc(mR), nB = nD + __popc(mD), total = nB + __popc(mR & mD);
+            if (done + pairFill + total > 2 * d.chunkTris) {
+                // The chunk's room is used up (rare): the group is queued.
+                small = one = false;
+                m0 = mR = mD = 0u;
+                total = 0;
+            }
+            const U64 pair = (U64)(U32)(grid.tileBase + t.ly * grid.widthTiles + t.lx) << 10 | (U64)((e >> 3) - (U32)t0);
+            const S32 tail = pairHead + pairFill;
+            if (one) sm.pairs[(tail + __popc(m0 & ltMask)) & (kRing - 1)] = pair;
+            if (mR >> lane & 1u) sm.pairs[(tail + nR + __popc(mR & ltMask)) & (kRing - 1)] = pair + (1u << 10);
+            if (mD) {
+                const U64 below = pair + ((U64)(U32)grid.widthTiles << 10);
+                if (mD >> lane & 1u) sm.pairs[(tail + nD + __popc(mD & ltMask)) & (kRing - 1)] = below;
+                const U32 mB = mR & mD;
+                if (mB >> lane & 1u) sm.pairs[(tail + nB + __popc(mB & ltMask)) & (kRing - 1)] = below + (1u << 10);
+            }
+            pairFill += total;
+            if (small) {
+                const S32 bin = grid.binBase + b.ly * grid.widthBins + b.lx;
+                countBin(bin);
+                if (b.hx > b.lx || b.hy > b.ly) {
+                    if (b.hx > b.lx) countBin(bin + 1);
+                    if (b.hy > b.ly) {
+                        countBin(bin + grid.widthBins);
+                        if (b.hx > b.lx) countBin(bin + grid.widthBins + 1);
+                    }
+                }
+            }
+            const bool queued = live && !small;
+            if (__any_sync(0xFFFFFFFFu, queued)) {
+                const S32 cells = t.count();
+                const U32 mm = __ballot_sync(0xFFFFFFFFu, queued && cells <= kMediumCells);
+                if (mm >> lane & 1u) sm.medium[mediumFill + __popc(mm & ltMask)] = e;
+                mediumFill += __popc(mm);
+                if (queued && cells > kMediumCells) queueLarge(d, e, cells > kHugeCells);
+            }
+            __syncwarp();
+            if (mediumFill >= 32) flushMedium(d, sm.medium, mediumFill);
+            while (pairFill >= 32 || (g == 0 && pairFill > 0)) {
+                const S32 n = min(pairFill, 32);
+                const PairBatch cur = countPairs(d, sm.pairs, pairHead, n, done);
+                pairHead += n;
+                pairFill -= n;
+                done += n;
+                writePairs(out, prev);
+                prev = cur;
+            }
+            __syncwarp();
+        }
+        writePairs(out, prev);
+        if (lane == 0) d.pairCount[chunk] = done;
+        chunk = warps + __shfl_sync(0xFFFFFFFFu, nextChunk, 0);
+    }
+    if (mediumFill > 0) flushMedium(d, sm.medium, mediumFill);
+    if (sharedBins) {
+        __syncthreads();
+        for (int b = threadIdx.x; b < d.totalBins; b += kListThreads) {
+            const S32 v = s_bins[b];
+            if (v) atomicAdd(&d.binWork[b * kBinWorkStride], v);
+        }
+    }
+}
+
+// ----------------------------------------------------------------- items
+//
+// A warp takes a unit of items -- a slice of one huge item's box, one large
+// item, or a group of medium ones -- and expands it into (item, cell) pairs
+// dealt evenly over the lanes, so lanes stay busy however uneven the boxes
+// are. The units with the most pairs come first.
+
+struct ItemUnits {
+    S32 hugeSlices, hugeUnits;     // units per huge item, their units
+    S32 largeSlices, largeUnits;   // likewise of the large items
+    S32 medium, group;             // medium items, items per unit
+    S32 total;
+};
+
+// Splits the items over the launched warps: huge items in up to 64 slices that
+// give about eight units a warp, large ones in up to 2 and medium ones in
+// groups of 4 to 32 that give about one.
+__device__ __forceinline__ ItemUnits planItems(const DrawDev& d) {
+    ItemUnits u;
+    const S32 warps = (S32)gridDim.x * kListWarps;
+    const S32 large = __ldcg(&d.counters->largeItems[0]), huge = __ldcg(&d.counters->largeItems[1]);
+    u.medium = __ldcg(&d.counters->mediumItems);
+    u.hugeSlices = min(max(8 * warps / max(huge, 1), 1), 64);
+    u.largeSlices = min(max(2 * warps / max(large, 1), 1), 2);
+    u.hugeUnits = huge * u.hugeSlices;
+    u.largeUnits = large * u.largeSlices;
+    u.group = min(max(u.medium / warps, 4), 32);
+    u.total = u.hugeUnits + u.largeUnits + (u.medium + u.group - 1) / u.group;
+    return u;
+}
+
+// Stages up to 32 items in shared memory: lane l < items has list entry
+// `entry`, of whose box it takes slice `slice` of `slices`; counts their bins
+// (a sliced item's with its first slice). Returns the number of (item, cell)
+// pairs.
+__device__ __forceinline__ S32 stageItems(const DrawDev& d, S32 items, U32 entry, S32 slice, S32 slices, ItemSmem& sm) {
+    const int lane = threadIdx.x & 31;
+    S32 n = 0, bins = 0;
+    if (lane < items) {
+        const uint4 h = __ldg(&d.triHeader[entrySlot(entry, d.triHeader)]);
+        const int ii = instanceOf(d, entry >> 3);
+        const InstanceDev* in = &d.inst[ii];
+        const TriGeom g = geomFromHeader(h);
+        const CellBox b = headerBox(g, in), bb = b.coarser(d.binLog2);
+        n = b.count();
+        U32 c0 = 0;
+        if (slices > 1) {   // at most 2^18 cells times 64 slices
+            c0 = (U32)n * (U32)slice / (U32)slices;
+            n = (S32)((U32)n * (U32)(slice + 1) / (U32)slices - c0);
+        }
+        stageItem(sm, lane, h, g, b, bb.small(), c0, ii, in);   // (an item without cells is never looked up)
+        if (slice == 0) {
+            bins = bb.count();
+            if (bins <= 4) {
+                const bool test = !bb.small();
+                const S32 wb = __ldg(&in->widthBins);
+                for (S32 by = bb.ly; by <= bb.hy; by++)
+                    for (S32 bx = bb.lx; bx <= bb.hx; bx++)
+                        if (!test || triTouchesCell(g, bx, by, d.binLog2, __ldg(&in->width), __ldg(&in->height)))
+                            atomicAdd(&d.binWork[(__ldg(&in->binBase) + by * wb + bx) * kBinWorkStride], 1);
+            }
+        }
+    }
+    const S32 incl = warpInclusiveScan(n);
+    sm.incl[lane] = incl;
+    __syncwarp();
+    // Boxes of more than four bins: the whole warp, one item at a time.
+    for (U32 m = __ballot_sync(0xFFFFFFFFu, bins > 4); m; m &= m - 1) {
+        const int j = __ffs(m) - 1;
+        const InstanceDev* in = &d.inst[sm.inst[j]];
+        const S32 width = __ldg(&in->width), height = __ldg(&in->height);
+        const TriGeom g = geomFromHeader(make_uint4(sm.v[0][j], sm.v[1][j], sm.v[2][j], 0u));
+        const CellBox bb = headerBox(g, in).coarser(d.binLog2);
+        const S32 w = bb.hx - bb.lx + 1, cnt = bb.count();
+        const bool test = !bb.small();
+        const S32 wb = __ldg(&in->widthBins), binBase = __ldg(&in->binBase);
+        for (S32 k = lane; k < cnt; k += 32) {
+            const S32 by = bb.ly + k / w, bx = bb.lx + k % w;
+            if (!test || triTouchesCell(g, bx, by, d.binLog2, width, height))
+                atomicAdd(&d.binWork[(binBase + by * wb + bx) * kBinWorkStride], 1);
+        }
+    }
     return __shfl_sync(0xFFFFFFFFu, incl, 31);
 }
 
-// Pair p of the group (p below the group's pair count): its item j and its
-// cell in the grid's local index space; returns whether the item's triangle
-// may touch the cell (always, for boxes of at most 2x2 cells). The quotient
-// k / w = umulhi(k, ceil(2^32 / w)) is exact for k * w < 2^32 (boxes have at
-// most 512 x 512 cells).
-__device__ __forceinline__ bool pairCell(const GroupSmem& gs, const Grid& gr, S32 p, int& j, int& cell) {
-    int jj = 0;
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1)
-        if (gs.incl[jj + s - 1] <= p) jj += s;
-    const S32 k = p - (jj ? gs.incl[jj - 1] : 0);
-    const U32 box = gs.box[jj];
-    const S32 w = (S32)((box >> 18) & 0x1FFu) + 1;
-    const U32 mul = gs.mul[jj];
-    const S32 q = mul ? (S32)__umulhi((U32)k, mul) : k;
-    const S32 lx = (S32)(box & 0x1FFu) + k - q * w;
-    const S32 ly = (S32)((box >> 9) & 0x1FFu) + q;
-    j = jj;
-    cell = ly * gr.stride + lx;
-    if (box >> 31) return true;
-    const TriGeom g = geomFromHeader(make_uint4(gs.v[0][jj], gs.v[1][jj], gs.v[2][jj], 0u));
-    const S32 side = 1 << gr.cellLog2;
-    const S32 rx0 = ((gr.cx0 + lx) << gr.cellLog2) - gr.halfW, ry0 = ((gr.cy0 + ly) << gr.cellLog2) - gr.halfH;
-    return triTouchesRect(g, rx0, ry0, rx0 + side - 1, ry0 + side - 1);
-}
+// A warp's current block of item pair records: its own first, then from a
+// counter. A warp leaves at most one block partly filled, so a draw whose tile
+// entries fit has blocks for all; past the last one nothing is written (the
+// scan reports the overflow).
+struct ItemBlock {
+    S32 block, fill;
+};
 
-// Next work item (bin chunk or coarse unit) for this warp, taken in order
-// from a counter; uniform across the warp.
-__device__ __forceinline__ int warpNextUnit(S32* counter) {
-    int u = 0;
-    if ((threadIdx.x & 31) == 0) u = atomicAdd(counter, 1);
-    return __shfl_sync(0xFFFFFFFFu, u, 0);
-}
-
-__device__ __forceinline__ Grid binGrid(const InstanceDev* in, int binLog2) {
-    Grid gr;
-    gr.halfW = __ldg(&in->width) << (kSubpixelLog2 - 1);
-    gr.halfH = __ldg(&in->height) << (kSubpixelLog2 - 1);
-    gr.cellLog2 = binLog2 + kTileLog2 + kSubpixelLog2;
-    gr.centerOnly = __ldg(&in->samplesLog2) == 0;
-    gr.cx0 = 0;
-    gr.cy0 = 0;
-    gr.cx1 = __ldg(&in->widthBins) - 1;
-    gr.cy1 = __ldg(&in->heightBins) - 1;
-    gr.stride = __ldg(&in->widthBins);
-    return gr;
-}
-
-// ------------------------------------------------------------------ bin
-
-// A warp's slice of a chunk streams its subtriangle items through a ring in
-// shared memory; culled triangles carry none. Items keep (triangle,
-// subtriangle) order.
-constexpr int kRing = 256;
-
-// Appends the items of the slice's next triangles until the ring holds at
-// least 32 items or the slice is exhausted: four triangles per lane, or one
-// per lane when four would overflow the ring (32 triangles carry at most 224
-// items, which always fit behind fewer than 32). next and fill are uniform.
-__device__ __forceinline__ void refillRing(const DrawDev& d, S64& next, S64 end, U32* ring, S32 head, S32& fill) {
+// Records the pairs of the lanes with `hit` and counts their tiles.
+__device__ __forceinline__ void recordItemPairs(const DrawDev& d, ItemBlock& blk, bool hit, U32 entry, S32 tile) {
     const int lane = threadIdx.x & 31;
-    while (fill < 32 && next < end) {
-        const S64 t = next + (S64)lane * 4;
-        int n[4];
-        int sum = 0;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            n[j] = (t + j < end) ? d.triSubtris[t + j] : 0;
-            sum += n[j];
+    const U32 mask = __ballot_sync(0xFFFFFFFFu, hit);
+    const S32 cnt = __popc(mask);
+    if (cnt == 0) return;
+    if (hit) atomicAdd(&d.tileItems[tile], 1);
+    S32 at = blk.fill + __popc(mask & ((1u << lane) - 1u));
+    S32 block = blk.block;
+    blk.fill += cnt;
+    if (blk.fill > kItemBlock) {
+        S32 fresh = 0;
+        if (lane == 0) {
+            fresh = gridDim.x * kListWarps + atomicAdd(&d.counters->itemBlocks, 1);
+            if (block < d.maxItemBlocks) d.itemBlockCount[block] = kItemBlock;
         }
-        const S32 incl = warpInclusiveScan(sum);
-        const S32 total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-        if (fill + total <= kRing) {
-            S32 pos = head + fill + incl - sum;
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-                for (int s = 0; s < n[j]; s++) ring[(pos++) & (kRing - 1)] = ((U32)(t + j) << 3) | (U32)(n[j] == 1 ? 7 : s);
-            fill += total;
-            next += 32 * 4;
-        } else {
-            const S64 t1 = next + lane;
-            const int m = (t1 < end) ? d.triSubtris[t1] : 0;
-            const S32 incl1 = warpInclusiveScan(m);
-            S32 pos = head + fill + incl1 - m;
-            for (int s = 0; s < m; s++) ring[(pos++) & (kRing - 1)] = ((U32)t1 << 3) | (U32)(m == 1 ? 7 : s);
-            fill += __shfl_sync(0xFFFFFFFFu, incl1, 31);
-            next += 32;
+        fresh = __shfl_sync(0xFFFFFFFFu, fresh, 0);
+        if (at >= kItemBlock) {
+            block = fresh;
+            at -= kItemBlock;
         }
+        blk.fill -= kItemBlock;
+        blk.block = fresh;
     }
-    __syncwarp();
+    if (hit && block < d.maxItemBlocks) d.itemPairs[(S64)block * kItemBlock + at] = (U64)entry << 32 | (U32)tile;
 }
 
-// Walks the items of triangles [next, end) over the bin grid: fn(hit, cell,
-// j, peers) is called by every lane for each batch of 32 pairs, hit telling
-// whether the lane's pair touches its cell, j the pair's lane in the group
-// (its item) and peers the lanes of the batch on the same cell.
-template <class Fn>
-__device__ __forceinline__ void walkSlice(const DrawDev& d, const Grid& gr, S64 next, S64 end, U32* ring,
-                                          GroupSmem& gs, Fn fn) {
+// Records the pairs of the items and counts their tiles and bins. Persistent
+// warps over the units.
+__global__ void __launch_bounds__(kListThreads, kItemWarpsPerSM / kListWarps) itemKernel(const __grid_constant__ DrawDev d) {
+    pdlWait();
+    __shared__ ItemSmem s_items[kListWarps];
+    if (__ldcg(&d.counters->overflow) & kOverflowSubtris) return;
+    ItemSmem& sm = s_items[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    S32 head = 0, fill = 0;
-    for (;;) {
-        refillRing(d, next, end, ring, head, fill);
-        if (fill == 0) break;
-        const int g = min(fill, 32);
-        const bool valid = lane < g;
-        const U32 entry = valid ? ring[(head + lane) & (kRing - 1)] : 0u;
-        head = (head + g) & (kRing - 1);
-        fill -= g;
-        S32 incl;
-        int cell1;
-        const S32 P = stageItems(d, gr, valid, entry, gs, incl, cell1);
-        if (P < 0) {
-            const bool hit = cell1 >= 0;
-            fn(hit, cell1, lane, __match_any_sync(0xFFFFFFFFu, hit ? (U32)cell1 : 0x80000000u + (U32)lane));
+    const ItemUnits iu = planItems(d);
+    if (blockIdx.x == 0 && threadIdx.x == 0) d.counters->numUnits = iu.total;
+    const S32 warps = gridDim.x * kListWarps;
+    ItemBlock blk{(S32)(blockIdx.x * kListWarps + (threadIdx.x >> 5)), 0};
+    for (S32 u = blockIdx.x * kListWarps + (threadIdx.x >> 5); u < iu.total; u += warps) {
+        S32 items = 1, slice = 0, slices = 1;
+        U32 entry = 0;
+        if (u < iu.hugeUnits + iu.largeUnits) {
+            const bool huge = u < iu.hugeUnits;
+            const S32 k = huge ? u : u - iu.hugeUnits;
+            slices = huge ? iu.hugeSlices : iu.largeSlices;
+            const S32 h = k / slices;
+            slice = k - h * slices;
+            entry = __ldcg(&d.largeItems[huge ? d.maxSubtris - 1 - h : (S64)h]);
+        } else {
+            const S32 first = (u - iu.hugeUnits - iu.largeUnits) * iu.group;
+            items = min(iu.group, iu.medium - first);
+            if (lane < items) entry = __ldcg(&d.mediumItems[first + lane]);
         }
+        const S32 P = stageItems(d, items, entry, slice, slices, sm);
         for (S32 base = 0; base < P; base += 32) {
             const S32 p = base + lane;
-            int j = 0, cell = 0;
-            const bool hit = p < P && pairCell(gs, gr, p, j, cell);
-            const U32 peers = __match_any_sync(0xFFFFFFFFu, hit ? (U32)cell : 0x80000000u + (U32)lane);
-            fn(hit, cell, j, peers);
+            int j = 0;
+            S32 tile = 0;
+            const bool hit = p < P && pairTile(d, sm, items, p, j, tile);
+            const U32 e = __shfl_sync(0xFFFFFFFFu, entry, j);
+            recordItemPairs(d, blk, hit, e, tile);
         }
         __syncwarp();
     }
+    if (lane == 0 && blk.block < d.maxItemBlocks) d.itemBlockCount[blk.block] = blk.fill;
+    if (blockIdx.x == 0 && threadIdx.x == 0) d.counters->itemWarps = warps;
 }
 
-// Bin count / scatter CTAs: warps work independently, one chunk at a time.
-constexpr int kWalkThreads = 256;
-constexpr int kWalkWarps = kWalkThreads / 32;
+// ------------------------------------------------------------------ scan
 
-struct ChunkInfo {
-    const InstanceDev* in;
-    int local;      // chunk index inside its instance
-    int nb;         // bins of the instance
-    S64 t0, t1;     // triangles of the chunk
-};
+// Four consecutive tiles per thread; a CTA's lists are one contiguous piece of
+// the list memory, allocated with one atomic. The first CTA also hands over
+// the bin counts. The work arrays end zeroed, for the next draw.
+constexpr int kScanTiles = kListThreads * 4;
 
-__device__ __forceinline__ ChunkInfo chunkInfo(const DrawDev& d, int chunk) {
-    ChunkInfo c;
-    c.in = &d.inst[findInstance(d.chunkPrefix, d.numInstances, chunk)];
-    c.local = chunk - __ldg(&c.in->chunkBase);
-    c.nb = __ldg(&c.in->widthBins) * __ldg(&c.in->heightBins);
-    const S64 triBase = __ldg(&c.in->triBase);
-    c.t0 = triBase + (S64)c.local * __ldg(&c.in->chunkTris);
-    c.t1 = min(c.t0 + __ldg(&c.in->chunkTris), triBase + __ldg(&c.in->numTris));
-    return c;
-}
-
-// Persistent warps over chunks: each chunk's entry count per bin, written to
-// the (bin, chunk) matrix where not zero (the matrix is zero between draws),
-// and, when d.binStageCap > 0, its (bin, entry) pairs in list order for the
-// scatter pass (as many as fit; their total in binStageCount).
-__global__ void __launch_bounds__(kWalkThreads) binCountKernel(DrawDev d) {
+__global__ void __launch_bounds__(kListThreads) listScanKernel(const __grid_constant__ DrawDev d) {
     pdlWait();
-    pdlTrigger();
-    extern __shared__ S32 s_cells[];   // [kWalkWarps][maxBins]
-    __shared__ U32 s_ring[kWalkWarps][kRing];
-    __shared__ GroupSmem s_group[kWalkWarps];
-    if (__ldg(&d.counters->overflow) & kOverflowSubtris) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const U32 ltMask = (1u << lane) - 1u;
-    S32* cnt = s_cells + warp * d.maxBins;
-    GroupSmem& gs = s_group[warp];
-    for (;;) {
-        const int chunk = warpNextUnit(&d.counters->binWork[0]);
-        if (chunk >= d.totalChunks) break;
-        const ChunkInfo c = chunkInfo(d, chunk);
-        const Grid gr = binGrid(c.in, d.binLog2);
-        for (int b = lane; b < c.nb; b += 32) cnt[b] = 0;
-        __syncwarp();
-        U64* stage = d.binStage + (S64)chunk * d.binStageCap;
-        S32 staged = 0;   // pairs of the chunk so far (uniform)
-        walkSlice(d, gr, c.t0, c.t1, s_ring[warp], gs, [&](bool hit, int cell, int j, U32 peers) {
-            if (hit && (peers >> lane) == 1u) cnt[cell] += __popc(peers);
-            if (d.binStageCap > 0) {
-                const U32 hits = __ballot_sync(0xFFFFFFFFu, hit);
-                const S32 pos = staged + __popc(hits & ltMask);
-                if (hit && pos < d.binStageCap) stage[pos] = (U64)(U32)cell << 32 | gs.entry[j];
-                staged += __popc(hits);
-            }
-        });
-        if (lane == 0 && d.binStageCap > 0) d.binStageCount[chunk] = staged;
-        S32* out = d.chunkBinCount + __ldg(&c.in->chunkCountBase) + c.local;
-        const S64 nc = __ldg(&c.in->numChunks);
-        for (int b = lane; b < c.nb; b += 32) {
-            const S32 v = cnt[b];
-            if (v) out[b * nc] = v;
-        }
-        __syncwarp();
-    }
-}
-
-// Run by the last bin-scan CTA to finish, once every bin's entry count is
-// known: the coarse unit size (the caller's, or the smallest power of two
-// from 64 that gives at most unitTarget units and fits maxUnits) and each
-// bin's first unit. Contains barriers; the whole CTA calls it.
-__device__ __forceinline__ void planUnits(const DrawDev& d, S32* s_scratch) {
-    const S64 total = __ldcg(&d.counters->binEntries);
-    S64 U = d.unitEntries;
-    if (U <= 0) {
-        const S64 room = max((S64)1, d.maxUnits - d.totalBins - 1);
-        U = 64;
-        while (U < 4096 && total > (S64)max(d.unitTarget, 1) * U) U *= 2;
-        while (total > room * U && U < ((S64)1 << 30)) U *= 2;
-    }
-    S32 carry = 0;
-    for (int b0 = 0; b0 < d.totalBins; b0 += kBinThreads) {
-        const int b = b0 + threadIdx.x;
-        const U32 c = b < d.totalBins ? (U32)__ldcg(&d.binCount[b]) : 0u;
-        const S32 n = (S32)(c / (U32)U + (c % (U32)U != 0u));
-        S32 tot;
-        const S32 ex = blockExclusiveScan(n, s_scratch, &tot);
-        if (b < d.totalBins) d.binUnitFirst[b] = carry + ex;
-        carry += tot;
-    }
-    if (threadIdx.x == 0) {
-        d.counters->unitEntries = (S32)U;
-        d.counters->numUnits = carry;
-    }
-}
-
-// One CTA per global bin: chunk-order exclusive offsets and list allocation;
-// the last CTA to finish plans the coarse units.
-__global__ void __launch_bounds__(kBinThreads) binScanKernel(DrawDev d) {
-    pdlWait();
-    pdlTrigger();
-    __shared__ S32 s_scratch[kBinWarps + 1];
-    __shared__ int s_inst;
-    __shared__ bool s_last;
-    if (__ldg(&d.counters->overflow) & kOverflowSubtris) return;
-    const int gb = blockIdx.x;
-    if (threadIdx.x == 0) s_inst = findInstance(d.binPrefix, d.numInstances, gb);
-    __syncthreads();
-    const InstanceDev* in = &d.inst[s_inst];
-    const int nb = __ldg(&in->widthBins) * __ldg(&in->heightBins);
-    const int b = gb - __ldg(&in->binBase);
-    const int nc = __ldg(&in->numChunks);
-    S32* counts = d.chunkBinCount + __ldg(&in->chunkCountBase) + (S64)b * nc;
-    S32* offs = d.chunkBinOffset + __ldg(&in->chunkCountBase) + b;
-    // Eight consecutive chunks per thread, loaded before they are summed.
-    constexpr int kPer = 8;
-    S32 carry = 0;
-    for (int c0 = 0; c0 < nc; c0 += kBinThreads * kPer) {
-        const int cb = c0 + threadIdx.x * kPer;
-        S32 v[kPer];
-#pragma unroll
-        for (int k = 0; k < kPer; k++) v[k] = (cb + k < nc) ? counts[cb + k] : 0;
-        S32 sum = 0;
-#pragma unroll
-        for (int k = 0; k < kPer; k++) sum += v[k];
-        S32 tot;
-        S32 ex = carry + blockExclusiveScan(sum, s_scratch, &tot);
-#pragma unroll
-        for (int k = 0; k < kPer; k++) {
-            if (v[k]) {
-                counts[cb + k] = 0;
-                offs[(S64)(cb + k) * nb] = ex;
-                ex += v[k];
-            }
-        }
-        carry += tot;
-    }
-    if (threadIdx.x == 0) {
-        S32 start = atomicAdd(&d.counters->binEntries, carry);
-        if ((S64)start + carry > d.maxBinEntries) atomicOr(&d.counters->overflow, kOverflowBin);
-        d.binStart[gb] = start;
-        d.binCount[gb] = carry;
-        __threadfence();
-        s_last = atomicAdd(&d.counters->binsDone, 1) == d.totalBins - 1;
-    }
-    __syncthreads();
-    if (s_last) {
-        __threadfence();
-        planUnits(d, s_scratch);
-    }
-}
-
-// Persistent warps over chunks: writes each chunk's entries into the bin
-// lists, from the chunk's offset in every bin it touches: from the pairs the
-// count pass recorded, 32 at a time (a pair's rank in its bin is the bin's
-// running index plus the lower lanes of the batch on the same bin), or, for a
-// chunk whose pairs did not fit, by walking its triangles again.
-__global__ void __launch_bounds__(kWalkThreads) binScatterKernel(DrawDev d) {
-    pdlWait();
-    pdlTrigger();
-    extern __shared__ S32 s_cells[];   // [kWalkWarps][maxBins]: next list index per bin
-    __shared__ U32 s_ring[kWalkWarps][kRing];
-    __shared__ GroupSmem s_group[kWalkWarps];
-    if (__ldg(&d.counters->overflow) & (kOverflowSubtris | kOverflowBin)) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const U32 ltMask = (1u << lane) - 1u;
-    S32* run = s_cells + warp * d.maxBins;
-    GroupSmem& gs = s_group[warp];
-    for (;;) {
-        const int chunk = warpNextUnit(&d.counters->binWork[1]);
-        if (chunk >= d.totalChunks) break;
-        const ChunkInfo c = chunkInfo(d, chunk);
-        const Grid gr = binGrid(c.in, d.binLog2);
-        // Offsets of bins the chunk does not touch are stale and never used.
-        const S32* offs = d.chunkBinOffset + __ldg(&c.in->chunkCountBase) + (S64)c.local * c.nb;
-        const S32 binBase = __ldg(&c.in->binBase);
-        for (int b = lane; b < c.nb; b += 32) run[b] = __ldg(&d.binStart[binBase + b]) + __ldg(&offs[b]);
-        __syncwarp();
-        const S32 staged = d.binStageCap > 0 ? __ldcg(&d.binStageCount[chunk]) : -1;
-        if (staged >= 0 && staged <= d.binStageCap) {
-            const U64* stage = d.binStage + (S64)chunk * d.binStageCap;
-            U64 next = lane < staged ? __ldcg(&stage[lane]) : 0ull;   // the next batch loads during this one
-            for (S32 i0 = 0; i0 < staged; i0 += 32) {
-                const bool valid = i0 + lane < staged;
-                const U64 pr = next;
-                if (i0 + 32 + lane < staged) next = __ldcg(&stage[i0 + 32 + lane]);
-                const int cell = (int)(pr >> 32);
-                const U32 peers = __match_any_sync(0xFFFFFFFFu, valid ? (U32)cell : 0x80000000u + (U32)lane);
-                if (valid) {
-                    const S64 idx = (S64)run[cell] + __popc(peers & ltMask);
-                    if (idx < d.maxBinEntries) d.binList[idx] = (U32)pr;
-                }
-                __syncwarp();
-                if (valid && (peers >> lane) == 1u) run[cell] += __popc(peers);
-                __syncwarp();
-            }
-            continue;
-        }
-        walkSlice(d, gr, c.t0, c.t1, s_ring[warp], gs, [&](bool hit, int cell, int j, U32 peers) {
-            if (hit) {
-                const S64 idx = (S64)run[cell] + __popc(peers & ltMask);
-                if (idx < d.maxBinEntries) d.binList[idx] = gs.entry[j];
-            }
-            __syncwarp();
-            if (hit && (peers >> lane) == 1u) run[cell] += __popc(peers);
-            __syncwarp();
-        });
-    }
-}
-
-// --------------------------------------------------------------- coarse
-//
-// A coarse unit (up to unitEntries consecutive entries of one bin list) is
-// taken by one warp, which walks it 32 entries (a group) at a time. No
-// CTA-wide barrier is involved: units, groups and ranks are all warp-local.
-
-constexpr int kCoarseThreads = 256;
-constexpr int kCoarseWarps = kCoarseThreads / 32;
-
-struct UnitInfo {
-    const InstanceDev* in;
-    S32 gb, seg, bx, by, e0, e1;
-};
-
-// Unit u: the last bin whose first unit is at most u (bins without units
-// share their first unit with the next bin), and its entry range.
-__device__ __forceinline__ void loadUnit(const DrawDev& d, int u, S32 unitEntries, UnitInfo& ui) {
-    int lo = 0, hi = d.totalBins - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(&d.binUnitFirst[mid]) <= u) lo = mid; else hi = mid - 1;
-    }
-    ui.gb = lo;
-    ui.in = &d.inst[findInstance(d.binPrefix, d.numInstances, ui.gb)];
-    ui.seg = u - __ldg(&d.binUnitFirst[lo]);
-    const S32 b = ui.gb - __ldg(&ui.in->binBase);
-    const S32 wb = __ldg(&ui.in->widthBins);
-    ui.bx = b % wb;
-    ui.by = b / wb;
-    const S32 start = __ldg(&d.binStart[ui.gb]), cnt = __ldg(&d.binCount[ui.gb]);
-    ui.e0 = start + ui.seg * unitEntries;
-    ui.e1 = min(ui.e0 + unitEntries, start + cnt);
-}
-
-__device__ __forceinline__ Grid tileGrid(const UnitInfo& ui, int binLog2) {
-    Grid gr;
-    const S32 side = 1 << binLog2;
-    gr.halfW = __ldg(&ui.in->width) << (kSubpixelLog2 - 1);
-    gr.halfH = __ldg(&ui.in->height) << (kSubpixelLog2 - 1);
-    gr.cellLog2 = kTileLog2 + kSubpixelLog2;
-    gr.centerOnly = __ldg(&ui.in->samplesLog2) == 0;
-    gr.cx0 = ui.bx << binLog2;
-    gr.cy0 = ui.by << binLog2;
-    gr.cx1 = min(gr.cx0 + side - 1, __ldg(&ui.in->widthTiles) - 1);
-    gr.cy1 = min(gr.cy0 + side - 1, __ldg(&ui.in->heightTiles) - 1);
-    gr.stride = side;
-    return gr;
-}
-
-// Persistent warps over coarse units (taken dynamically): per-unit tile
-// counts, and, for units below d.tileStageUnits, their (tile, entry) pairs in
-// list order for the scatter pass (as many as fit; their total in
-// tileStageCount).
-__global__ void __launch_bounds__(kCoarseThreads) coarseCountKernel(DrawDev d) {
-    pdlWait();
-    pdlTrigger();
-    extern __shared__ S32 smem[];
-    __shared__ GroupSmem s_group[kCoarseWarps];
-    if (__ldg(&d.counters->overflow) & (kOverflowSubtris | kOverflowBin)) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int tpb = 1 << (2 * d.binLog2);
-    S32* cnt = smem + warp * tpb;
-    GroupSmem& gs = s_group[warp];
-    const U32 ltMask = (1u << lane) - 1u;
-    const S32 numUnits = (S32)min((S64)__ldg(&d.counters->numUnits), d.maxUnits);
-    const S32 unitEntries = __ldg(&d.counters->unitEntries);
-    for (;;) {
-        const int u = warpNextUnit(&d.counters->coarseWork[0]);   // count pass
-        if (u >= numUnits) break;
-        UnitInfo ui;
-        loadUnit(d, u, unitEntries, ui);
-        const Grid gr = tileGrid(ui, d.binLog2);
-        for (int t = lane; t < tpb; t += 32) cnt[t] = 0;
-        __syncwarp();
-        const bool record = u < d.tileStageUnits;
-        U64* stage = d.tileStage + (S64)u * d.tileStageCap;
-        S32 staged = 0;   // pairs of the unit so far (uniform)
-        // Records the batch's hits in lane order, which is list order.
-        auto recordHits = [&](bool hit, int cell, U32 entry) {
-            const U32 hits = __ballot_sync(0xFFFFFFFFu, hit);
-            const S32 pos = staged + __popc(hits & ltMask);
-            if (hit && pos < d.tileStageCap) stage[pos] = (U64)(U32)cell << 32 | entry;
-            staged += __popc(hits);
-        };
-        for (S32 e0 = ui.e0; e0 < ui.e1; e0 += 32) {
-            S32 incl;
-            int cell1;
-            const bool valid = e0 + lane < ui.e1;
-            const S32 P = stageItems(d, gr, valid, valid ? __ldg(&d.binList[e0 + lane]) : 0u, gs, incl, cell1);
-            if (P < 0) {
-                if (cell1 >= 0) atomicAdd(&cnt[cell1], 1);
-                if (record) recordHits(cell1 >= 0, cell1, gs.entry[lane]);
-            }
-            for (S32 base = 0; base < P; base += 32) {
-                const S32 p = base + lane;
-                int j = 0, cell = 0;
-                const bool hit = p < P && pairCell(gs, gr, p, j, cell);
-                if (hit) atomicAdd(&cnt[cell], 1);
-                if (record) recordHits(hit, cell, gs.entry[j]);
-            }
-            __syncwarp();
-        }
-        if (lane == 0 && record) d.tileStageCount[u] = staged;
-        S32* out = d.unitTileCount + (S64)u * tpb;
-        for (int t = lane; t < tpb; t += 32) out[t] = cnt[t];
-        __syncwarp();
-    }
-}
-
-// One CTA per global bin: unit-order offsets per tile and tile list
-// allocation. Each warp takes a contiguous slice of the bin's units: it sums
-// its slice per tile, the slice sums are scanned across warps per tile, and
-// each warp then writes its slice's running offsets.
-__global__ void __launch_bounds__(kBinThreads) coarseScanKernel(DrawDev d) {
-    pdlWait();
-    pdlTrigger();
-    extern __shared__ S32 s_part[];   // [kBinWarps][tpb]: slice sums, then slice starts
-    __shared__ S32 s_scratch[kBinWarps + 1];
-    __shared__ int s_inst;
+    __shared__ S32 s_warp[kListWarps];
     __shared__ S32 s_base;
-    if (__ldg(&d.counters->overflow) & (kOverflowSubtris | kOverflowBin)) return;
-    const int gb = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x == 0) s_inst = findInstance(d.binPrefix, d.numInstances, gb);
-    __syncthreads();
-    const InstanceDev* in = &d.inst[s_inst];
-    const int tpb = 1 << (2 * d.binLog2);
-    const S32 side = 1 << d.binLog2;
-    const S32 b = gb - __ldg(&in->binBase);
-    const S32 wb = __ldg(&in->widthBins);
-    const S32 bx = b % wb, by = b / wb;
-    const S32 wt = __ldg(&in->widthTiles), ht = __ldg(&in->heightTiles);
-    const S32 tileBase = __ldg(&in->tileBase);
-    const S32 cnt = __ldg(&d.binCount[gb]);
-    const S32 unitEntries = __ldg(&d.counters->unitEntries);
-    const S32 units = (cnt + unitEntries - 1) / unitEntries;
-    S32* counts = d.unitTileCount + (S64)__ldg(&d.binUnitFirst[gb]) * tpb;
-    const S32 per = (units + kBinWarps - 1) / kBinWarps;
-    const S32 k0 = min(warp * per, units), k1 = min(k0 + per, units);
-    for (int t = lane; t < tpb; t += 32) {
-        S32 acc = 0;
-        for (S32 k = k0; k < k1; k++) acc += counts[(S64)k * tpb + t];
-        s_part[warp * tpb + t] = acc;
+    const bool failed = (__ldcg(&d.counters->overflow) & kOverflowSubtris) != 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const S32 t0 = blockIdx.x * kScanTiles + threadIdx.x * 4;
+    S32 c[4], own[4];   // entries, and those recorded by setup
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        c[k] = own[k] = 0;
+        if (t0 + k < d.totalTiles) own[k] = __ldcg(&d.tileWork[(t0 + k) << d.tileWorkLog2]);
     }
-    __syncthreads();
-    S32 carry = 0;
-    for (int t0 = 0; t0 < tpb; t0 += kBinThreads) {
-        const int t = t0 + threadIdx.x;
-        S32 acc = 0;
-        if (t < tpb) {
-            for (int w = 0; w < kBinWarps; w++) {
-                const S32 v = s_part[w * tpb + t];
-                s_part[w * tpb + t] = acc;
-                acc += v;
+    if (t0 + 3 < d.totalTiles) {
+        const int4 x = __ldcg((const int4*)(d.tileItems + t0));
+        c[0] = own[0] + x.x, c[1] = own[1] + x.y, c[2] = own[2] + x.z, c[3] = own[3] + x.w;
+        *(int4*)(d.tileItems + t0) = make_int4(0, 0, 0, 0);
+        *(int4*)(d.tileCount + t0) = make_int4(c[0], c[1], c[2], c[3]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (t0 + k < d.totalTiles) {
+                c[k] = own[k] + __ldcg(&d.tileItems[t0 + k]);
+                d.tileItems[t0 + k] = 0;
+                d.tileCount[t0 + k] = c[k];
             }
         }
-        S32 tot;
-        const S32 ex = blockExclusiveScan(acc, s_scratch, &tot);
-        if (t < tpb) {
-            const S32 tx = (bx << d.binLog2) + (t & (side - 1));
-            const S32 ty = (by << d.binLog2) + (t >> d.binLog2);
-            if (tx < wt && ty < ht) {
-                const S32 g = tileBase + ty * wt + tx;
-                d.tileCount[g] = acc;
-                d.tileStart[g] = carry + ex;   // relative; rebased below
-            }
-        }
-        carry += tot;
     }
-    if (threadIdx.x == 0) {
-        const S32 base = atomicAdd(&d.counters->tileEntries, carry);
-        if ((S64)base + carry > d.maxTileEntries) atomicOr(&d.counters->overflow, kOverflowTile);
-        s_base = base;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (t0 + k < d.totalTiles) d.tileWork[(t0 + k) << d.tileWorkLog2] = 0;
+    const S32 sum = c[0] + c[1] + c[2] + c[3];
+    const S32 incl = warpInclusiveScan(sum);
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        const S32 v = lane < kListWarps ? s_warp[lane] : 0;
+        const S32 i = warpInclusiveScan(v);
+        if (lane < kListWarps) s_warp[lane] = i - v;
+        if (lane == kListWarps - 1 && !failed) {
+            const S32 base = atomicAdd(&d.counters->tileEntries, i);
+            if ((S64)base + i > d.maxTileEntries) atomicOr(&d.counters->overflow, kOverflowTile);
+            s_base = base;
+        }
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < tpb; t += kBinThreads) {
-        const S32 tx = (bx << d.binLog2) + (t & (side - 1));
-        const S32 ty = (by << d.binLog2) + (t >> d.binLog2);
-        if (tx < wt && ty < ht) d.tileStart[tileBase + ty * wt + tx] += s_base;
+    S32 s = s_base + s_warp[warp] + incl - sum;
+    if (!failed) {
+        if (t0 + 3 < d.totalTiles) {
+            const int4 v = make_int4(s, s + c[0], s + c[0] + c[1], s + c[0] + c[1] + c[2]);
+            *(int4*)(d.tileStart + t0) = v;
+            *(int4*)(d.tileCursor + t0) = make_int4(v.x + own[0], v.y + own[1], v.z + own[2], v.w + own[3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (t0 + k < d.totalTiles) {
+                    d.tileStart[t0 + k] = s;
+                    d.tileCursor[t0 + k] = s + own[k];
+                }
+                s += c[k];
+            }
+        }
     }
-    for (int t = lane; t < tpb; t += 32) {
-        S32 run = s_part[warp * tpb + t];
-        for (S32 k = k0; k < k1; k++) {
-            S32* p = &counts[(S64)k * tpb + t];
-            const S32 c = *p;
-            *p = run;
-            run += c;
+    if (blockIdx.x == 0) {
+        S32 mine = 0;
+        for (S32 b = threadIdx.x; b < d.totalBins; b += kListThreads) {
+            const S32 v = __ldcg(&d.binWork[b * kBinWorkStride]);
+            d.binWork[b * kBinWorkStride] = 0;
+            d.binCount[b] = v;
+            mine += v;
+        }
+        mine = __reduce_add_sync(0xFFFFFFFFu, mine);
+        __syncthreads();
+        if (lane == 0) s_warp[warp] = mine;
+        __syncthreads();
+        if (threadIdx.x == 0 && !failed) {
+            S64 total = 0;
+            for (int w = 0; w < kListWarps; w++) total += s_warp[w];
+            d.counters->binEntries = (S32)total;
+            if (total > d.maxBinEntries) atomicOr(&d.counters->overflow, kOverflowBin);
         }
     }
 }
 
-// Persistent warps over coarse units (taken dynamically): writes tile list
-// entries, from the pairs the count pass recorded or, for a unit whose pairs
-// were not recorded, by walking its entries again. Pairs are taken 32 at a
-// time in list order; the rank of a pair in its tile list is the tile's
-// running index plus the number of lower lanes of the batch on the same tile
-// (a match on the tile index).
-__global__ void __launch_bounds__(kCoarseThreads) coarseScatterKernel(DrawDev d) {
+// --------------------------------------------------------------- scatter
+
+__device__ __forceinline__ void putEntry(const DrawDev& d, S32 idx, U32 entry) {
+    if ((S64)idx < d.maxTileEntries) d.tileList[idx] = entry;
+}
+
+// Persistent warps: the pair records, then those of the items.
+__global__ void __launch_bounds__(kListThreads) listScatterKernel(const __grid_constant__ DrawDev d) {
     pdlWait();
-    pdlTrigger();
-    extern __shared__ S32 smem[];
-    __shared__ GroupSmem s_group[kCoarseWarps];
-    if (__ldg(&d.counters->overflow) & (kOverflowSubtris | kOverflowBin | kOverflowTile)) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const U32 ltMask = (1u << lane) - 1u;
-    const int tpb = 1 << (2 * d.binLog2);
-    const S32 side = 1 << d.binLog2;
-    S32* run = smem + (size_t)warp * tpb;
-    GroupSmem& gs = s_group[warp];
-    const S32 numUnits = (S32)min((S64)__ldg(&d.counters->numUnits), d.maxUnits);
-    const S32 unitEntries = __ldg(&d.counters->unitEntries);
-    for (;;) {
-        const int u = warpNextUnit(&d.counters->coarseWork[1]);
-        if (u >= numUnits) break;
-        UnitInfo ui;
-        loadUnit(d, u, unitEntries, ui);
-        const Grid gr = tileGrid(ui, d.binLog2);
-        const S32 wt = __ldg(&ui.in->widthTiles);
-        const S32 tileBase = __ldg(&ui.in->tileBase);
-        const S32* unitCount = d.unitTileCount + (S64)u * tpb;
-        for (int t = lane; t < tpb; t += 32) {
-            const S32 tx = gr.cx0 + (t & (side - 1)), ty = gr.cy0 + (t >> d.binLog2);
-            S32 v = 0;
-            if (tx <= gr.cx1 && ty <= gr.cy1) v = __ldg(&d.tileStart[tileBase + ty * wt + tx]) + __ldg(&unitCount[t]);
-            run[t] = v;
+    if (__ldcg(&d.counters->overflow)) return;
+    const int lane = threadIdx.x & 31;
+    const S32 warps = gridDim.x * kListWarps, warpIdx = blockIdx.x * kListWarps + (threadIdx.x >> 5);
+    // A chunk's pairs by one warp, or by several where there are few chunks.
+    const S32 split = max(1, min(8, 2 * warps / max(d.numChunks, 1)));
+    for (S32 u = warpIdx; u < d.numChunks * split; u += warps) {
+        const S32 chunk = u / split, part = u - chunk * split;
+        const S32 count = __ldcg(&d.pairCount[chunk]);
+        const U64* pairs = d.pairs + (S64)chunk * 2 * d.chunkTris;
+        const U32 t0 = (U32)chunk * (U32)d.chunkTris;
+        // Four pairs per lane in flight.
+        for (S32 p0 = part * 128 + lane; p0 < count; p0 += split * 128) {
+            U64 rec[4];
+            S32 start[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) rec[k] = p0 + k * 32 < count ? __ldcg(&pairs[p0 + k * 32]) : 0ull;
+#pragma unroll
+            for (int k = 0; k < 4; k++) start[k] = __ldg(&d.tileStart[(U32)(rec[k] >> 10) & (U32)(kMaxRecord - 1)]);
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (p0 + k * 32 < count)
+                    putEntry(d, start[k] + (S32)(rec[k] >> 37), (t0 + ((U32)rec[k] & 1023u)) << 3 | 7u);
         }
-        __syncwarp();
-        const S32 staged = u < d.tileStageUnits ? __ldcg(&d.tileStageCount[u]) : -1;
-        if (staged >= 0 && staged <= d.tileStageCap) {
-            const U64* stage = d.tileStage + (S64)u * d.tileStageCap;
-            U64 next = lane < staged ? __ldcg(&stage[lane]) : 0ull;   // the next batch loads during this one
-            for (S32 i0 = 0; i0 < staged; i0 += 32) {
-                const bool valid = i0 + lane < staged;
-                const U64 pr = next;
-                if (i0 + 32 + lane < staged) next = __ldcg(&stage[i0 + 32 + lane]);
-                const int cell = (int)(pr >> 32);
-                const U32 peers = __match_any_sync(0xFFFFFFFFu, valid ? (U32)cell : 0x80000000u + (U32)lane);
-                if (valid) {
-                    const S64 idx = (S64)run[cell] + __popc(peers & ltMask);
-                    if (idx < d.maxTileEntries) d.tileList[idx] = (U32)pr;
-                }
-                __syncwarp();
-                if (valid && (peers >> lane) == 1u) run[cell] += __popc(peers);
-                __syncwarp();
-            }
-            continue;
+    }
+    const S32 blocks = min(__ldcg(&d.counters->itemWarps) + __ldcg(&d.counters->itemBlocks), d.maxItemBlocks);
+    constexpr int kParts = kItemBlock / 32;
+    for (S64 u = warpIdx; u < (S64)blocks * kParts; u += warps) {
+        const S32 block = (S32)(u / kParts), at = (S32)(u % kParts) * 32 + lane;
+        if (at >= __ldcg(&d.itemBlockCount[block])) continue;
+        const U64 rec = __ldcg(&d.itemPairs[(S64)block * kItemBlock + at]);
+        putEntry(d, atomicAdd(&d.tileCursor[(U32)rec], 1), (U32)(rec >> 32));
+    }
+}
+
+// ------------------------------------------------------------------ sort
+//
+// A warp sorts the lists of four neighbouring tiles at a time where they have
+// at most 8 entries each, of two with at most 16, and single ones of up to 256
+// in registers; longer
+// ones are sorted by their CTA: runs of 256 by its warps, then merged pair by
+// pair in shared memory (an entry's place in a merged run is its own index
+// plus its rank in the other run: the entries of a list are distinct), up to
+// kSortShared entries; lists beyond that are merged in place in global memory
+// with a bitonic network from runs of kSortShared.
+
+constexpr int kSortRun = 256;
+constexpr int kSortShared = 4096;
+constexpr int kSparseLists = 16;   // mean list length below which a warp takes four tiles at a time
+constexpr int kSortCtas = 6;   // resident CTAs per SM
+
+// Sorts each W consecutive lanes' values (bitonic).
+template <int W>
+__device__ __forceinline__ U32 laneSort(U32 v) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 2; k <= W; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const U32 o = __shfl_xor_sync(0xFFFFFFFFu, v, j);
+            const bool up = k == W || (lane & k) == 0;
+            v = ((lane & j) == 0) == up ? min(v, o) : max(v, o);
         }
-        for (S32 e0 = ui.e0; e0 < ui.e1; e0 += 32) {
-            S32 incl;
-            int cell1;
-            const bool valid = e0 + lane < ui.e1;
-            const S32 P = stageItems(d, gr, valid, valid ? __ldg(&d.binList[e0 + lane]) : 0u, gs, incl, cell1);
-            if (P < 0) {
-                const bool hit = cell1 >= 0;
-                const U32 peers = __match_any_sync(0xFFFFFFFFu, hit ? (U32)cell1 : 0x80000000u + (U32)lane);
-                if (hit) {
-                    const S64 idx = (S64)run[cell1] + __popc(peers & ltMask);
-                    if (idx < d.maxTileEntries) d.tileList[idx] = gs.entry[lane];
+    }
+    return v;
+}
+
+// Sorts the lists of up to W entries of 32 / W tiles, the lanes of a tile
+// holding its list's extent.
+template <int W>
+__device__ __forceinline__ void sortShort(U32* tileList, S32 n, S32 start) {
+    const int at = (threadIdx.x & 31) & (W - 1);
+    U32 v = at < n ? tileList[start + at] : 0xFFFFFFFFu;
+    v = laneSort<W>(v);
+    if (at < n) tileList[start + at] = v;
+}
+
+// Sorts 32 * E values, lane l holding values l, l + 32, ... (bitonic).
+template <int E>
+__device__ __forceinline__ void warpSort(U32 (&v)[E]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 2; k <= 32 * E; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            if (j >= 32) {
+#pragma unroll
+                for (int e = 0; e < E; e++) {
+                    const int f = e ^ (j >> 5);
+                    if (f > e) {
+                        const bool up = ((e << 5) & k) == 0;
+                        const U32 a = v[e], b = v[f];
+                        v[e] = up ? min(a, b) : max(a, b);
+                        v[f] = up ? max(a, b) : min(a, b);
+                    }
                 }
-                __syncwarp();
-                if (hit && (peers >> lane) == 1u) run[cell1] += __popc(peers);
-                __syncwarp();
-            }
-            for (S32 base = 0; base < P; base += 32) {
-                const S32 p = base + lane;
-                int j = 0, cell = 0;
-                const bool hit = p < P && pairCell(gs, gr, p, j, cell);
-                const U32 peers = __match_any_sync(0xFFFFFFFFu, hit ? (U32)cell : 0x80000000u + (U32)lane);
-                if (hit) {
-                    const S64 idx = (S64)run[cell] + __popc(peers & ltMask);
-                    if (idx < d.maxTileEntries) d.tileList[idx] = gs.entry[j];
+            } else {
+#pragma unroll
+                for (int e = 0; e < E; e++) {
+                    const U32 o = __shfl_xor_sync(0xFFFFFFFFu, v[e], j);
+                    const bool up = k >= 32 ? (((e << 5) & k) == 0) : ((lane & k) == 0);
+                    v[e] = ((lane & j) == 0) == up ? min(v[e], o) : max(v[e], o);
                 }
-                __syncwarp();
-                if (hit && (peers >> lane) == 1u) run[cell] += __popc(peers);
-                __syncwarp();
             }
         }
+    }
+}
+
+// Sorts src[0, n), n <= 32 * E, into dst.
+template <int E>
+__device__ __forceinline__ void warpSortList(const U32* src, U32* dst, S32 n) {
+    const int lane = threadIdx.x & 31;
+    U32 v[E];
+#pragma unroll
+    for (int e = 0; e < E; e++) v[e] = e * 32 + lane < n ? src[e * 32 + lane] : 0xFFFFFFFFu;
+    warpSort<E>(v);
+#pragma unroll
+    for (int e = 0; e < E; e++)
+        if (e * 32 + lane < n) dst[e * 32 + lane] = v[e];
+}
+
+__device__ __forceinline__ void warpSortAny(const U32* src, U32* dst, S32 n) {
+    if (n <= 32) warpSortList<1>(src, dst, n);
+    else if (n <= 64) warpSortList<2>(src, dst, n);
+    else if (n <= 128) warpSortList<4>(src, dst, n);
+    else warpSortList<8>(src, dst, n);
+}
+
+// Sorts list[0, n), n <= kSortShared, through the two shared buffers; called
+// by the whole CTA.
+__device__ __forceinline__ void ctaSort(U32* list, S32 n, U32* a, U32* b) {
+    for (S32 r = (threadIdx.x >> 5) * kSortRun; r < n; r += kListWarps * kSortRun)
+        warpSortAny(list + r, a + r, min(n - r, kSortRun));
+    __syncthreads();
+    for (S32 run = kSortRun; run < n; run *= 2) {
+        for (S32 i = threadIdx.x; i < n; i += kListThreads) {
+            const U32 x = a[i];
+            const S32 r0 = i & ~(2 * run - 1);
+            const bool right = (i & run) != 0;
+            const S32 o0 = right ? r0 : r0 + run;                       // the sibling run
+            S32 lo = min(o0, n), hi = min(o0 + run, n);
+            const S32 ofirst = lo;
+            while (lo < hi) {
+                const S32 mid = (lo + hi) >> 1;
+                if (a[mid] < x) lo = mid + 1; else hi = mid;
+            }
+            b[r0 + (i & (run - 1)) + (lo - ofirst)] = x;
+        }
+        __syncthreads();
+        U32* t = a;
+        a = b;
+        b = t;
+    }
+    for (S32 i = threadIdx.x; i < n; i += kListThreads) list[i] = a[i];
+    __syncthreads();
+}
+
+// One step of an ascending bitonic merge of v[0, n): compares i with its
+// partner at distance j, or (flip) with its mirror image in blocks of 2 j.
+// Partners at or beyond n count as larger than everything.
+__device__ __forceinline__ void mergeStep(U32* v, S32 n, S32 j, bool flip) {
+    for (S32 p = threadIdx.x; p < n; p += kListThreads) {
+        const S32 i = (p / j) * 2 * j + p % j;                          // the lower partner of pair p
+        const S32 o = flip ? (i | (2 * j - 1)) - (i & (2 * j - 1)) : i + j;
+        if (i < n && o < n) {
+            const U32 x = v[i], y = v[o];
+            if (x > y) {
+                v[i] = y;
+                v[o] = x;
+            }
+        }
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ void ctaSortLong(U32* list, S32 n, U32* a, U32* b) {
+    for (S32 r = 0; r < n; r += kSortShared) ctaSort(list + r, min(n - r, kSortShared), a, b);
+    for (S64 run = kSortShared; run < n; run *= 2) {
+        mergeStep(list, n, (S32)run, true);
+        for (S32 j = (S32)(run / 2); j > 0; j >>= 1) mergeStep(list, n, j, false);
+    }
+}
+
+__global__ void __launch_bounds__(kListThreads) listSortKernel(const __grid_constant__ DrawDev d, S32 tileBegin,
+                                                               S32 tileEnd) {
+    pdlWait();
+    __shared__ U32 s_a[kSortShared], s_b[kSortShared];
+    __shared__ S32 s_long[kListThreads];
+    if (__ldcg(&d.counters->overflow)) return;
+    const int lane = threadIdx.x & 31;
+    const S32 warps = gridDim.x * kListWarps;
+    const S32 quads = (tileEnd - tileBegin + 3) / 4;
+    bool anyLong = false;
+    // A warp takes quads of tiles, every gridDim.x-th one per CTA. Neighbouring quads go to different CTAs: a crowded
+    // viewport's long lists would otherwise pile up on a few.
+    if (__ldcg(&d.counters->tileEntries) < kSparseLists * d.totalTiles) {
+        // Mostly short lists: a quad at a time, its extents (of the tile lane /
+        // 8) loaded during the sort of the quad before it.
+        S32 quad = blockIdx.x + (threadIdx.x >> 5) * gridDim.x;
+        S32 n = 0, start = 0;
+        auto load = [&]() {
+            const S32 tile = tileBegin + quad * 4 + (lane >> 3);
+            const bool on = quad < quads && tile < tileEnd;
+            n = on ? __ldg(&d.tileCount[tile]) : 0;
+            start = on ? __ldg(&d.tileStart[tile]) : 0;
+        };
+        load();
+        while (quad < quads) {
+            const S32 cnt = n, first = start;
+            quad += warps;
+            load();
+            const S32 most = __reduce_max_sync(0xFFFFFFFFu, cnt);
+            if (most <= 8) {
+                if (most > 1) sortShort<8>(d.tileList, cnt, first);
+                continue;
+            }
+            anyLong = anyLong || most > kSortRun;
+#pragma unroll 1
+            for (int half = 0; half < 2; half++) {
+                const S32 c0 = __shfl_sync(0xFFFFFFFFu, cnt, half * 16), c1 = __shfl_sync(0xFFFFFFFFu, cnt, half * 16 + 8);
+                const S32 s0 = __shfl_sync(0xFFFFFFFFu, first, half * 16), s1 = __shfl_sync(0xFFFFFFFFu, first, half * 16 + 8);
+                if (max(c0, c1) <= 16) {
+                    sortShort<16>(d.tileList, lane < 16 ? c0 : c1, lane < 16 ? s0 : s1);
+                } else {
+                    if (c0 > 1 && c0 <= kSortRun) warpSortAny(d.tileList + s0, d.tileList + s0, c0);
+                    if (c1 > 1 && c1 <= kSortRun) warpSortAny(d.tileList + s1, d.tileList + s1, c1);
+                }
+            }
+        }
+    } else {
+        // A tile at a time, its extent loaded during the sort of the one before.
+        const S32 step = gridDim.x * 4;
+        S32 k = blockIdx.x * 4 + (threadIdx.x & 96) / 32 + (threadIdx.x >> 7) * step;   // tile of the range
+        const S32 tiles = tileEnd - tileBegin;
+        S32 n = k < tiles ? __ldg(&d.tileCount[tileBegin + k]) : 0, start = k < tiles ? __ldg(&d.tileStart[tileBegin + k]) : 0;
+        while (k < tiles) {
+            U32* list = d.tileList + start;
+            const S32 cnt = n;
+            k += (kListWarps / 4) * step;
+            if (k < tiles) {
+                n = __ldg(&d.tileCount[tileBegin + k]);
+                start = __ldg(&d.tileStart[tileBegin + k]);
+            }
+            if (cnt > 1 && cnt <= kSortRun) warpSortAny(list, list, cnt);
+            anyLong = anyLong || cnt > kSortRun;
+        }
+    }
+    // The long lists among the CTA's tiles, by the whole CTA.
+    if (!__syncthreads_or(anyLong)) return;
+    for (S32 q0 = blockIdx.x; q0 < quads; q0 += (kListThreads / 4) * gridDim.x) {
+        // The CTA's quads are every gridDim.x-th one, in both cases.
+        const S32 t = tileBegin + (q0 + (threadIdx.x >> 2) * gridDim.x) * 4 + (threadIdx.x & 3);
+        const bool isLong = t < tileEnd && __ldg(&d.tileCount[t]) > kSortRun;
+        s_long[threadIdx.x] = isLong ? t : -1;
+        if (!__syncthreads_or(isLong)) continue;
+        for (int k = 0; k < kListThreads; k++) {
+            const S32 lt = s_long[k];
+            if (lt < 0) continue;
+            const S32 ln = __ldg(&d.tileCount[lt]);
+            U32* l = d.tileList + __ldg(&d.tileStart[lt]);
+            if (ln <= kSortShared) ctaSort(l, ln, s_a, s_b); else ctaSortLong(l, ln, s_a, s_b);
+        }
+        __syncthreads();
     }
 }
 
 // ------------------------------------------------------------ launchers
 
-size_t binWalkSmem(int maxBins) { return sizeof(S32) * kWalkWarps * (size_t)maxBins; }
-size_t coarseCountSmem(int binLog2) { return sizeof(S32) * kCoarseWarps * ((size_t)1 << (2 * binLog2)); }
-size_t coarseScatterSmem(int binLog2) { return sizeof(S32) * kCoarseWarps * ((size_t)1 << (2 * binLog2)); }
-
-cudaError_t launchBinning(const DrawDev& d, int maxBins, int numSMs, cudaStream_t stream, cudaEvent_t evCoarse) {
-    // Shared-memory limits are per device: set them once on each device used.
-    static OncePerDevice attributes;
-    attributes.run([] {
-        cudaFuncSetAttribute(binScatterKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-        cudaFuncSetAttribute(binCountKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-        cudaFuncSetAttribute(coarseScatterKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-        cudaFuncSetAttribute(coarseCountKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-        cudaFuncSetAttribute(coarseScanKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    });
-    // Resident coarse CTAs per SM for bins of 8, 16 and 32 tiles a side.
-    static IntsPerDevice<6> coarseCountCtas, coarseScatterCtas;
-    const int bl = d.binLog2 >= 3 && d.binLog2 <= 5 ? d.binLog2 : 4;
-    const int countCtas = coarseCountCtas.get(bl, [](int b) {
+// The list stages after setup; evCoarse (may be null) is recorded between the
+// bin (pairs, items) and coarse (list) stages.
+cudaError_t launchBinning(const DrawDev& d, int numSMs, cudaStream_t stream, cudaEvent_t evCoarse) {
+    static IntsPerDevice<2> ctas;   // resident CTAs per SM of the pair and scatter kernels
+    const int pairCtas = ctas.get(0, [](int) {
         int n = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, coarseCountKernel, kCoarseThreads, coarseCountSmem(b));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pairKernel, kListThreads, 0);
         return n > 0 ? n : 1;
     });
-    const int scatterCtas = coarseScatterCtas.get(bl, [](int b) {
+    const int scatterCtas = ctas.get(1, [](int) {
         int n = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, coarseScatterKernel, kCoarseThreads, coarseScatterSmem(b));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, listScatterKernel, kListThreads, 0);
         return n > 0 ? n : 1;
     });
-    // Units sized on the device: about two per resident coarse-scatter warp.
-    DrawDev dl = d;
-    dl.unitTarget = 2 * numSMs * scatterCtas * kCoarseWarps;
-    // binScan also runs for a draw without triangles: it zeroes the bin counts.
-    // Persistent bin warps: as many CTAs as are resident at once, and no more
-    // than the draw's chunks can keep busy.
-    dl.maxBins = maxBins;
-    const int walkSmem = (int)binWalkSmem(maxBins);
-    static IntsPerDevice<1025> walkCtasFor;   // resident bin CTAs per SM, by bins of the largest instance
-    const int mb = maxBins >= 1 && maxBins <= 1024 ? maxBins : 1024;
-    const int walkCtas = walkCtasFor.get(mb, [](int bins) {
-        int n = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, binScatterKernel, kWalkThreads, (int)binWalkSmem(bins));
-        return n > 0 ? n : 1;
-    });
-    const int walkGrid = (int)min((S64)numSMs * walkCtas, (S64)(dl.totalChunks + kWalkWarps - 1) / kWalkWarps);
     cudaError_t e = cudaSuccess;
-    if (dl.totalChunks > 0) e = launchKernel(binCountKernel, walkGrid, kWalkThreads, walkSmem, stream, true, dl);
-    if (e == cudaSuccess) e = launchKernel(binScanKernel, dl.totalBins, kBinThreads, 0, stream, true, dl);
-    if (e == cudaSuccess && dl.totalChunks > 0)
-        e = launchKernel(binScatterKernel, walkGrid, kWalkThreads, walkSmem, stream, true, dl);
+    if (d.totalTris > 0) {
+        const int pairGrid = std::min(numSMs * pairCtas, (d.numChunks + kListWarps - 1) / kListWarps);
+        e = launchKernel(pairKernel, pairGrid, kListThreads, 0, stream, true, d);
+        if (e == cudaSuccess) e = launchKernel(itemKernel, numSMs * (kItemWarpsPerSM / kListWarps), kListThreads, 0, stream, true, d);
+    }
     if (e == cudaSuccess && evCoarse) e = cudaEventRecord(evCoarse, stream);
-    if (e != cudaSuccess) return e;
-    // Persistent coarse warps: as many CTAs as are resident at once, and no
-    // more than the draw's units can keep busy.
-    const S64 unitCtas = (dl.maxUnits + kCoarseWarps - 1) / kCoarseWarps;
-    const int countGrid = (int)min((S64)numSMs * countCtas, unitCtas);
-    const int scatterGrid = (int)min((S64)numSMs * scatterCtas, unitCtas);
-    e = launchKernel(coarseCountKernel, countGrid, kCoarseThreads, coarseCountSmem(dl.binLog2), stream, true, dl);
+    // The scan also runs for a draw without triangles: it zeroes the counts.
     if (e == cudaSuccess)
-        e = launchKernel(coarseScanKernel, dl.totalBins, kBinThreads,
-                         sizeof(S32) * kBinWarps * ((size_t)1 << (2 * dl.binLog2)), stream, true, dl);
-    if (e == cudaSuccess)
-        e = launchKernel(coarseScatterKernel, scatterGrid, kCoarseThreads, coarseScatterSmem(dl.binLog2), stream, true,
-                         dl);
+        e = launchKernel(listScanKernel, (d.totalTiles + kScanTiles - 1) / kScanTiles, kListThreads, 0, stream, true, d);
+    if (e == cudaSuccess && d.totalTris > 0)
+        e = launchKernel(listScatterKernel, numSMs * scatterCtas, kListThreads, 0, stream, true, d);
     return e;
+}
+
+// Sorts the lists of tiles [tileBegin, tileEnd) into submission order.
+cudaError_t launchListSort(const DrawDev& d, int32_t tileBegin, int32_t tileEnd, int numSMs, cudaStream_t stream) {
+    if (d.totalTris <= 0 || tileEnd <= tileBegin) return cudaSuccess;
+    const int64_t need = ((int64_t)tileEnd - tileBegin + 4 * kListWarps - 1) / (4 * kListWarps);
+    return launchKernel(listSortKernel, (unsigned)std::min<int64_t>(need, (int64_t)numSMs * kSortCtas), kListThreads, 0, stream,
+                        true, d, tileBegin, tileEnd);
 }
 
 }  // namespace cr

@@ -8,6 +8,7 @@
 // message in cr_last_error() instead of exiting the process; the C++
 // wrapper (CudaRaster.hpp) turns them into the reference's fail().
 #include "cudaraster.h"
+#include "cudaraster/detail/binning.cuh"
 #include "cudaraster/detail/device.cuh"
 #include "cudaraster/detail/launch.h"
 #include "cudaraster/detail/pipe_registry.h"
@@ -19,11 +20,13 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
 namespace cr {
-cudaError_t launchBinning(const DrawDev& d, int maxBins, int numSMs, cudaStream_t stream, cudaEvent_t evCoarse);
+cudaError_t launchBinning(const DrawDev& d, int numSMs, cudaStream_t stream, cudaEvent_t evCoarse);
+cudaError_t launchListSort(const DrawDev& d, int32_t tileBegin, int32_t tileEnd, int numSMs, cudaStream_t stream);
 }
 
 using namespace cr;
@@ -81,7 +84,8 @@ struct DevBuf {
     cudaError_t ensureZeroed(size_t need) {
         if (need <= bytes) return cudaSuccess;
         cudaError_t e = ensure(need);
-        return e == cudaSuccess ? cudaMemset(ptr, 0, bytes) : e;
+        if (e == cudaSuccess) e = cudaMemset(ptr, 0, bytes);
+        return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;   // draws may use non-blocking streams
     }
     void release() {
         if (ptr) cudaFree(ptr);
@@ -122,10 +126,8 @@ struct cr_context {
     int64_t maxSubtris = 0, maxBinEntries = 0, maxTileEntries = 0;
     bool userCapacity = false;  // capacities set by cr_set_capacity replace the estimates
     // Device memory.
-    DevBuf triSubtris, triHeader, triData, chunkBinCount, chunkBinOffset, binCount, binStart, binUnitFirst, binList;
-    DevBuf unitTileCount, tileCount, tileStart, tileList;
-    DevBuf binStage, binStageCount;     // bin pairs recorded by the count pass (DrawDev::binStage)
-    DevBuf tileStage, tileStageCount;   // tile pairs recorded by the coarse count pass (DrawDev::tileStage)
+    DevBuf triSubtris, triHeader, triData, pairs, pairCount, mediumItems, largeItems, binWork, binCount;
+    DevBuf itemPairs, itemBlockCount, tileWork, tileItems, tileCursor, tileCount, tileStart, tileList;
     // Per-draw block, written by one copy per draw: the zeroed Counters and one
     // fine-stage tile counter per pipe group, then the instance descriptors
     // and the prefix arrays.
@@ -150,6 +152,9 @@ struct cr_context {
     // Last draw.
     cr_counters last{};
     cr_queue_layout lastLayout{};
+    int lastWidth = 0, lastHeight = 0;   // viewport and samples of the last single draw
+    int lastSamplesLog2 = 0;
+    int64_t lastTris = 0;
 };
 
 namespace {
@@ -265,11 +270,9 @@ cr_status cr_create(cr_context** out) {
 cr_status cr_destroy(cr_context* ctx) {
     if (!ctx) return CR_ERR_INVALID_ARGUMENT;
     cudaDeviceSynchronize();
-    DevBuf* bufs[] = {&ctx->triSubtris, &ctx->triHeader, &ctx->triData, &ctx->chunkBinCount, &ctx->chunkBinOffset,
-                      &ctx->binCount,
-                      &ctx->binStart, &ctx->binUnitFirst, &ctx->binList, &ctx->unitTileCount,
-                      &ctx->tileCount, &ctx->tileStart, &ctx->tileList, &ctx->binStage, &ctx->binStageCount,
-                      &ctx->tileStage, &ctx->tileStageCount, &ctx->drawBlock};
+    DevBuf* bufs[] = {&ctx->triSubtris, &ctx->triHeader, &ctx->triData,    &ctx->pairs, &ctx->pairCount, &ctx->mediumItems, &ctx->itemPairs, &ctx->itemBlockCount,
+                      &ctx->largeItems, &ctx->binWork,   &ctx->binCount,   &ctx->tileWork,  &ctx->tileItems, &ctx->tileCursor,
+                      &ctx->tileCount,  &ctx->tileStart, &ctx->tileList,   &ctx->drawBlock};
     for (DevBuf* b : bufs) b->release();
     for (int i = 0; i < cr_context::kStageSlots; i++) {
         if (ctx->hostStage[i]) cudaFreeHost(ctx->hostStage[i]);
@@ -367,6 +370,54 @@ cr_status cr_read_setup_output(cr_context* ctx, uint8_t* tri_subtris, uint32_t* 
     return CR_OK;
 }
 
+}  // extern "C"
+
+namespace {
+// The bin lists of the last single draw, from its setup output: the draw
+// counts each bin's entries (they size and report the bin queue) but builds
+// the tile lists without writing bin lists, so this inspection call does.
+cr_status readBinLists(cr_context* ctx, size_t numBins, int64_t numEntries, int32_t* binStart, uint32_t* binList) {
+    const int64_t tris = ctx->lastTris, slots = tris + ctx->hostCounters->extraSubtris;
+    std::vector<uint8_t> sub((size_t)tris);
+    std::vector<uint4> hdr((size_t)slots);
+    if (tris > 0) {
+        CR_CUDA(cudaMemcpy(sub.data(), ctx->triSubtris.ptr, (size_t)tris, cudaMemcpyDeviceToHost), "cudaMemcpy");
+        CR_CUDA(cudaMemcpy(hdr.data(), ctx->triHeader.ptr, (size_t)slots * 16, cudaMemcpyDeviceToHost), "cudaMemcpy");
+    }
+    const cr_queue_layout& l = ctx->lastLayout;
+    const int w = ctx->lastWidth, h = ctx->lastHeight;
+    std::vector<std::vector<uint32_t>> lists(numBins);
+    int64_t total = 0;
+    for (int64_t t = 0; t < tris; t++) {
+        for (int s = 0; s < sub[(size_t)t]; s++) {
+            const bool own = sub[(size_t)t] == 1;
+            const TriGeom g = geomFromHeader(hdr[own ? (size_t)t : (size_t)hdr[(size_t)t].w + s]);
+            const CellBox b = tileBox(std::min({g.x0, g.x1, g.x2}), std::min({g.y0, g.y1, g.y2}),
+                                      std::max({g.x0, g.x1, g.x2}), std::max({g.y0, g.y1, g.y2}), w, h, l.tiles_x,
+                                      l.tiles_y, ctx->lastSamplesLog2 == 0)
+                                  .coarser(l.bin_log2);
+            for (int y = b.ly; y <= b.hy; y++)
+                for (int x = b.lx; x <= b.hx; x++)
+                    if (b.small() || triTouchesCell(g, x, y, l.bin_log2, w, h)) {
+                        lists[(size_t)y * l.bins_x + x].push_back((uint32_t)t << 3 | (own ? 7u : (uint32_t)s));
+                        total++;
+                    }
+        }
+    }
+    if (total != numEntries)
+        return fail(ctx, CR_ERR_CUDA, "CudaRaster: %lld bin entries read back, %lld counted", (long long)total, (long long)numEntries);
+    int32_t start = 0;
+    for (size_t b = 0; b < numBins; b++) {
+        if (binStart) binStart[b] = start;
+        if (binList) std::copy(lists[b].begin(), lists[b].end(), binList + start);
+        start += (int32_t)lists[b].size();
+    }
+    return CR_OK;
+}
+}  // namespace
+
+extern "C" {
+
 cr_status cr_read_queue_output(cr_context* ctx, int32_t* bin_start, int32_t* bin_count, uint32_t* bin_list,
                                int64_t max_bin_entries, int32_t* tile_start, int32_t* tile_count,
                                uint32_t* tile_list, int64_t max_tile_entries, int64_t* num_bin_entries,
@@ -386,15 +437,27 @@ cr_status cr_read_queue_output(cr_context* ctx, int32_t* bin_start, int32_t* bin
                     (long long)c.bin_entries, (long long)c.tile_entries);
     CR_CUDA(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
     const size_t nb = (size_t)c.num_bins, nt = (size_t)c.num_tiles;
-    if (bin_start) CR_CUDA(cudaMemcpy(bin_start, ctx->binStart.ptr, nb * 4, cudaMemcpyDeviceToHost), "cudaMemcpy");
     if (bin_count) CR_CUDA(cudaMemcpy(bin_count, ctx->binCount.ptr, nb * 4, cudaMemcpyDeviceToHost), "cudaMemcpy");
     if (tile_start) CR_CUDA(cudaMemcpy(tile_start, ctx->tileStart.ptr, nt * 4, cudaMemcpyDeviceToHost), "cudaMemcpy");
     if (tile_count) CR_CUDA(cudaMemcpy(tile_count, ctx->tileCount.ptr, nt * 4, cudaMemcpyDeviceToHost), "cudaMemcpy");
-    if (bin_list && c.bin_entries > 0)
-        CR_CUDA(cudaMemcpy(bin_list, ctx->binList.ptr, (size_t)c.bin_entries * 4, cudaMemcpyDeviceToHost), "cudaMemcpy");
-    if (tile_list && c.tile_entries > 0)
-        CR_CUDA(cudaMemcpy(tile_list, ctx->tileList.ptr, (size_t)c.tile_entries * 4, cudaMemcpyDeviceToHost),
-                "cudaMemcpy");
+    try {
+        if (bin_start || bin_list) {
+            cr_status bs = readBinLists(ctx, nb, c.bin_entries, bin_start, bin_list);
+            if (bs != CR_OK) return bs;
+        }
+        if (tile_list && c.tile_entries > 0) {
+            CR_CUDA(cudaMemcpy(tile_list, ctx->tileList.ptr, (size_t)c.tile_entries * 4, cudaMemcpyDeviceToHost),
+                    "cudaMemcpy");
+            // Pipes that do not depend on the lists' order draw from unordered
+            // ones: the export gives them in submission order.
+            std::vector<int32_t> ts(nt), tc(nt);
+            CR_CUDA(cudaMemcpy(ts.data(), ctx->tileStart.ptr, nt * 4, cudaMemcpyDeviceToHost), "cudaMemcpy");
+            CR_CUDA(cudaMemcpy(tc.data(), ctx->tileCount.ptr, nt * 4, cudaMemcpyDeviceToHost), "cudaMemcpy");
+            for (size_t t = 0; t < nt; t++) std::sort(tile_list + ts[t], tile_list + ts[t] + tc[t]);
+        }
+    } catch (const std::bad_alloc&) {
+        return fail(ctx, CR_ERR_OUT_OF_MEMORY, "CudaRaster: out of host memory reading the queues back");
+    }
     return CR_OK;
 }
 
@@ -479,50 +542,26 @@ cr_status cr_set_capacity(cr_context* ctx, int64_t ms, int64_t mb, int64_t mt) {
 namespace {
 
 // Prefix arrays staged behind the instance descriptors, numInstances + 1
-// entries each: triangles (8 bytes), chunks, bins, tiles.
-constexpr size_t kPrefixBytesPerInstance = 8 + 3 * 4;
+// entries each: triangles (8 bytes), tiles.
+constexpr size_t kPrefixBytesPerInstance = 8 + 4;
 
 struct Plan {
     std::vector<HostInstance> inst;
-    std::vector<int32_t> chunkPrefix, binPrefix, tilePrefix;
+    std::vector<int32_t> tilePrefix;
     std::vector<int64_t> triPrefix;
     struct Group { const PipeDesc* pipe; int instBegin, instEnd; int64_t triBegin, triEnd; int32_t tileBegin, tileEnd; };
     std::vector<Group> groups;
-    int64_t totalTris = 0, chunkCountEntries = 0;
-    int32_t totalBins = 0, totalTiles = 0, totalChunks = 0, maxBins = 0, maxChunkTris = 0;
-    int binLog2 = 4, unitEntries = 0;
+    int64_t totalTris = 0;
+    int32_t totalBins = 0, totalTiles = 0, chunkTris = 0, numChunks = 0;
+    int binLog2 = 4;
     // Fused vertex transform (single draws only).
     const float* model = nullptr;
     int modelStride = 0;
     float mvp[16] = {};
 };
 
-// Coarse units a draw may use. A unit size set by the caller bounds them by
-// the bin capacity; units sized on the device (unitEntries 0, at least 64
-// entries each) are also capped at 8M per-unit tile counters, and the device
-// grows the unit size until the draw's bin entries fit.
-// Bin pairs a chunk may record for the scatter pass: twice its triangles (a
-// chunk of small triangles makes about one bin entry per live triangle), at
-// most 1024; chunks with more are walked again by the scatter pass.
-int binStageCap(const Plan& plan) {
-    const int cap = std::min(2 * plan.maxChunkTris, 1024);
-    return (cap + 31) & ~31;
-}
-
-// Coarse units that record their tile pairs (units are sized on the device
-// to about two per resident coarse warp), and the pairs each may record;
-// later units and fuller ones are walked again by the coarse scatter pass.
-constexpr int kTileStageUnits = 16384;
-constexpr int kTileStageCap = 1024;
-
-int64_t unitCapacity(int64_t maxBinEntries, int unitEntries, int32_t totalBins, int tpb) {
-    if (unitEntries > 0) return maxBinEntries / unitEntries + totalBins + 1;
-    return std::min<int64_t>(maxBinEntries / 64, std::max<int64_t>(4096, (8 << 20) / tpb)) + totalBins + 1;
-}
-
 cr_status buildPlan(cr_context* ctx, const std::vector<HostInstance>& in, Plan& plan) {
     plan.binLog2 = ctx->tuning.bin_log2 > 0 ? ctx->tuning.bin_log2 : 4;
-    plan.unitEntries = std::max(0, ctx->tuning.coarse_unit_entries);   // 0: sized on the device
     // Group instances by pipe, keeping first-seen pipe order (outputs do not depend on it).
     std::vector<const PipeDesc*> order;
     for (const HostInstance& h : in)
@@ -531,19 +570,8 @@ cr_status buildPlan(cr_context* ctx, const std::vector<HostInstance>& in, Plan& 
         for (const HostInstance& h : in)
             if (h.pipe == p) plan.inst.push_back(h);
     const int side = 1 << plan.binLog2;
-    // Bin chunks are taken by warps, in order: about 80 per SM (two per
-    // resident bin warp), of at most 65536 triangles and at least 256 (fewer,
-    // down to 32, for draws under 128K triangles, whose chunks would
-    // otherwise be too few to keep the warps busy), a multiple of 32.
-    int64_t allTris = 0;
-    for (const HostInstance& h : plan.inst) allTris += h.dev.numTris;
-    const int64_t wantChunks = std::max<int64_t>(1, (int64_t)ctx->numSMs * 80);
-    const int64_t floorChunk = std::min<int64_t>(256, std::max<int64_t>(32, allTris / 512));
-    int64_t chunk = std::min<int64_t>(std::max<int64_t>((allTris + wantChunks - 1) / wantChunks, floorChunk), 65536);
-    const int autoChunk = (int)((chunk + 31) & ~(int64_t)31);
     int64_t tri = 0;
-    int32_t bins = 0, tiles = 0, chunks = 0;
-    int64_t countBase = 0;
+    int32_t bins = 0, tiles = 0;
     for (size_t i = 0; i < plan.inst.size(); i++) {
         InstanceDev& d = plan.inst[i].dev;
         d.widthTiles = (d.width + 7) >> 3;
@@ -553,38 +581,27 @@ cr_status buildPlan(cr_context* ctx, const std::vector<HostInstance>& in, Plan& 
         int nb = d.widthBins * d.heightBins;
         if (nb > 1024)
             return fail(ctx, CR_ERR_CAPACITY, "CudaRaster: %d bins exceed 1024; use a larger bin_log2", nb);
-        plan.maxBins = std::max(plan.maxBins, nb);
         d.rowWords = (int64_t)(d.widthTiles * 8) << d.samplesLog2;
         d.triBase = tri;
         d.binBase = bins;
         d.tileBase = tiles;
-        int chunkTris = ctx->tuning.bin_chunk_tris;
-        if (chunkTris <= 0) chunkTris = autoChunk;
-        d.chunkTris = chunkTris;
-        d.numChunks = (d.numTris + chunkTris - 1) / chunkTris;
-        plan.maxChunkTris = std::max(plan.maxChunkTris, chunkTris);
-        d.chunkBase = chunks;
-        d.chunkCountBase = countBase;
-        countBase += (int64_t)d.numChunks * nb;
         tri += d.numTris;
         bins += nb;
         tiles += d.widthTiles * d.heightTiles;
-        chunks += d.numChunks;
         if (tri > CR_MAX_TRIANGLES) return fail(ctx, CR_ERR_CAPACITY, "CudaRaster: CR_MAXSUBTRIS_SIZE exceeded!");
     }
     plan.totalTris = tri;
+    plan.chunkTris = kMinChunkTris;
+    const int64_t wantChunk = ctx->tuning.bin_chunk_tris > 0 ? ctx->tuning.bin_chunk_tris
+                                                             : tri / ((int64_t)ctx->numSMs * kChunksPerSM) + 1;
+    while (plan.chunkTris < kMaxChunkTris && plan.chunkTris < wantChunk) plan.chunkTris *= 2;
+    plan.numChunks = (int32_t)((tri + plan.chunkTris - 1) / plan.chunkTris);
     plan.totalBins = bins;
     plan.totalTiles = tiles;
-    plan.totalChunks = chunks;
-    plan.chunkCountEntries = countBase;
     for (const HostInstance& h : plan.inst) {
-        plan.chunkPrefix.push_back(h.dev.chunkBase);
-        plan.binPrefix.push_back(h.dev.binBase);
         plan.tilePrefix.push_back(h.dev.tileBase);
         plan.triPrefix.push_back(h.dev.triBase);
     }
-    plan.chunkPrefix.push_back(chunks);
-    plan.binPrefix.push_back(bins);
     plan.tilePrefix.push_back(tiles);
     plan.triPrefix.push_back(tri);
     for (size_t i = 0; i < plan.inst.size();) {
@@ -615,6 +632,12 @@ size_t drawBlockBytes(const Plan& plan) {
            kPrefixBytesPerInstance * (plan.inst.size() + 1) + 64;
 }
 
+// Blocks of item pair records: every tile entry may come from an item, and each
+// warp of the item kernel may leave one block partly filled.
+int64_t itemBlocks(const cr_context* ctx, int64_t maxTileEntries) {
+    return (maxTileEntries + kItemBlock - 1) / kItemBlock + (int64_t)ctx->numSMs * kItemWarpsPerSM;
+}
+
 cr_status ensureCapacity(cr_context* ctx, const Plan& plan) {
     int64_t T = plan.totalTris;
     // Initial sizes in the spirit of CudaRaster.cpp:263-275 (subtriangle
@@ -630,27 +653,24 @@ cr_status ensureCapacity(cr_context* ctx, const Plan& plan) {
         ctx->maxBinEntries = std::max<int64_t>(ctx->maxBinEntries, 2 * T + 65536);
         ctx->maxTileEntries = std::max<int64_t>(ctx->maxTileEntries, 4 * T + 65536);
     }
-    const int tpb = 1 << (2 * plan.binLog2);
-    const int64_t maxUnits = unitCapacity(ctx->maxBinEntries, plan.unitEntries, plan.totalBins, tpb);
-    CR_CUDA(ctx->triSubtris.ensure((size_t)std::max<int64_t>(T, 1)), "cudaMalloc");
+    CR_CUDA(ctx->triSubtris.ensure((size_t)T + 4), "cudaMalloc");
     CR_CUDA(ctx->triHeader.ensure((size_t)ctx->maxSubtris * 16), "cudaMalloc");
     CR_CUDA(ctx->triData.ensure((size_t)ctx->maxSubtris * 64), "cudaMalloc");
-    CR_CUDA(ctx->chunkBinCount.ensureZeroed((size_t)std::max<int64_t>(plan.chunkCountEntries, 1) * 4), "cudaMalloc");
-    CR_CUDA(ctx->chunkBinOffset.ensure((size_t)std::max<int64_t>(plan.chunkCountEntries, 1) * 4), "cudaMalloc");
+    CR_CUDA(ctx->pairs.ensure((size_t)std::max(plan.numChunks, 1) * 2 * plan.chunkTris * 8), "cudaMalloc");
+    CR_CUDA(ctx->pairCount.ensure((size_t)std::max(plan.numChunks, 1) * 4), "cudaMalloc");
+    CR_CUDA(ctx->mediumItems.ensure((size_t)std::max<int64_t>(T, 1) * 4), "cudaMalloc");
+    CR_CUDA(ctx->largeItems.ensure((size_t)ctx->maxSubtris * 4), "cudaMalloc");
+    CR_CUDA(ctx->binWork.ensureZeroed((size_t)plan.totalBins * kBinWorkStride * 4), "cudaMalloc");
     CR_CUDA(ctx->binCount.ensure((size_t)plan.totalBins * 4), "cudaMalloc");
-    CR_CUDA(ctx->binStart.ensure((size_t)plan.totalBins * 4), "cudaMalloc");
-    CR_CUDA(ctx->binUnitFirst.ensure((size_t)plan.totalBins * 4), "cudaMalloc");
-    CR_CUDA(ctx->binList.ensure((size_t)ctx->maxBinEntries * 4), "cudaMalloc");
-    CR_CUDA(ctx->unitTileCount.ensure((size_t)maxUnits * tpb * 4), "cudaMalloc");
+    CR_CUDA(ctx->tileWork.ensureZeroed(((size_t)plan.totalTiles << tileWorkLog2(plan.totalTiles)) * 4), "cudaMalloc");
+    CR_CUDA(ctx->tileItems.ensureZeroed((size_t)plan.totalTiles * 4), "cudaMalloc");
+    CR_CUDA(ctx->tileCursor.ensure((size_t)plan.totalTiles * 4), "cudaMalloc");
+    const int64_t blocks = itemBlocks(ctx, ctx->maxTileEntries);
+    CR_CUDA(ctx->itemPairs.ensure((size_t)blocks * kItemBlock * 8), "cudaMalloc");
+    CR_CUDA(ctx->itemBlockCount.ensure((size_t)blocks * 4), "cudaMalloc");
     CR_CUDA(ctx->tileCount.ensure((size_t)plan.totalTiles * 4), "cudaMalloc");
     CR_CUDA(ctx->tileStart.ensure((size_t)plan.totalTiles * 4), "cudaMalloc");
     CR_CUDA(ctx->tileList.ensure((size_t)ctx->maxTileEntries * 4), "cudaMalloc");
-    const int stageCap = binStageCap(plan);
-    CR_CUDA(ctx->binStage.ensure((size_t)std::max(plan.totalChunks, 1) * stageCap * 8), "cudaMalloc");
-    CR_CUDA(ctx->binStageCount.ensure((size_t)std::max(plan.totalChunks, 1) * 4), "cudaMalloc");
-    const int64_t stageUnits = std::min<int64_t>(maxUnits, kTileStageUnits);
-    CR_CUDA(ctx->tileStage.ensure((size_t)stageUnits * kTileStageCap * 8), "cudaMalloc");
-    CR_CUDA(ctx->tileStageCount.ensure((size_t)stageUnits * 4), "cudaMalloc");
     const size_t stage = drawBlockBytes(plan);
     CR_CUDA(ctx->drawBlock.ensure(stage), "cudaMalloc");
     if (stage > ctx->hostStageBytes) {
@@ -679,8 +699,6 @@ DrawDev makeDrawDev(cr_context* ctx, const Plan& plan) {
     d.binLog2 = plan.binLog2;
     d.totalBins = plan.totalBins;
     d.totalTiles = plan.totalTiles;
-    d.totalChunks = plan.totalChunks;
-    d.unitEntries = plan.unitEntries;
     d.totalTris = plan.totalTris;
     d.model = plan.model;
     d.modelStride = plan.modelStride;
@@ -690,17 +708,23 @@ DrawDev makeDrawDev(cr_context* ctx, const Plan& plan) {
     d.triHeader = ctx->triHeader.as<uint4>();
     d.triData = ctx->triData.as<uint4>();
     d.maxSubtris = ctx->maxSubtris;
-    d.chunkBinCount = ctx->chunkBinCount.as<int32_t>();
-    d.chunkBinOffset = ctx->chunkBinOffset.as<int32_t>();
-    d.maxBins = plan.maxBins;
+    d.pairs = ctx->pairs.as<U64>();
+    d.pairCount = ctx->pairCount.as<int32_t>();
+    d.chunkTris = plan.chunkTris;
+    d.numChunks = plan.numChunks;
+    d.mediumItems = ctx->mediumItems.as<uint32_t>();
+    d.largeItems = ctx->largeItems.as<uint32_t>();
     d.fineSelfPixels = ctx->tuning.fine_self_pixels;
+    d.binWork = ctx->binWork.as<int32_t>();
     d.binCount = ctx->binCount.as<int32_t>();
-    d.binStart = ctx->binStart.as<int32_t>();
-    d.binUnitFirst = ctx->binUnitFirst.as<int32_t>();
-    d.binList = ctx->binList.as<uint32_t>();
     d.maxBinEntries = ctx->maxBinEntries;
-    d.unitTileCount = ctx->unitTileCount.as<int32_t>();
-    d.maxUnits = unitCapacity(ctx->maxBinEntries, plan.unitEntries, plan.totalBins, 1 << (2 * plan.binLog2));
+    d.tileWork = ctx->tileWork.as<int32_t>();
+    d.tileWorkLog2 = tileWorkLog2(plan.totalTiles);
+    d.tileItems = ctx->tileItems.as<int32_t>();
+    d.tileCursor = ctx->tileCursor.as<int32_t>();
+    d.itemPairs = ctx->itemPairs.as<U64>();
+    d.itemBlockCount = ctx->itemBlockCount.as<int32_t>();
+    d.maxItemBlocks = (int32_t)itemBlocks(ctx, ctx->maxTileEntries);
     d.tileCount = ctx->tileCount.as<int32_t>();
     d.tileStart = ctx->tileStart.as<int32_t>();
     d.tileList = ctx->tileList.as<uint32_t>();
@@ -708,23 +732,14 @@ DrawDev makeDrawDev(cr_context* ctx, const Plan& plan) {
     char* pref = ctx->drawBlock.as<char>() + cb + sizeof(InstanceDev) * plan.inst.size();
     size_t n1 = plan.inst.size() + 1;
     d.triPrefix = (const int64_t*)pref;
-    d.chunkPrefix = (const int32_t*)(pref + 8 * n1);
-    d.binPrefix = d.chunkPrefix + n1;
-    d.tilePrefix = d.binPrefix + n1;
+    d.tilePrefix = (const int32_t*)(pref + 8 * n1);
     d.counters = ctx->drawBlock.as<Counters>();
     d.fineTileCounter = (int32_t*)(ctx->drawBlock.as<char>() + sizeof(Counters));
-    d.binStage = ctx->binStage.as<U64>();
-    d.binStageCount = ctx->binStageCount.as<int32_t>();
-    d.binStageCap = binStageCap(plan);
-    d.tileStage = ctx->tileStage.as<U64>();
-    d.tileStageCount = ctx->tileStageCount.as<int32_t>();
-    d.tileStageCap = kTileStageCap;
-    d.tileStageUnits = (int32_t)std::min<int64_t>(d.maxUnits, kTileStageUnits);
     return d;
 }
 
 static_assert(sizeof(InstanceDev) % 8 == 0, "the prefix arrays follow the descriptors with 8-byte alignment");
-static_assert(offsetof(Counters, coarseWork) == 6 * sizeof(int32_t) && sizeof(Counters) >= 8 * sizeof(int32_t),
+static_assert(offsetof(Counters, largeItems) == 6 * sizeof(int32_t) && sizeof(Counters) >= 8 * sizeof(int32_t),
               "cr_queue_counts exports the first 8 words of Counters");
 
 // A draw's block (zeroed counters, instance descriptors, prefix arrays) as a
@@ -780,9 +795,7 @@ cr_status launchDrawWith(cr_context* ctx, const Plan& plan, cudaStream_t stream,
     for (size_t i = 0; i < plan.inst.size(); i++) memcpy(hs + i * sizeof(InstanceDev), &plan.inst[i].dev, sizeof(InstanceDev));
     char* hp = hs + instBytes;
     memcpy(hp, plan.triPrefix.data(), 8 * n1);
-    memcpy(hp + 8 * n1, plan.chunkPrefix.data(), 4 * n1);
-    memcpy(hp + 12 * n1, plan.binPrefix.data(), 4 * n1);
-    memcpy(hp + 16 * n1, plan.tilePrefix.data(), 4 * n1);
+    memcpy(hp + 8 * n1, plan.tilePrefix.data(), 4 * n1);
     const size_t blockBytes = cb + instBytes + kPrefixBytesPerInstance * n1;
     writeKernel = writeKernel && !capturing(stream);
     if (writeKernel && blockBytes <= 1024)
@@ -797,7 +810,10 @@ cr_status launchDrawWith(cr_context* ctx, const Plan& plan, cudaStream_t stream,
     for (const Plan::Group& g : plan.groups)
         CR_CUDA(g.pipe->launchSetup(d, g.instBegin, g.instEnd, g.triBegin, g.triEnd, stream), "setup launch");
     if (events) CR_CUDA(cudaEventRecord(ctx->ev[1], stream), "cudaEventRecord");
-    CR_CUDA(launchBinning(d, plan.maxBins, ctx->numSMs, stream, events ? ctx->ev[2] : nullptr), "bin/coarse launch");
+    CR_CUDA(launchBinning(d, ctx->numSMs, stream, events ? ctx->ev[2] : nullptr), "bin/coarse launch");
+    for (const Plan::Group& g : plan.groups)
+        if (g.pipe->needsOrder)
+            CR_CUDA(launchListSort(d, g.tileBegin, g.tileEnd, ctx->numSMs, stream), "list sort launch");
     if (events) CR_CUDA(cudaEventRecord(ctx->ev[3], stream), "cudaEventRecord");
     // The first fine launch that has tiles writes the counters into the
     // pinned host buffer (its device address); without one, a copy follows.
@@ -861,6 +877,10 @@ cr_status drawPlan(cr_context* ctx, const Plan& plan, cudaStream_t stream, bool 
     const InstanceDev& first = plan.inst[0].dev;
     ctx->lastLayout = cr_queue_layout{first.widthBins, first.heightBins, first.widthTiles, first.heightTiles,
                                       plan.binLog2, plan.totalBins, plan.totalTiles, (int32_t)plan.inst.size()};
+    ctx->lastWidth = first.width;
+    ctx->lastHeight = first.height;
+    ctx->lastSamplesLog2 = first.samplesLog2;
+    ctx->lastTris = plan.totalTris;
     ctx->last.num_bins = plan.totalBins;
     ctx->last.num_tiles = plan.totalTiles;
     for (int reruns = 0;; reruns++) {

@@ -30,6 +30,7 @@
 #include "cudaraster/detail/device.cuh"
 #include "cudaraster/detail/pipe_registry.h"
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstddef>
 #include <cstdio>
@@ -37,7 +38,8 @@
 #include <mutex>
 
 namespace cr {
-cudaError_t launchBinning(const DrawDev& d, int maxBins, int numSMs, cudaStream_t stream, cudaEvent_t evCoarse);
+cudaError_t launchBinning(const DrawDev& d, int numSMs, cudaStream_t stream, cudaEvent_t evCoarse);
+cudaError_t launchListSort(const DrawDev& d, int32_t tileBegin, int32_t tileEnd, int numSMs, cudaStream_t stream);
 }
 namespace cr {
 const PipeDesc* findRegisteredPipe(const char* name);
@@ -50,16 +52,18 @@ namespace {
 constexpr int kStaticMaxTris = 65536;
 constexpr int kStaticMaxViewport = 1024;
 constexpr int kStaticBinLog2 = 4;
-constexpr int kStaticChunkTris = 1024;
-constexpr int kStaticUnitEntries = 512;
 constexpr int kStaticMaxTiles = (kStaticMaxViewport / 8) * (kStaticMaxViewport / 8);
 constexpr int kStaticMaxBins = (kStaticMaxViewport / 128) * (kStaticMaxViewport / 128);
+constexpr int kStaticChunkTris = kMinChunkTris;
 constexpr int kStaticMaxChunks = kStaticMaxTris / kStaticChunkTris;
 constexpr int64_t kStaticMaxSubtris = kStaticMaxTris + 16384;
 constexpr int64_t kStaticMaxBinEntries = 4 * kStaticMaxTris;
 constexpr int64_t kStaticMaxTileEntries = 16 * kStaticMaxTris;
-constexpr int64_t kStaticMaxUnits = kStaticMaxBinEntries / kStaticUnitEntries + kStaticMaxBins + 1;
-constexpr int kStaticTilesPerBin = 1 << (2 * kStaticBinLog2);
+// The list stages of a static draw run on at most this many SMs' worth of
+// CTAs: each warp of the item kernel may leave a block of records partly
+// filled.
+constexpr int kStaticSMs = 16;
+constexpr int kStaticMaxItemBlocks = kStaticMaxTileEntries / kItemBlock + kStaticSMs * kItemWarpsPerSM;
 
 constexpr size_t alignUp(size_t v) { return (v + 255) & ~(size_t)255; }
 
@@ -69,23 +73,27 @@ constexpr size_t kOffFine = alignUp(kOffCounters + sizeof(Counters));
 constexpr size_t kOffInst = alignUp(kOffFine + sizeof(int32_t));
 constexpr size_t kOffPrefix = alignUp(kOffInst + sizeof(InstanceDev));
 constexpr size_t kOffSubtris = alignUp(kOffPrefix + 64);
-constexpr size_t kOffHeader = alignUp(kOffSubtris + kStaticMaxTris);
+constexpr size_t kOffHeader = alignUp(kOffSubtris + kStaticMaxTris + 4);
 constexpr size_t kOffData = alignUp(kOffHeader + 16 * kStaticMaxSubtris);
-constexpr size_t kOffChunkCount = alignUp(kOffData + 64 * kStaticMaxSubtris);
-constexpr size_t kOffChunkOffset = alignUp(kOffChunkCount + 4 * (size_t)kStaticMaxChunks * kStaticMaxBins);
-constexpr size_t kOffBinCount = alignUp(kOffChunkOffset + 4 * (size_t)kStaticMaxChunks * kStaticMaxBins);
-constexpr size_t kOffBinStart = alignUp(kOffBinCount + 4 * kStaticMaxBins);
-constexpr size_t kOffBinUnitFirst = alignUp(kOffBinStart + 4 * kStaticMaxBins);
-constexpr size_t kOffBinList = alignUp(kOffBinUnitFirst + 4 * kStaticMaxBins);
-constexpr size_t kOffUnitTileCount = alignUp(kOffBinList + 4 * kStaticMaxBinEntries);
-constexpr size_t kOffTileCount = alignUp(kOffUnitTileCount + 4 * (size_t)kStaticMaxUnits * kStaticTilesPerBin);
+constexpr size_t kOffPairs = alignUp(kOffData + 64 * kStaticMaxSubtris);
+constexpr size_t kOffPairCount = alignUp(kOffPairs + 8 * 2 * (size_t)kStaticMaxTris);
+constexpr size_t kOffMediumItems = alignUp(kOffPairCount + 4 * kStaticMaxChunks);
+constexpr size_t kOffLargeItems = alignUp(kOffMediumItems + 4 * kStaticMaxTris);
+constexpr size_t kOffBinWork = alignUp(kOffLargeItems + 4 * kStaticMaxSubtris);
+constexpr size_t kOffBinCount = alignUp(kOffBinWork + 4 * kBinWorkStride * kStaticMaxBins);
+constexpr size_t kOffTileWork = alignUp(kOffBinCount + 4 * kStaticMaxBins);
+constexpr size_t kOffTileItems = alignUp(kOffTileWork + ((size_t)4 << tileWorkLog2(kStaticMaxTiles)) * kStaticMaxTiles);
+constexpr size_t kOffTileCursor = alignUp(kOffTileItems + 4 * kStaticMaxTiles);
+constexpr size_t kOffTileCount = alignUp(kOffTileCursor + 4 * kStaticMaxTiles);
 constexpr size_t kOffTileStart = alignUp(kOffTileCount + 4 * kStaticMaxTiles);
 constexpr size_t kOffTileList = alignUp(kOffTileStart + 4 * kStaticMaxTiles);
-constexpr size_t kStaticScratchBytes = alignUp(kOffTileList + 4 * kStaticMaxTileEntries);
+constexpr size_t kOffItemPairs = alignUp(kOffTileList + 4 * kStaticMaxTileEntries);
+constexpr size_t kOffItemBlockCount = alignUp(kOffItemPairs + 8 * kItemBlock * (size_t)kStaticMaxItemBlocks);
+constexpr size_t kStaticScratchBytes = alignUp(kOffItemBlockCount + 4 * kStaticMaxItemBlocks);
 
 }  // namespace
 
-// The scratch array (about 13 MiB, held by every GPU that loads the library).
+// The scratch array (about 25 MiB, held by every GPU that loads the library).
 static __device__ __align__(256) unsigned char g_staticScratch[kStaticScratchBytes];
 
 namespace {
@@ -184,17 +192,15 @@ extern "C" cr_status cr_draw_triangles_static(const char* pipe_name, void* color
     in.widthBins = (in.widthTiles + side - 1) / side;
     in.heightBins = (in.heightTiles + side - 1) / side;
     in.rowWords = (int64_t)(in.widthTiles * 8) << samplesLog2;
-    in.chunkTris = kStaticChunkTris;
-    in.numChunks = (num_tris + kStaticChunkTris - 1) / kStaticChunkTris;
     const int numBins = in.widthBins * in.heightBins;
     const int numTiles = in.widthTiles * in.heightTiles;
 
-    // Descriptor block: instance, then prefixes (tri int64[2], chunk/bin/tile int32[2] each).
+    // Descriptor block: instance, then prefixes (tri int64[2], tile int32[2]).
     struct Prefixes {
         int64_t tri[2];
-        int32_t chunk[2], bin[2], tile[2];
+        int32_t tile[2];
     };
-    Prefixes pref = {{0, num_tris}, {0, in.numChunks}, {0, numBins}, {0, numTiles}};
+    Prefixes pref = {{0, num_tris}, {0, numTiles}};
     static_assert(sizeof(pref) <= 64, "prefix block");
 
     DrawDev d;
@@ -204,34 +210,36 @@ extern "C" cr_status cr_draw_triangles_static(const char* pipe_name, void* color
     d.binLog2 = kStaticBinLog2;
     d.totalBins = numBins;
     d.totalTiles = numTiles;
-    d.totalChunks = in.numChunks;
-    d.unitEntries = kStaticUnitEntries;
     d.totalTris = num_tris;
     d.triSubtris = scratch + kOffSubtris;
     d.triHeader = (uint4*)(scratch + kOffHeader);
     d.triData = (uint4*)(scratch + kOffData);
     d.maxSubtris = kStaticMaxSubtris;
-    d.chunkBinCount = (int32_t*)(scratch + kOffChunkCount);   // zero at load; each bin scan clears it again
-    d.chunkBinOffset = (int32_t*)(scratch + kOffChunkOffset);
-    d.maxBins = numBins;
+    d.pairs = (U64*)(scratch + kOffPairs);
+    d.pairCount = (int32_t*)(scratch + kOffPairCount);
+    d.chunkTris = kStaticChunkTris;
+    d.numChunks = (num_tris + kStaticChunkTris - 1) / kStaticChunkTris;
+    d.mediumItems = (uint32_t*)(scratch + kOffMediumItems);
+    d.largeItems = (uint32_t*)(scratch + kOffLargeItems);
     d.fineSelfPixels = 0;
     d.model = nullptr;
     d.modelStride = 0;
     d.modelVec4 = 0;
+    d.binWork = (int32_t*)(scratch + kOffBinWork);     // zero at load; each list scan clears it again
     d.binCount = (int32_t*)(scratch + kOffBinCount);
-    d.binStart = (int32_t*)(scratch + kOffBinStart);
-    d.binUnitFirst = (int32_t*)(scratch + kOffBinUnitFirst);
-    d.binList = (uint32_t*)(scratch + kOffBinList);
     d.maxBinEntries = kStaticMaxBinEntries;
-    d.unitTileCount = (int32_t*)(scratch + kOffUnitTileCount);
-    d.maxUnits = kStaticMaxUnits;
+    d.tileWork = (int32_t*)(scratch + kOffTileWork);   // likewise
+    d.tileWorkLog2 = tileWorkLog2(numTiles);
+    d.tileItems = (int32_t*)(scratch + kOffTileItems);
+    d.tileCursor = (int32_t*)(scratch + kOffTileCursor);
+    d.itemPairs = (U64*)(scratch + kOffItemPairs);
+    d.itemBlockCount = (int32_t*)(scratch + kOffItemBlockCount);
+    d.maxItemBlocks = kStaticMaxItemBlocks;
     d.tileCount = (int32_t*)(scratch + kOffTileCount);
     d.tileStart = (int32_t*)(scratch + kOffTileStart);
     d.tileList = (uint32_t*)(scratch + kOffTileList);
     d.maxTileEntries = kStaticMaxTileEntries;
     d.triPrefix = (const int64_t*)(scratch + kOffPrefix);
-    d.chunkPrefix = (const int32_t*)(scratch + kOffPrefix + offsetof(Prefixes, chunk));
-    d.binPrefix = (const int32_t*)(scratch + kOffPrefix + offsetof(Prefixes, bin));
     d.tilePrefix = (const int32_t*)(scratch + kOffPrefix + offsetof(Prefixes, tile));
     d.counters = (Counters*)(scratch + kOffCounters);
     d.fineTileCounter = (int32_t*)(scratch + kOffFine);
@@ -250,7 +258,8 @@ extern "C" cr_status cr_draw_triangles_static(const char* pipe_name, void* color
     CR_STATIC_CUDA(cudaMemsetAsync(scratch + kOffCounters, 0, kOffInst - kOffCounters, s));
 
     CR_STATIC_CUDA(pipe->launchSetup(d, 0, 1, 0, num_tris, s));
-    CR_STATIC_CUDA(launchBinning(d, numBins, numSMs, s, nullptr));
+    CR_STATIC_CUDA(launchBinning(d, std::min(numSMs, kStaticSMs), s, nullptr));
+    if (pipe->needsOrder) CR_STATIC_CUDA(launchListSort(d, 0, numTiles, numSMs, s));
     const int warps = 8;
     CR_STATIC_CUDA(pipe->launchFine(d, 0, 0, numTiles, warps, pipe->fineOccupancy(warps), numSMs, s));
 

@@ -305,7 +305,7 @@ class QueuePredictor:
     def counters_of(self, frame: int) -> np.ndarray:
         """The 8 device counters of a stepped frame (extra subtriangles, bin
         entries, coarse units, tile entries, fine tiles, overflow flags, and
-        the two coarse work counters)."""
+        the coarse stage's large and huge items)."""
         return self._host[frame % self.ring][4:].view(np.int32)
 
     # ---------------------------------------------------------------- sizing

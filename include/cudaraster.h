@@ -82,7 +82,8 @@ typedef struct cr_counters {
     int64_t num_subtris;          /* subtriangle slots used (num_tris + clip extras)  */
     int64_t bin_entries;          /* (bin, subtriangle) list entries                  */
     int64_t tile_entries;         /* (tile, subtriangle) list entries                 */
-    int64_t coarse_units;         /* coarse work units                                */
+    int64_t coarse_units;         /* coarse work units: groups or slices of the       */
+                                  /* subtriangles that cover more than 2x2 tiles      */
     int64_t max_subtris;
     int64_t max_bin_entries;
     int64_t max_tile_entries;
@@ -117,8 +118,9 @@ typedef struct cr_debug_params {
  * Any value <= 0 keeps the default. Output bits do not depend on them. */
 typedef struct cr_tuning {
     int32_t bin_log2;             /* tiles per bin side, log2: 3, 4 (default) or 5    */
-    int32_t bin_chunk_tris;       /* triangles per bin-stage work chunk               */
-    int32_t coarse_unit_entries;  /* bin entries per coarse work unit                 */
+    int32_t bin_chunk_tris;       /* triangles per bin-stage work chunk (taken as the */
+                                  /* power of two from 128 to 512 next above)         */
+    int32_t coarse_unit_entries;  /* accepted; the coarse stage sizes its own units   */
     int32_t fine_warps;           /* warps per fine-raster CTA                        */
     int32_t fine_ctas_per_sm;     /* resident fine CTAs per SM                        */
     int32_t fine_self_pixels;     /* fine stage: triangles whose pixel box in a tile  */
@@ -243,7 +245,7 @@ cr_status cr_batch_graph_destroy(cr_batch_graph* graph);
  * that owns a fixed memory budget, a real-time loop where cudaMalloc would
  * stall the frame, a plugin that only receives device pointers): no context,
  * no cudaMalloc/cudaFree, no pinned host buffers. The intermediate queues
- * live in one static array of about 13 MiB compiled into this library, held
+ * live in one static array of about 25 MiB compiled into this library, held
  * by every GPU that loads it until the process exits, and shared by every
  * call: calls that overlap on the GPU race, so order them on one stream.
  * Limits: num_tris <= 65536, width and height <= 1024, fixed queue sizes;
@@ -382,8 +384,8 @@ cr_status cr_get_queue_buffers(cr_context* ctx, const int32_t** bin_counts, cons
 /* Device-to-device copies, ordered on `stream` after the last draw, of its
  * per-bin bin-queue entry counts [num_bins], per-tile tile-queue entry counts
  * [num_tiles] and its 8 device counters (extra subtriangles, bin entries,
- * coarse units, tile entries, fine tiles taken, overflow flags, and the two
- * coarse work counters).
+ * coarse units, tile entries, fine tiles taken, overflow flags, and the
+ * numbers of large and huge items of the coarse stage).
  * Any of the three pointers may be NULL. After an overflow the counts of the
  * overflowing stage and later ones are incomplete. */
 cr_status cr_queue_counts(cr_context* ctx, int32_t* bin_counts, int32_t num_bins, int32_t* tile_counts,

@@ -82,6 +82,7 @@ struct PipeImpl {
         p.vertexStructSize = (int32_t)sizeof(V);
         p.renderModeFlags = F;
         p.profilingMode = CR_PROFILING_MODE;
+        p.needsOrder = FineTraits<FS, BS, S, F>::kVisibility ? 0 : 1;
         p.launchSetup = &launchSetup;
         p.launchFine = &launchFine;
         p.fineOccupancy = &fineOccupancy;

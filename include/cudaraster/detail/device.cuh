@@ -69,25 +69,57 @@ struct InstanceDev {
     S64 triBase;              // first triangle slot of this instance
     S32 binBase;              // first global bin id
     S32 tileBase;             // first global tile id
-    S32 chunkBase;            // first global bin-stage chunk
-    S32 numChunks;
-    S64 chunkCountBase;       // first entry of this instance in chunkBinCount / chunkBinOffset
-    S32 chunkTris;            // triangles per chunk
     S32 pipeGroup;            // index of the pipe this instance renders with
+    S32 pad;
 };
 
 struct Counters {
     S32 extraSubtris;         // subtriangle slots allocated past the triangle slots
     S32 binEntries;           // total bin list entries
-    S32 numUnits;             // coarse work units
+    S32 numUnits;             // coarse work units (slices of the large items)
     S32 tileEntries;          // total tile list entries
     S32 fineTile;             // fine-stage work counter
     S32 overflow;             // kOverflow* bits
-    S32 coarseWork[2];        // coarse count / scatter unit counters (dynamic unit assignment)
-    S32 binWork[2];           // bin count / scatter chunk counters (dynamic chunk assignment)
-    S32 binsDone;             // bin-scan CTAs finished (the last one plans the coarse units)
-    S32 unitEntries;          // bin entries per coarse unit, as planned for this draw
+    S32 largeItems[2];        // large and huge items queued by the pair stage
+    S32 mediumItems;          // medium items
+    S32 chunkWork;            // pair-stage chunk counter (dynamic chunk assignment)
+    S32 itemWarps;            // warps of the item kernel: blocks of item pair records that are theirs from the start
+    S32 itemBlocks;           // blocks taken beyond those
 };
+// Item pair records come in blocks of this many, each filled by one warp.
+constexpr int kItemBlock = 256;
+constexpr int kItemWarpsPerSM = 40;   // resident warps of the item kernel (its grid)
+
+// Subtriangles by the size of their tile box, as the pair stage sorts them.
+// Those in at most 2x2 tiles become (tile, triangle) pair records at once. The
+// others are queued as items: boxes of at most kMediumCells tiles (many to a
+// warp), of at most kHugeCells (up to four warps to one), and larger (many).
+constexpr int kMediumCells = 64;
+constexpr int kHugeCells = 1024;
+// The pair stage takes the triangles in chunks, one warp each, of 128 to 512:
+// about 160 chunks per SM (five per resident warp) where the draw has the
+// triangles, so that the last ones end close together (8.4M-triangle
+// heightfield: 166 us with 1024, 125 with 512, 117 with 256; the 33.5M-triangle
+// one 222, 175, 195: shorter chunks leave more groups of fewer than 32). A
+// chunk has room for two pair records per triangle; what does not fit is
+// queued.
+constexpr int kMinChunkTris = 128, kMaxChunkTris = 512;
+constexpr int kChunksPerSM = 160;
+// A pair record packs the pair's place in its tile, the global tile and the
+// triangle within the chunk into 27 + 27 + 10 bits; draws with more triangles
+// or tiles queue every subtriangle.
+constexpr S64 kMaxRecord = 1 << 27;
+// Tile counters are a 32-byte sector apart while the pair stage counts, in
+// draws of up to this many tiles: a small viewport's counters would share few
+// lines, and a line passes about 1.4 atomics per ns (random adds over 510
+// counters: 7.6 per ns side by side, 37 a sector apart; over 32,400: 87 and
+// 100).
+constexpr int kMaxSpreadTiles = 1 << 20;
+__host__ __device__ constexpr int tileWorkLog2(S32 totalTiles) { return totalTiles <= kMaxSpreadTiles ? 3 : 0; }
+// Bin counters are a 128-byte line apart while the stages count: random atomic
+// adds over 135 counters ran at 5.6 per ns side by side (five lines) and at 38
+// per ns so.
+constexpr int kBinWorkStride = 32;
 
 // Buffers shared by every instance of a draw.
 struct DrawDev {
@@ -96,11 +128,7 @@ struct DrawDev {
     S32 binLog2;              // tiles per bin side (log2)
     S32 totalBins;
     S32 totalTiles;
-    S32 totalChunks;
-    S32 maxBins;              // bins of the largest instance
     S32 fineSelfPixels;       // fine stage: pixel-box size up to which a lane rasterizes a triangle alone
-    S32 unitEntries;          // bin entries per coarse unit; <= 0: sized on the device from the bin entries
-    S32 unitTarget;           // coarse units wanted when sized on the device (set by the launcher)
     S64 totalTris;
     // Fused vertex transform (single draws): when model is set, setup takes a
     // vertex's clip position as mvp * (model[i], 1) -- the reference's
@@ -113,43 +141,34 @@ struct DrawDev {
     uint8_t* triSubtris;      // [totalTris]
     uint4* triHeader;         // [maxSubtris]
     uint4* triData;           // [maxSubtris * 4]
-    S32* subtriOwner;         // [maxSubtris - totalTris] triangle of an extra slot
     S64 maxSubtris;
+    // pairs
+    U64* pairs;               // [numChunks * 2 * chunkTris] place << 37 | global tile << 10 | triangle of the chunk
+    S32* pairCount;           // [numChunks]
+    S32 chunkTris, numChunks;
+    U32* mediumItems;         // [totalTris] list entries
+    U64* itemPairs;           // [maxItemBlocks * kItemBlock] list entry << 32 | global tile
+    S32* itemBlockCount;      // [maxItemBlocks]
+    S32 maxItemBlocks;
+    U32* largeItems;          // [maxSubtris] list entries: boxes of at most kHugeCells tiles from the front, larger from the back
     // bin
-    S32* chunkBinCount;       // per (bin, chunk): entry count; zero between draws (the bin scan clears it)
-    S32* chunkBinOffset;      // per (chunk, bin): exclusive offset of the chunk in the bin list
+    S32* binWork;             // [totalBins * kBinWorkStride] entries counted so far; zero between draws (the list scan clears it)
     S32* binCount;            // [totalBins]
-    S32* binStart;            // [totalBins]
-    S32* binUnitFirst;        // [totalBins]
-    U32* binList;             // [maxBinEntries]
     S64 maxBinEntries;
-    // coarse
-    S32* unitTileCount;       // [maxUnits << 2*binLog2]: count, then offset
-    S64 maxUnits;
+    // tile lists
+    S32* tileWork;            // [totalTiles << tileWorkLog2] pair records so far; zero between draws (the list scan clears it)
+    S32 tileWorkLog2;         // spacing of the counters in words (log2)
+    S32* tileItems;           // [totalTiles] pairs of queued items so far, likewise
+    S32* tileCursor;          // [totalTiles] next list index for the pairs of queued items
     S32* tileCount;           // [totalTiles]
     S32* tileStart;           // [totalTiles]
     U32* tileList;            // [maxTileEntries]
     S64 maxTileEntries;
     // instance lookup tables (prefix sums, numInstances + 1 entries)
-    const S32* chunkPrefix;   // chunks
-    const S32* binPrefix;     // bins
     const S32* tilePrefix;    // tiles
     const S64* triPrefix;     // triangles
     Counters* counters;
     S32* fineTileCounter;     // [pipe groups] fine-stage tile work counters
-    // Pairs recorded by the bin count pass for the bin scatter pass: chunk c's
-    // (bin << 32 | list entry) pairs in list order at binStage[c * binStageCap],
-    // their number in binStageCount[c]. A chunk with more pairs than
-    // binStageCap (or binStageCap 0) is walked again by the scatter pass.
-    U64* binStage;
-    S32* binStageCount;       // [totalChunks]
-    S32 binStageCap;
-    // Likewise for the coarse passes: unit u < tileStageUnits records its
-    // (tile of the bin << 32 | list entry) pairs at tileStage[u * tileStageCap].
-    U64* tileStage;
-    S32* tileStageCount;      // [tileStageUnits]
-    S32 tileStageCap;
-    S32 tileStageUnits;
     // Device address of the pinned host copy of the counters: the draw's first
     // fine launch writes them there (every stage that changes them has
     // finished by then), in place of a device-to-host copy after the draw.
@@ -325,7 +344,7 @@ __device__ __forceinline__ U32 centroidCode(int s, U32 mask) {
     return (U32)(msaaPatternX(s, best) * 0x02 + best * 0x20 + 0x11) & 0xFF;
 }
 
-__device__ __forceinline__ S32 lo16(U32 v) { return (S32)(int16_t)(uint16_t)(v & 0xFFFF); }
-__device__ __forceinline__ S32 hi16(U32 v) { return (S32)(int16_t)(uint16_t)(v >> 16); }
+__host__ __device__ __forceinline__ S32 lo16(U32 v) { return (S32)(int16_t)(uint16_t)(v & 0xFFFF); }
+__host__ __device__ __forceinline__ S32 hi16(U32 v) { return (S32)(int16_t)(uint16_t)(v >> 16); }
 
 }  // namespace cr

@@ -29,7 +29,8 @@
 //   sample are those of its front-most covering fragment, the earliest one in
 //   submission order on equal depth -- the same result as applying every
 //   fragment in order with a LESS test. Each sample keeps a 64-bit key
-//   (depth << 32 | list position + 1) that fragments lower with atomicMin;
+//   (depth << 32 | list entry + 1) that fragments lower with atomicMin, so the
+//   tile's list may come in any order (entries grow in submission order);
 //   after the list, the tile's winners are listed and each is shaded once,
 //   32 at a time.
 //
@@ -93,8 +94,9 @@ template <int S>
 struct FineVisSmem {
     static constexpr int kTileWords = 64 << S;
     U32 color[kTileWords];
-    U64 key[kTileWords];        // depth << 32 | order (order << 8 | coverage mask with MSAA)
+    U64 key[kTileWords];        // depth << 32 | order (order << NS | coverage mask with MSAA)
     TriRec rec[32];             // the batch's triangles
+    U32 order[32];              // their order: list entry within the scene + 1
     U32 box[32];                // bx0 | by0 << 4 | w << 8 | ceil(2^16 / w) << 12: a small triangle's pixel box
     S32 head[32];               // batch triangle whose pairs start at position i of the current pass
     U32 winners[kTileWords];    // resolve: (pixel | first sample << 6 | samples won << 9)
@@ -355,10 +357,12 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
         const S32 stride4 = __ldg(&in->stride4);
         const float4* verts = (const float4*)__ldg((const unsigned long long*)&in->vertices);
 
-        // Visibility keys: depth << 32 | order, order = list position + 1; with
-        // MSAA the low word also carries the winner's coverage mask of the
-        // pixel (order << 8 | mask) while positions fit in 24 bits.
-        const bool packed = S != 0 && count < (1 << 24) - 1;
+        // Visibility keys: depth << 32 | order, order = list entry within the
+        // scene + 1; with MSAA the low word also carries the winner's coverage
+        // mask of the pixel (order << NS | mask) where the scene's entries
+        // leave room for it (at 4 samples, up to 2^25 triangles).
+        const U32 entryBase = (U32)triBase << 3;
+        const bool packed = S != 0 && (U32)__ldg(&in->numTris) <= (1u << (S != 0 ? 29 - NS : 0)) - 1u;
 
         for (S32 batch = 0; batch < count; batch += 32) {
             if constexpr (kVisibility) {
@@ -389,6 +393,7 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                             const S32 w = bx1 - bx0 + 1;
                             const S32 cnt = w * (by1 - by0 + 1);
                             big = cnt > selfPixels;
+                            sm.order[lane] = entry - entryBase + 1u;
                             sm.rec[lane].q[0] = make_uint4((U32)te.E[0], (U32)te.E[1], (U32)te.E[2], (U32)te.A[0]);
                             sm.rec[lane].q[1] = make_uint4((U32)te.A[1], (U32)te.A[2], (U32)te.B[0], (U32)te.B[1]);
                             sm.rec[lane].q[2] = make_uint4((U32)te.B[2], q0.x, q0.y, q0.z);
@@ -442,8 +447,8 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                     const S32 B[3] = {(S32)r1.z, (S32)r1.w, (S32)r2.x};
                     const U32 smask = sampleMaskOf<S>(E, A, B, px, py);
                     if (!smask) continue;
-                    const U32 order = (U32)(batch + j + 1);
-                    const U64 low = packed ? (order << 8 | smask) : order;
+                    const U32 order = sm.order[j];
+                    const U64 low = packed ? (order << NS | smask) : order;
                     const U32 X = (U32)(tx * 8 + px), Y = (U32)(ty * 8 + py);
                     const U32 zx = r2.y, zy = r2.z, zb = r2.w;
 #pragma unroll
@@ -480,7 +485,7 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                         const S32 e11 = e01 + ((S32)r1.w << (kSubpixelLog2 + 2));
                         const S32 e12 = e02 + ((S32)r2.x << (kSubpixelLog2 + 2));
                         const U32 z0 = r2.y * pX + r2.z * pY0 + r2.w, z1 = z0 + (r2.z << 2);
-                        const U32 order = (U32)(batch + j + 1);
+                        const U32 order = sm.order[j];
                         const U64 key0 = ((U64)z0 << 32) | order, key1 = ((U64)z1 << 32) | order;
                         if ((e00 | e01 | e02) >= 0 && key0 < k0) k0 = key0;
                         if ((e10 | e11 | e12) >= 0 && key1 < k1) k1 = key1;
@@ -495,13 +500,13 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                     const S32 A[3] = {(S32)r0.w, (S32)r1.x, (S32)r1.y};
                     const S32 B[3] = {(S32)r1.z, (S32)r1.w, (S32)r2.x};
                     const U32 zx = r2.y, zy = r2.z, zb = r2.w;
-                    const U32 order = (U32)(batch + j + 1);
+                    const U32 order = sm.order[j];
 #pragma unroll
                     for (int half = 0; half < 2; half++) {
                         const S32 pyy = half ? py1 : py0;
                         const U32 Y = half ? pY1 : pY0;
                         const U32 smask = sampleMaskOf<S>(E, A, B, px, pyy);
-                        const U64 low = packed ? (order << 8 | smask) : order;
+                        const U64 low = packed ? (order << NS | smask) : order;
 #pragma unroll
                         for (int i = 0; i < NS; i++) {
                             if (!(smask >> i & 1)) continue;
@@ -891,7 +896,7 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                 const int rowBase = py * 8 * NS + px;
                 U32 low = (U32)sm.key[rowBase + i0 * 8];
                 U32 td[16];
-                const U32 entry = __ldg(&d.tileList[start + (S32)(packed ? (low >> 8) : low) - 1]);
+                const U32 entry = (packed ? low >> NS : low) - 1u + entryBase;
                 const U32 sub = entry & 7;
                 const U32 tri = entry >> 3;
                 const S64 slot = (sub == 7) ? (S64)tri : (S64)__ldg(&d.triHeader[tri].w) + sub;
@@ -904,7 +909,7 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                     const TileEdges te = tileEdges(__ldg(&d.triHeader[slot]), cx0, cy0);
                     low = sampleMaskOf<S>(te.E, te.A, te.B, px, py);
                 } else if (S != 0) {
-                    low &= 0xFFu;
+                    low &= (1u << NS) - 1u;
                 }
                 bool discard;
                 const S32 X = tx * 8 + px, Y = ty * 8 + py;

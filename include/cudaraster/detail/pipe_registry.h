@@ -21,6 +21,7 @@ struct PipeDesc {
     int32_t profilingMode;
     char blendShaderName[64];
     char fragmentShaderName[64];
+    int32_t needsOrder;   // the fine stage needs each tile's list in submission order
     // Launch the setup kernel over triangles [triBegin, triEnd) of instances
     // [instBegin, instEnd).
     cudaError_t (*launchSetup)(const DrawDev& d, int instBegin, int instEnd, int64_t triBegin,
