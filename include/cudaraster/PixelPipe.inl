@@ -34,8 +34,8 @@ struct PipeImpl {
                                    cudaStream_t stream) {
         int64_t n = triEnd - triBegin;
         if (n <= 0) return cudaSuccess;
-        unsigned grid = (unsigned)((n + 255) / 256);
-        return launchKernel(setupKernel<S, F & (kRenderDepth | kRenderLerp)>, grid, 256, 0, stream, true, d, instBegin,
+        unsigned grid = (unsigned)((n + kSetupThreads - 1) / kSetupThreads);
+        return launchKernel(setupKernel<S, F & (kRenderDepth | kRenderLerp)>, grid, kSetupThreads, 0, stream, true, d, instBegin,
                             instEnd, (S64)triBegin, (S64)triEnd);
     }
     static size_t smemBytes(int warps) { return sizeof(typename FineTraits<FS, BS, S, F>::Smem) * (size_t)warps; }

@@ -207,8 +207,6 @@ __device__ __forceinline__ F32 fdiv(F32 a, F32 b) { return __fdiv_rn(a, b); }
 __device__ __forceinline__ F32 frcp(F32 a) { return __frcp_rn(a); }  // 1 / a, correctly rounded (= __fdiv_rn(1, a))
 __device__ __forceinline__ S32 min3i(S32 a, S32 b, S32 c) { return min(min(a, b), c); }
 __device__ __forceinline__ S32 max3i(S32 a, S32 b, S32 c) { return max(max(a, b), c); }
-// shr.s64 semantics: shift amounts >= 64 give the sign fill.
-__device__ __forceinline__ S64 sar64(S64 a, S32 n) { return ((U32)n >= 64u) ? (a >> 63) : (a >> n); }
 __device__ __forceinline__ U32 absWrap(S32 v) { return v < 0 ? 0u - (U32)v : (U32)v; }
 
 // toABGR (Util.inl:30-38): fma.rm then cvt.rmi.sat.u32, top byte.
@@ -244,29 +242,55 @@ __device__ __forceinline__ U32 selectFlips(S32 dx, S32 dy) {
     return flips;
 }
 
-// setupPleq (Util.inl:65-91). v0 = subpixels relative to the first sample.
-__device__ __forceinline__ void setupPleq(F32 vx, F32 vy, F32 vz, int2 v0, int2 d1, int2 d2,
-                                          F32 areaRcp, int s, U32& ox, U32& oy, U32& oz) {
-    F32 mx = fmaxf(fmaxf(vx, vy), vz);
-    int sh = min(max((__float_as_int(mx) >> 23) - (127 + 22), 0), 8);
-    S32 t0 = (S32)(f32_to_u32_rz(vx) >> sh);
-    S32 t1 = (S32)((f32_to_u32_rz(vy) >> sh) - (U32)t0);
-    S32 t2 = (S32)((f32_to_u32_rz(vz) >> sh) - (U32)t0);
-    U32 rcpMant = ((U32)__float_as_int(areaRcp) & 0x007FFFFFu) | 0x00800000u;
-    int rcpShift = (23 + 127) - (__float_as_int(areaRcp) >> 23);
-    S64 xc = (S64)((U64)((S64)t1 * d2.y - (S64)t2 * d1.y) * (U64)rcpMant);
-    S64 yc = (S64)((U64)((S64)t2 * d1.x - (S64)t1 * d2.x) * (U64)rcpMant);
-    ox = (U32)sar64(xc, rcpShift - (sh + kSubpixelLog2 - s));
-    oy = (U32)sar64(yc, rcpShift - (sh + kSubpixelLog2 - s));
-    S32 centerX = (S32)((U32)v0.x * 2u + (U32)min3i(d1.x, d2.x, 0) + (U32)max3i(d1.x, d2.x, 0)) >> (kSubpixelLog2 - s + 1);
-    S32 centerY = (S32)((U32)v0.y * 2u + (U32)min3i(d1.y, d2.y, 0) + (U32)max3i(d1.y, d2.y, 0)) >> (kSubpixelLog2 - s + 1);
-    S32 vcx = (S32)((U32)v0.x - ((U32)centerX << (kSubpixelLog2 - s)));
-    S32 vcy = (S32)((U32)v0.y - ((U32)centerY << (kSubpixelLog2 - s)));
+// setupPleq (Util.inl:65-91). v0 = subpixels relative to the first sample;
+// area = 1 / areaRcp is a whole number from 1 to 2^34, so rcpShift lies in
+// [23, 57] and every shift below in [2, 57]: the reference's shr.s64 never
+// clamps. PleqFrame holds what the planes of one triangle share.
+struct PleqFrame {
+    int2 d1, d2;
+    U32 rcpMant;
+    int rcpShift, s;
+    S32 centerX, centerY, vcx, vcy;
+};
+
+__device__ __forceinline__ PleqFrame pleqFrame(int2 v0, int2 d1, int2 d2, F32 areaRcp, int s) {
+    PleqFrame f;
+    f.d1 = d1;
+    f.d2 = d2;
+    f.s = s;
+    f.rcpMant = ((U32)__float_as_int(areaRcp) & 0x007FFFFFu) | 0x00800000u;
+    f.rcpShift = (23 + 127) - (__float_as_int(areaRcp) >> 23);
+    f.centerX = (S32)((U32)v0.x * 2u + (U32)min3i(d1.x, d2.x, 0) + (U32)max3i(d1.x, d2.x, 0)) >> (kSubpixelLog2 - s + 1);
+    f.centerY = (S32)((U32)v0.y * 2u + (U32)min3i(d1.y, d2.y, 0) + (U32)max3i(d1.y, d2.y, 0)) >> (kSubpixelLog2 - s + 1);
+    f.vcx = (S32)((U32)v0.x - ((U32)f.centerX << (kSubpixelLog2 - s)));
+    f.vcy = (S32)((U32)v0.y - ((U32)f.centerY << (kSubpixelLog2 - s)));
+    return f;
+}
+
+// The plane from its gradients' numerators (gx, gy, before the multiplication
+// by the area's reciprocal), its value t0 at v0 and the values' shift sh.
+__device__ __forceinline__ void pleqPlane(const PleqFrame& f, S64 gx, S64 gy, S32 t0, int sh, U32& ox, U32& oy, U32& oz) {
+    const S64 xc = (S64)((U64)gx * (U64)f.rcpMant);
+    const S64 yc = (S64)((U64)gy * (U64)f.rcpMant);
+    ox = (U32)(xc >> (f.rcpShift - (sh + kSubpixelLog2 - f.s)));
+    oy = (U32)(yc >> (f.rcpShift - (sh + kSubpixelLog2 - f.s)));
     U32 z = (U32)t0 << sh;
-    U64 cross = (U64)sar64(xc, 13) * (U64)(S64)vcx + (U64)sar64(yc, 13) * (U64)(S64)vcy;
-    z -= (U32)sar64((S64)cross, rcpShift - (sh + 13));
-    z -= ox * (U32)centerX + oy * (U32)centerY;
+    const U64 cross = (U64)(xc >> 13) * (U64)(S64)f.vcx + (U64)(yc >> 13) * (U64)(S64)f.vcy;
+    z -= (U32)((S64)cross >> (f.rcpShift - (sh + 13)));
+    z -= ox * (U32)f.centerX + oy * (U32)f.centerY;
     oz = z;
+}
+
+__device__ __forceinline__ int pleqValueShift(F32 most) {
+    return min(max((__float_as_int(most) >> 23) - (127 + 22), 0), 8);
+}
+
+__device__ __forceinline__ void setupPleq(F32 vx, F32 vy, F32 vz, const PleqFrame& f, U32& ox, U32& oy, U32& oz) {
+    const int sh = pleqValueShift(fmaxf(fmaxf(vx, vy), vz));
+    const S32 t0 = (S32)(f32_to_u32_rz(vx) >> sh);
+    const S32 t1 = (S32)((f32_to_u32_rz(vy) >> sh) - (U32)t0);
+    const S32 t2 = (S32)((f32_to_u32_rz(vz) >> sh) - (U32)t0);
+    pleqPlane(f, (S64)t1 * f.d2.y - (S64)t2 * f.d1.y, (S64)t2 * f.d1.x - (S64)t1 * f.d2.x, t0, sh, ox, oy, oz);
 }
 
 // clipPolygonWithPlane (Util.hpp:221-250), unfused.

@@ -14,6 +14,18 @@
 
 namespace cr {
 
+// Threads of a setup CTA, and resident CTAs per SM the compiler must allow
+// (register budget: 48). Issue and load latency bound it about equally (64% of
+// issue slots, 50% occupancy): CTAs of 128 instead of 256 threads end closer
+// together (4096^2 heightfield 594 -> 570 us, 1M-triangle soup 31.7 -> 29.7; 64
+// threads: 577 and 30.0). At 256 threads, six CTAs (40 registers, spilling)
+// and four (64) measured no faster than five.
+constexpr int kSetupThreads = 128;
+#ifndef CR_SETUP_MIN_BLOCKS
+#define CR_SETUP_MIN_BLOCKS 10
+#endif
+constexpr S64 kSetupAhead = 2 * 152 * CR_SETUP_MIN_BLOCKS * kSetupThreads;   // triangles, of prefetchIndices
+
 struct SnapOut {
     int2 p0, p1, p2, lo, hi;
     F32 rcpW0, rcpW1, rcpW2;
@@ -35,16 +47,23 @@ __device__ __forceinline__ SnapOut snapTriangle(float4 v0, float4 v1, float4 v2,
     return o;
 }
 
-__device__ __forceinline__ S64 cross2(S32 ax, S32 ay, S32 bx, S32 by) { return (S64)ax * by - (S64)ay * bx; }
+// Whether the origin lies outside an edge of triangle a, b, c.
+template <class T>
+__device__ __forceinline__ bool outsideEdge(S32 ax, S32 ay, S32 bx, S32 by, S32 cx, S32 cy) {
+    const T ab = (T)ax * by - (T)ay * bx, bc = (T)bx * cy - (T)by * cx, ca = (T)cx * ay - (T)cy * ax;
+    return (ab | bc | ca) < 0;
+}
 
 // prepareTriangle (TriangleSetup.inl:38-100): 0 visible, 1 backfacing, 2 between samples.
-// The area is formed in 64 bits (equal to the reference's S32 product up to
-// 2048-px viewports, overflow-free beyond).
-template <int S>
-__device__ __forceinline__ int prepareTriangle(const SnapOut& t, S32 width, S32 height, int2& d1, int2& d2, S64& area) {
+// T = S32 for triangles inside the fast path's bound, whose edge vectors stay
+// below 2^15 in each coordinate: twice the area fits in 31 bits and is the
+// reference's S32 product. T = S64 otherwise (equal up to 2048-px viewports,
+// overflow-free beyond).
+template <int S, class T>
+__device__ __forceinline__ int prepareTriangle(const SnapOut& t, S32 width, S32 height, int2& d1, int2& d2, T& area) {
     d1 = make_int2((S32)((U32)t.p1.x - (U32)t.p0.x), (S32)((U32)t.p1.y - (U32)t.p0.y));
     d2 = make_int2((S32)((U32)t.p2.x - (U32)t.p0.x), (S32)((U32)t.p2.y - (U32)t.p0.y));
-    area = (S64)d1.x * d2.y - (S64)d1.y * d2.x;
+    area = (T)d1.x * d2.y - (T)d1.y * d2.x;
     if (area <= 0) return 1;
     const S32 sampleSize = 1 << (kSubpixelLog2 - S);
     S32 biasX = (width << (kSubpixelLog2 - 1)) - (sampleSize >> 1);
@@ -56,29 +75,32 @@ __device__ __forceinline__ int prepareTriangle(const SnapOut& t, S32 width, S32 
     if (lox > hix || loy > hiy) return 2;
     S32 diff = (S32)((U32)hix + (U32)hiy - (U32)lox - (U32)loy);
     if (diff <= sampleSize) {
+        // (One or two samples in the box, whose sides are then below three
+        // sample distances: the edge functions are small.)
         S32 ax = t.p0.x + biasX - lox, ay = t.p0.y + biasY - loy;
         S32 bx = t.p1.x + biasX - lox, by = t.p1.y + biasY - loy;
         S32 cx = t.p2.x + biasX - lox, cy = t.p2.y + biasY - loy;
-        if (cross2(ax, ay, bx, by) < 0 || cross2(bx, by, cx, cy) < 0 || cross2(cx, cy, ax, ay) < 0) {
+        if (outsideEdge<T>(ax, ay, bx, by, cx, cy)) {
             if (diff == 0) return 2;
             ax = t.p0.x + biasX - hix; ay = t.p0.y + biasY - hiy;
             bx = t.p1.x + biasX - hix; by = t.p1.y + biasY - hiy;
             cx = t.p2.x + biasX - hix; cy = t.p2.y + biasY - hiy;
-            if (cross2(ax, ay, bx, by) < 0 || cross2(bx, by, cx, cy) < 0 || cross2(cx, cy, ax, ay) < 0) return 2;
+            if (outsideEdge<T>(ax, ay, bx, by, cx, cy)) return 2;
         }
     }
     return 0;
 }
 
 // setupTriangle (TriangleSetup.inl:104-215): writes one header + data slot.
-template <int S, U32 F>
+// With kWhole the triangle is a whole one: barycentrics (0, 0), (1, 0), (0, 1).
+template <int S, U32 F, bool kWhole>
 __device__ __forceinline__ void setupTriangle(uint4* th, uint4* td, int3 vidx, float4 v0, float4 v1, float4 v2,
                                               float2 b0, float2 b1, float2 b2, const SnapOut& t,
-                                              int2 d1, int2 d2, S64 area, S32 width, S32 height) {
+                                              int2 d1, int2 d2, F32 area, S32 width, S32 height) {
     F32 areaRcp = 0.0f;
     int2 wv0 = make_int2(0, 0);
     if (F & (kRenderDepth | kRenderLerp)) {
-        areaRcp = frcp(__ll2float_rn(area));
+        areaRcp = frcp(area);
         wv0.x = t.p0.x + (width << (kSubpixelLog2 - 1));
         wv0.y = t.p0.y + (height << (kSubpixelLog2 - 1));
     }
@@ -90,7 +112,7 @@ __device__ __forceinline__ void setupTriangle(uint4* th, uint4* td, int3 vidx, f
         F32 z1 = fadd(fmul(fmul(v1.z, zcoef), t.rcpW1), zbias);
         F32 z2 = fadd(fmul(fmul(v2.z, zcoef), t.rcpW2), zbias);
         int2 zv0 = make_int2(wv0.x - (1 << (kSubpixelLog2 - S - 1)), wv0.y - (1 << (kSubpixelLog2 - S - 1)));
-        setupPleq(z0, z1, z2, zv0, d1, d2, areaRcp, S, zx, zy, zb);
+        setupPleq(z0, z1, z2, pleqFrame(zv0, d1, d2, areaRcp, S), zx, zy, zb);
         zmin = f32_to_u32_sat(fsub(fminf(fminf(z0, z1), z2), (F32)lerpError(S)));
         if (S != 0) {
             U32 tmp = absWrap((S32)zx) + absWrap(max((S32)zy, -0x7FFFFFFF));
@@ -103,9 +125,21 @@ __device__ __forceinline__ void setupTriangle(uint4* th, uint4* td, int3 vidx, f
     if (F & kRenderLerp) {
         F32 wcoef = fmul(fminf(fminf(v0.w, v1.w), v2.w), (F32)kBaryMax);
         F32 w0 = fmul(wcoef, t.rcpW0), w1 = fmul(wcoef, t.rcpW1), w2 = fmul(wcoef, t.rcpW2);
-        setupPleq(w0, w1, w2, wv0, d1, d2, areaRcp, S + 1, wx, wy, wb);
-        setupPleq(fmul(b0.x, w0), fmul(b1.x, w1), fmul(b2.x, w2), wv0, d1, d2, areaRcp, S + 1, ux, uy, ub);
-        setupPleq(fmul(b0.y, w0), fmul(b1.y, w1), fmul(b2.y, w2), wv0, d1, d2, areaRcp, S + 1, vx, vy, vb);
+        const PleqFrame f = pleqFrame(wv0, d1, d2, areaRcp, S + 1);
+        setupPleq(w0, w1, w2, f, wx, wy, wb);
+        if (kWhole && fmaxf(fmaxf(w0, w1), w2) < 3.0e38f && fminf(fminf(w0, w1), w2) >= 0.0f) {
+            // Finite and not negative: u is 0, w1, 0 and v is 0, 0, w2 at the
+            // vertices, so that one term of each gradient remains.
+            int sh = pleqValueShift(w1);
+            S32 t1 = (S32)(f32_to_u32_rz(w1) >> sh);
+            pleqPlane(f, (S64)t1 * d2.y, -(S64)t1 * d2.x, 0, sh, ux, uy, ub);
+            sh = pleqValueShift(w2);
+            t1 = (S32)(f32_to_u32_rz(w2) >> sh);
+            pleqPlane(f, -(S64)t1 * d1.y, (S64)t1 * d1.x, 0, sh, vx, vy, vb);
+        } else {
+            setupPleq(fmul(b0.x, w0), fmul(b1.x, w1), fmul(b2.x, w2), f, ux, uy, ub);
+            setupPleq(fmul(b0.y, w0), fmul(b1.y, w1), fmul(b2.y, w2), f, vx, vy, vb);
+        }
     }
     td[0] = make_uint4(zx, zy, zb, zslope);
     td[1] = make_uint4(wx, wy, wb, ux);
@@ -123,54 +157,6 @@ __device__ __forceinline__ void setupTriangle(uint4* th, uint4* td, int3 vidx, f
 __device__ __forceinline__ float4 lerpClip(float4 o, float4 a, float4 b, F32 bu, F32 bv) {
     return make_float4(fadd(fadd(o.x, fmul(a.x, bu)), fmul(b.x, bv)), fadd(fadd(o.y, fmul(a.y, bu)), fmul(b.y, bv)),
                        fadd(fadd(o.z, fmul(a.z, bu)), fmul(b.z, bv)), fadd(fadd(o.w, fmul(a.w, bu)), fmul(b.w, bv)));
-}
-
-// Clip path of triangleSetupImpl (TriangleSetup.inl:326-412), out of line so
-// the common path keeps its registers.
-template <int S, U32 F>
-__device__ __noinline__ void setupClipped(const DrawDev& d, S64 gt, int3 vidx, float4 v0, float4 v1, float4 v2,
-                                          S32 width, S32 height) {
-    int2 d1, d2;
-    S64 area;
-    float4 ov0 = v0;
-    float4 od1 = make_float4(fsub(v1.x, v0.x), fsub(v1.y, v0.y), fsub(v1.z, v0.z), fsub(v1.w, v0.w));
-    float4 od2 = make_float4(fsub(v2.x, v0.x), fsub(v2.y, v0.y), fsub(v2.z, v0.z), fsub(v2.w, v0.w));
-    F32 bary[18];
-    int numVerts = clipTriangle(bary, &ov0.x, &v1.x, &v2.x, &od1.x, &od2.x);
-    float4 c0 = lerpClip(ov0, od1, od2, bary[0], bary[1]);
-    float4 c1 = lerpClip(ov0, od1, od2, bary[2], bary[3]);
-    float4 tc1 = c1;
-
-    int numSubtris = 0;
-    for (int i = 2; i < numVerts; i++) {
-        float4 c2 = lerpClip(ov0, od1, od2, bary[i * 2], bary[i * 2 + 1]);
-        SnapOut sn = snapTriangle(c0, c1, c2, width, height);
-        if (prepareTriangle<S>(sn, width, height, d1, d2, area) == 0) numSubtris++;
-        c1 = c2;
-    }
-    d.triSubtris[gt] = (uint8_t)numSubtris;
-
-    S64 base = gt;
-    if (numSubtris > 1) {
-        base = d.totalTris + atomicAdd(&d.counters->extraSubtris, numSubtris);
-        d.triHeader[gt].w = (U32)base;
-        if (base + numSubtris > d.maxSubtris) {
-            atomicOr(&d.counters->overflow, kOverflowSubtris);
-            numVerts = 0;
-        }
-    }
-    c1 = tc1;
-    for (int i = 2; i < numVerts; i++) {
-        float4 c2 = lerpClip(ov0, od1, od2, bary[i * 2], bary[i * 2 + 1]);
-        SnapOut sn = snapTriangle(c0, c1, c2, width, height);
-        if (prepareTriangle<S>(sn, width, height, d1, d2, area) == 0) {
-            setupTriangle<S, F>(&d.triHeader[base], &d.triData[base * 4], vidx, c0, c1, c2,
-                                make_float2(bary[0], bary[1]), make_float2(bary[i * 2 - 2], bary[i * 2 - 1]),
-                                make_float2(bary[i * 2], bary[i * 2 + 1]), sn, d1, d2, area, width, height);
-            base++;
-        }
-        c1 = c2;
-    }
 }
 
 // Clip position of vertex i: its record's clipPos, or, with the fused vertex
@@ -209,35 +195,111 @@ __device__ __forceinline__ void fetchClip(const DrawDev& d, const float4* verts,
     }
 }
 
-// Resident setup CTAs per SM the compiler must allow (register budget):
-// five (48 registers). Six (40 registers, 52 bytes
-// spilled) measured slower on the soup and the 4x MSAA grid (setup 36.7 ->
-// 38.4 us and 0.168 -> 0.172 ms) and level on the fly-through.
-#ifndef CR_SETUP_MIN_BLOCKS
-#define CR_SETUP_MIN_BLOCKS 5
-#endif
+// Vertex indices and clip positions of triangle slot gt of instance `in`.
+__device__ __forceinline__ void fetchTriangle(const DrawDev& d, const InstanceDev* in, S64 gt, int3& vidx, float4& v0,
+                                              float4& v1, float4& v2) {
+    const int* indices = (const int*)__ldg((const unsigned long long*)&in->indices);
+    const float4* verts = (const float4*)__ldg((const unsigned long long*)&in->vertices);
+    const S64 t = gt - __ldg(&in->triBase);
+    vidx = make_int3(__ldg(&indices[3 * t + 0]), __ldg(&indices[3 * t + 1]), __ldg(&indices[3 * t + 2]));
+    fetchClip(d, verts, __ldg(&in->stride4), vidx, v0, v1, v2);
+}
+
+// Asks L2 for the indices that the CTA two waves of CTAs on will read (12
+// lines of 128 bytes): a thread's index and vertex loads are a dependent chain,
+// and this takes the first trip to DRAM out of it (4096^2 heightfield 570 ->
+// 550 us, 2048^2 157 -> 151).
+__device__ __forceinline__ void prefetchIndices(const InstanceDev* in, S64 gt) {
+    if (threadIdx.x >= kSetupThreads * 12 / 128) return;
+    const char* indices = (const char*)__ldg((const unsigned long long*)&in->indices);
+    const S64 ahead = gt - threadIdx.x - __ldg(&in->triBase) + kSetupAhead;
+    const S64 at = ahead * 12 + threadIdx.x * 128;
+    if (at < (S64)__ldg(&in->numTris) * 12) asm volatile("prefetch.global.L2 [%0];" ::"l"(indices + at));
+}
+
+// Clip path of triangleSetupImpl (TriangleSetup.inl:326-412), out of line (it
+// reads its triangle again) so the common path keeps its registers.
+template <int S, U32 F>
+__device__ __noinline__ void setupClipped(const DrawDev& d, U32 gt, int ii) {
+    const InstanceDev* in = &d.inst[ii];
+    const S32 width = __ldg(&in->width), height = __ldg(&in->height);
+    int3 vidx;
+    float4 v0, v1, v2;
+    fetchTriangle(d, in, gt, vidx, v0, v1, v2);
+    int2 d1, d2;
+    S64 area;
+    float4 ov0 = v0;
+    float4 od1 = make_float4(fsub(v1.x, v0.x), fsub(v1.y, v0.y), fsub(v1.z, v0.z), fsub(v1.w, v0.w));
+    float4 od2 = make_float4(fsub(v2.x, v0.x), fsub(v2.y, v0.y), fsub(v2.z, v0.z), fsub(v2.w, v0.w));
+    F32 bary[18];
+    int numVerts = clipTriangle(bary, &ov0.x, &v1.x, &v2.x, &od1.x, &od2.x);
+    float4 c0 = lerpClip(ov0, od1, od2, bary[0], bary[1]);
+    float4 c1 = lerpClip(ov0, od1, od2, bary[2], bary[3]);
+    float4 tc1 = c1;
+
+    int numSubtris = 0;
+    for (int i = 2; i < numVerts; i++) {
+        float4 c2 = lerpClip(ov0, od1, od2, bary[i * 2], bary[i * 2 + 1]);
+        SnapOut sn = snapTriangle(c0, c1, c2, width, height);
+        if (prepareTriangle<S, S64>(sn, width, height, d1, d2, area) == 0) numSubtris++;
+        c1 = c2;
+    }
+    d.triSubtris[gt] = (uint8_t)numSubtris;
+
+    S64 base = gt;
+    if (numSubtris > 1) {
+        base = d.totalTris + atomicAdd(&d.counters->extraSubtris, numSubtris);
+        d.triHeader[gt].w = (U32)base;
+        if (base + numSubtris > d.maxSubtris) {
+            atomicOr(&d.counters->overflow, kOverflowSubtris);
+            numVerts = 0;
+        }
+    }
+    c1 = tc1;
+    for (int i = 2; i < numVerts; i++) {
+        float4 c2 = lerpClip(ov0, od1, od2, bary[i * 2], bary[i * 2 + 1]);
+        SnapOut sn = snapTriangle(c0, c1, c2, width, height);
+        if (prepareTriangle<S, S64>(sn, width, height, d1, d2, area) == 0) {
+            setupTriangle<S, F, false>(&d.triHeader[base], &d.triData[base * 4], vidx, c0, c1, c2,
+                                       make_float2(bary[0], bary[1]), make_float2(bary[i * 2 - 2], bary[i * 2 - 1]),
+                                       make_float2(bary[i * 2], bary[i * 2 + 1]), sn, d1, d2, __ll2float_rn(area), width,
+                                       height);
+            base++;
+        }
+        c1 = c2;
+    }
+}
+
+// The fast path's bound on the snapped vertices (TriangleSetup.inl:289-294).
+__device__ __forceinline__ bool inFastBound(const SnapOut& sn) {
+    const S32 loxy = min(sn.lo.x, sn.lo.y);
+    const S32 hixy = max(sn.hi.x, sn.hi.y);
+    return loxy >= -32768 && hixy <= 32767 && hixy - loxy <= (1 << (kMaxViewportLog2Ref + kSubpixelLog2)) - 1;
+}
+
+// Whether the clipper would cut a triangle with this vertex (Util.hpp:268).
+__device__ __forceinline__ bool cutByPlane(float4 v) {
+    return (v.w < fabsf(v.x)) | (v.w < fabsf(v.y)) | (v.w < fabsf(v.z));
+}
 
 // triangleSetupImpl (TriangleSetup.inl:219-417), over the triangle range of
 // one pipe group [triBegin, triEnd) (global triangle slots).
 template <int S, U32 F>
-__global__ void __launch_bounds__(256, CR_SETUP_MIN_BLOCKS) setupKernel(DrawDev d, int instBegin, int instEnd, S64 triBegin, S64 triEnd) {
+__global__ void __launch_bounds__(kSetupThreads, CR_SETUP_MIN_BLOCKS) setupKernel(DrawDev d, int instBegin, int instEnd, S64 triBegin, S64 triEnd) {
     pdlWait();
     pdlTrigger();
-    S64 gt = triBegin + (S64)blockIdx.x * 256 + threadIdx.x;
+    const S64 gt = triBegin + (S64)blockIdx.x * kSetupThreads + threadIdx.x;
     if (gt >= triEnd) return;
-    int ii = instBegin + findInstance64(d.triPrefix + instBegin, instEnd - instBegin, gt);
+    const int ii = instBegin + findInstance64(d.triPrefix + instBegin, instEnd - instBegin, gt);
     const InstanceDev* in = &d.inst[ii];
-    const S32 width = __ldg(&in->width), height = __ldg(&in->height), stride4 = __ldg(&in->stride4);
-    const int* indices = (const int*)__ldg((const unsigned long long*)&in->indices);
-    const float4* verts = (const float4*)__ldg((const unsigned long long*)&in->vertices);
-    S64 t = gt - __ldg(&in->triBase);
-
-    int3 vidx = make_int3(__ldg(&indices[3 * t + 0]), __ldg(&indices[3 * t + 1]), __ldg(&indices[3 * t + 2]));
+    const S32 width = __ldg(&in->width), height = __ldg(&in->height);
+    int3 vidx;
     float4 v0, v1, v2;
-    fetchClip(d, verts, stride4, vidx, v0, v1, v2);
+    prefetchIndices(in, gt);
+    fetchTriangle(d, in, gt, vidx, v0, v1, v2);
 
     // Outside view frustum => cull (TriangleSetup.inl:262-281).
-    if ((v0.w < fabsf(v0.x)) | (v0.w < fabsf(v0.y)) | (v0.w < fabsf(v0.z))) {
+    if (cutByPlane(v0)) {
         if (((v0.w < +v0.x) & (v1.w < +v1.x) & (v2.w < +v2.x)) |
             ((v0.w < -v0.x) & (v1.w < -v1.x) & (v2.w < -v2.x)) |
             ((v0.w < +v0.y) & (v1.w < +v1.y) & (v2.w < +v2.y)) |
@@ -249,27 +311,46 @@ __global__ void __launch_bounds__(256, CR_SETUP_MIN_BLOCKS) setupKernel(DrawDev 
         }
     }
 
-    int2 d1, d2;
-    S64 area;
     // Inside depth range and small enough => fast path (TriangleSetup.inl:285-322).
-    if ((v0.w >= fabsf(v0.z)) & (v1.w >= fabsf(v1.z)) & (v2.w >= fabsf(v2.z))) {
-        SnapOut sn = snapTriangle(v0, v1, v2, width, height);
-        S32 loxy = min(sn.lo.x, sn.lo.y);
-        S32 hixy = max(sn.hi.x, sn.hi.y);
-        const S32 aabbLimit = (1 << (kMaxViewportLog2Ref + kSubpixelLog2)) - 1;
-        if (loxy >= -32768 && hixy <= 32767 && hixy - loxy <= aabbLimit) {
-            int res = prepareTriangle<S>(sn, width, height, d1, d2, area);
-            d.triSubtris[gt] = (res == 0) ? 1 : 0;
-            if (res == 0)
-                setupTriangle<S, F>(&d.triHeader[gt], &d.triData[gt * 4], vidx, v0, v1, v2,
-                                    make_float2(0.0f, 0.0f), make_float2(1.0f, 0.0f), make_float2(0.0f, 1.0f),
-                                    sn, d1, d2, area, width, height);
+    SnapOut sn;
+    int2 d1, d2;
+    F32 area = 0.0f;
+    bool live;
+    bool fast = (v0.w >= fabsf(v0.z)) & (v1.w >= fabsf(v1.z)) & (v2.w >= fabsf(v2.z));
+    if (fast) {
+        sn = snapTriangle(v0, v1, v2, width, height);
+        fast = inFastBound(sn);
+    }
+    if (fast) {
+        S32 a;
+        live = prepareTriangle<S, S32>(sn, width, height, d1, d2, a) == 0;
+        area = __int2float_rn(a);
+    } else {
+        // Clip to the view frustum (TriangleSetup.inl:326-412); out of line.
+        if (cutByPlane(v0) | cutByPlane(v1) | cutByPlane(v2)) {
+            setupClipped<S, F>(d, (U32)gt, ii);
             return;
         }
+        // A triangle that no plane cuts comes out of the clipper with its
+        // vertices re-formed from the edge vectors (barycentrics 0 and 1).
+        // Beyond 2048 px these are many: the fast path's bound, taken over x
+        // and y together, sends here all triangles of two viewport corners (a
+        // tenth of a 3840x2160 frame).
+        const float4 o = v0;
+        const float4 e1 = make_float4(fsub(v1.x, o.x), fsub(v1.y, o.y), fsub(v1.z, o.z), fsub(v1.w, o.w));
+        const float4 e2 = make_float4(fsub(v2.x, o.x), fsub(v2.y, o.y), fsub(v2.z, o.z), fsub(v2.w, o.w));
+        v0 = lerpClip(o, e1, e2, 0.0f, 0.0f);
+        v1 = lerpClip(o, e1, e2, 1.0f, 0.0f);
+        v2 = lerpClip(o, e1, e2, 0.0f, 1.0f);
+        sn = snapTriangle(v0, v1, v2, width, height);
+        S64 a;
+        live = prepareTriangle<S, S64>(sn, width, height, d1, d2, a) == 0;
+        area = __ll2float_rn(a);
     }
-
-    // Clip to the view frustum (TriangleSetup.inl:326-412); rare, kept out of line.
-    setupClipped<S, F>(d, gt, vidx, v0, v1, v2, width, height);
+    d.triSubtris[gt] = live ? 1 : 0;
+    if (live)
+        setupTriangle<S, F, true>(&d.triHeader[gt], &d.triData[gt * 4], vidx, v0, v1, v2, make_float2(0.0f, 0.0f),
+                                  make_float2(1.0f, 0.0f), make_float2(0.0f, 1.0f), sn, d1, d2, area, width, height);
 }
 
 }  // namespace cr
