@@ -7,6 +7,17 @@
 // the tile's current maximum depth as FineRaster.inl:229-240, edge functions
 // at the tile origin). Then one of two algorithms runs, chosen at compile time:
 //
+// What bounds it: the shared-memory and L1 data pipe (70% of its wavefronts on
+// 1M small triangles, 72% on the 8.4M-triangle 4x MSAA heightfield) and
+// instruction issue (72%, 68%), at 30 to 38 resident warps. So triangles are
+// kept in packed records read by 128-bit loads (two 16-bit edge steps to a
+// word, an edge value in one dp2a), tiles move 8 bytes a lane, and tiles that
+// no triangle touches are written without passing through shared memory. These
+// took the stage from 84 to 80 us on the 1M soup, 107 to 96 on 20,000
+// triangles of 60 pixels, 627 to 606 on the heightfield, 613 to 457 on 300k
+// triangles at 8x MSAA, 160 to 152 on 300k blended ones, 471 to 457 on the
+// textured terrain.
+//
 // Both paths deal the (triangle, pixel) pairs of the batch's small triangles
 // (pixel box of at most fineSelfPixels pixels) over the lanes; larger
 // triangles are rasterized by the 32 pixel-owning lanes, two pixels each.
@@ -55,19 +66,25 @@ constexpr int kFineMaxThreads = 256;
 __host__ __device__ constexpr int fineSelfPixelsDefault(int, bool) { return 16; }
 
 
+// A triangle of a batch in 12 words. Edge k's value at a sample whose offset
+// from the tile's pixel (0, 0) centre, plus 8 subpixels on each axis, is the
+// byte pair q is E[k] + A[k] * q.x + B[k] * q.y, one dp2a with the two steps
+// as 16-bit halves (see packTri). Lanes read a record with 128-bit loads: all
+// lanes the same one (a broadcast) on the large-triangle path; on the pair
+// path lanes of a quarter warp read consecutive records, whose 48-byte stride
+// puts any eight of them on distinct banks.
+struct TriRec {
+    uint4 q[3];   // E0 E1 E2 AB0 | AB1 AB2 zx zy | zb id box -
+};
+
 // The ordered path's per-warp state (one warp per tile).
 template <int S>
 struct FineWarpSmem {
     static constexpr int kTileWords = 64 << S;
     U32 color[kTileWords];
     U32 depth[kTileWords];
-    U32 pairBox[32];       // bx0 | by0 << 4 | w << 8 of each small triangle's pixel box
-    U32 pairMul[32];       // ceil(2^16 / w)
-    S32 E[3][32];          // edge functions at the tile's pixel (0, 0) centre, bias folded in
-    S32 A[3][32];          // per-subpixel x step (-dy)
-    S32 B[3][32];          // per-subpixel y step (+dx)
-    U32 td[16][32];        // triangle data slots (CRTriangleData words)
-    S32 tri[32];           // triangle index within the draw
+    TriRec rec[32];        // id: triangle index within the draw
+    TriRec data[32];       // words 4 to 15 of the triangle data slots
     U32 covLo[32];
     U32 covHi[32];
     // One sample, depth test on, no discard: each pixel's minimum of
@@ -78,16 +95,6 @@ struct FineWarpSmem {
     F32 shared[32];
 };
 
-// A triangle of the visibility path's batch in 12 words: edge functions
-// E0-2, A0-2, B0-2 (see TileEdges) and depth plane zx, zy, zb. Lanes read a
-// record with three 128-bit loads: all lanes the same one (a broadcast) on
-// the large-triangle path; on the pair path lanes of a quarter warp read
-// consecutive records, whose 48-byte stride puts any eight of them on
-// distinct banks.
-struct TriRec {
-    uint4 q[3];   // E0 E1 E2 A0 | A1 A2 B0 B1 | B2 zx zy zb
-};
-
 // The visibility path's per-warp state: no separate depth array (a key's high
 // word is its sample's depth) and only the triangle words it reads.
 template <int S>
@@ -95,9 +102,7 @@ struct FineVisSmem {
     static constexpr int kTileWords = 64 << S;
     U32 color[kTileWords];
     U64 key[kTileWords];        // depth << 32 | order (order << NS | coverage mask with MSAA)
-    TriRec rec[32];             // the batch's triangles
-    U32 order[32];              // their order: list entry within the scene + 1
-    U32 box[32];                // bx0 | by0 << 4 | w << 8 | ceil(2^16 / w) << 12: a small triangle's pixel box
+    TriRec rec[32];             // id: list entry within the scene + 1
     S32 head[32];               // batch triangle whose pairs start at position i of the current pass
     U32 winners[kTileWords];    // resolve: (pixel | first sample << 6 | samples won << 9)
     F32 shared[32];
@@ -166,27 +171,35 @@ __device__ __forceinline__ TileEdges tileEdges(uint4 h, S32 cx0, S32 cy0) {
     TileEdges t;
     S32 vx[3] = {lo16(h.x) - cx0, lo16(h.y) - cx0, lo16(h.z) - cx0};
     S32 vy[3] = {hi16(h.x) - cy0, hi16(h.y) - cy0, hi16(h.z) - cy0};
+    t.minX = min3i(vx[0], vx[1], vx[2]);
+    t.maxX = max3i(vx[0], vx[1], vx[2]);
+    t.minY = min3i(vy[0], vy[1], vy[2]);
+    t.maxY = max3i(vy[0], vy[1], vy[2]);
     const int oi[3] = {0, 1, 0};
     S32 ddx[3] = {vx[1] - vx[0], vx[2] - vx[1], vx[0] - vx[2]};
     S32 ddy[3] = {vy[1] - vy[0], vy[2] - vy[1], vy[0] - vy[2]};
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        S64 e = (S64)vx[oi[k]] * ddy[k] - (S64)vy[oi[k]] * ddx[k];
-        if (ddy[k] > 0 || (ddy[k] == 0 && ddx[k] <= 0)) e -= 1;
-        t.E[k] = clampEdge(e);
         t.A[k] = -ddy[k];
         t.B[k] = ddx[k];
     }
-    t.minX = min3i(vx[0], vx[1], vx[2]);
-    t.maxX = max3i(vx[0], vx[1], vx[2]);
-    t.minY = min3i(vy[0], vy[1], vy[2]);
-    t.maxY = max3i(vy[0], vy[1], vy[2]);
+    // With all vertices within 2^14 subpixels (1,024 pixels) of the tile the
+    // products stay within 2^29 and the values within 2^30: no 64-bit step and
+    // no clamp.
+    const bool near = min(t.minX, t.minY) >= -(1 << 14) && max(t.maxX, t.maxY) <= 1 << 14;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const S32 bias = ddy[k] > 0 || (ddy[k] == 0 && ddx[k] <= 0) ? 1 : 0;
+        if (near)
+            t.E[k] = vx[oi[k]] * ddy[k] - vy[oi[k]] * ddx[k] - bias;
+        else
+            t.E[k] = clampEdge((S64)vx[oi[k]] * ddy[k] - (S64)vy[oi[k]] * ddx[k] - bias);
+    }
     return t;
 }
 
 __device__ __forceinline__ bool edgesCover(const S32* E, const S32* A, const S32* B, S32 qx, S32 qy) {
-    return (E[0] + A[0] * qx + B[0] * qy >= 0) && (E[1] + A[1] * qx + B[1] * qy >= 0) &&
-           (E[2] + A[2] * qx + B[2] * qy >= 0);
+    return ((E[0] + A[0] * qx + B[0] * qy) | (E[1] + A[1] * qx + B[1] * qy) | (E[2] + A[2] * qx + B[2] * qy)) >= 0;
 }
 
 // Exact sample mask of pixel (px, py) of the tile.
@@ -198,6 +211,69 @@ __device__ __forceinline__ U32 sampleMaskOf(const S32* E, const S32* A, const S3
         if (edgesCover(E, A, B, (px << kSubpixelLog2) + sampleOffsetX(S, i), (py << kSubpixelLog2) + sampleOffsetY(S, i)))
             m |= 1u << i;
     return m;
+}
+
+// Steps of an edge as two signed 16-bit halves, for triangles of at most 32,767
+// subpixels (2,048 pixels) across; larger ones take farEdges.
+__device__ __forceinline__ bool packable(const TileEdges& t) {
+    return max(t.maxX - t.minX, t.maxY - t.minY) <= 32767;
+}
+__device__ __forceinline__ TriRec packTri(const TileEdges& t, uint4 z, U32 id, U32 box) {
+    U32 E[3], AB[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        E[k] = (U32)(t.E[k] - 8 * (t.A[k] + t.B[k]));
+        AB[k] = __byte_perm((U32)t.A[k], (U32)t.B[k], 0x5410);
+    }
+    return TriRec{make_uint4(E[0], E[1], E[2], AB[0]), make_uint4(AB[1], AB[2], z.x, z.y), make_uint4(z.z, id, box, 0u)};
+}
+// Byte pair of pixel (px, py)'s centre, and the step to sample i.
+__device__ __forceinline__ S32 packedPixel(S32 px, S32 py) { return ((px | py << 8) << kSubpixelLog2) + 0x0808; }
+__host__ __device__ constexpr S32 packedSample(int s, int i) { return sampleOffsetX(s, i) + 256 * sampleOffsetY(s, i); }
+
+// Negative iff the sample at byte pair q is not covered.
+__device__ __forceinline__ S32 packedEdges(uint4 r0, U32 ab1, U32 ab2, S32 q) {
+    return __dp2a_lo((S32)r0.w, q, (S32)r0.x) | __dp2a_lo((S32)ab1, q, (S32)r0.y) | __dp2a_lo((S32)ab2, q, (S32)r0.z);
+}
+// Exact sample mask of the pixel at byte pair q.
+template <int S>
+__device__ __forceinline__ U32 packedMask(uint4 r0, U32 ab1, U32 ab2, S32 q) {
+    U32 m = 0;
+#pragma unroll
+    for (int i = 0; i < (1 << S); i++)
+        if (packedEdges(r0, ab1, ab2, q + packedSample(S, i)) >= 0) m |= 1u << i;
+    return m;
+}
+// Whether the pixel can hold covered samples (exact at one sample).
+template <int S>
+__device__ __forceinline__ bool packedCover(uint4 r0, U32 ab1, U32 ab2, S32 q) {
+    if (S == 0) return packedEdges(r0, ab1, ab2, q) >= 0;
+    const U32 E[3] = {r0.x, r0.y, r0.z}, AB[3] = {r0.w, ab1, ab2};
+    S32 any = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        any |= __dp2a_lo((S32)AB[k], q, (S32)E[k]) + ((abs(lo16(AB[k])) + abs(hi16(AB[k]))) << (kSubpixelLog2 - 1));
+    return any >= 0;
+}
+template <int S>
+__device__ __forceinline__ bool edgesMayCover(const TileEdges& t, S32 px, S32 py) {
+    S32 any = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const S32 slack = (S == 0) ? 0 : (abs(t.A[k]) + abs(t.B[k])) << (kSubpixelLog2 - 1);
+        any |= t.E[k] + t.A[k] * (px << kSubpixelLog2) + t.B[k] * (py << kSubpixelLog2) + slack;
+    }
+    return any >= 0;
+}
+
+// Slot of a list entry's subtriangle, and the edges of a triangle that a record
+// cannot hold, formed anew wherever they are needed.
+__device__ __forceinline__ S64 entrySlotOf(const DrawDev& d, U32 entry) {
+    const U32 tri = entry >> 3, sub = entry & 7;
+    return (sub == 7) ? (S64)tri : (S64)__ldg(&d.triHeader[tri].w) + sub;
+}
+__device__ __forceinline__ TileEdges farEdges(const DrawDev& d, S32 listIndex, S32 cx0, S32 cy0) {
+    return tileEdges(__ldg(&d.triHeader[entrySlotOf(d, __ldg(&d.tileList[listIndex]))]), cx0, cy0);
 }
 
 // Depth of sample i of pixel (X, Y) (FineRaster.inl:695, 1047, 1096).
@@ -216,6 +292,21 @@ __device__ __forceinline__ bool pixelBox(const TileEdges& t, S32& bx0, S32& bx1,
     by0 = max(0, (t.minY - pad + 15) >> kSubpixelLog2);
     by1 = min(7, (t.maxY + pad) >> kSubpixelLog2);
     return bx0 <= bx1 && by0 <= by1;
+}
+
+// A small triangle's pixel box as bx0 | by0 << 4 | w << 8 | m << 12, where
+// m = ceil(2^8 / w) gives the row of the box's pixel k as (k * m) >> 8, exact
+// for k < 64 and w <= 8 (the error k * (m * w - 256) stays below 256). m - 1
+// comes from a table in two registers, since a division takes some 20
+// instructions.
+__device__ __forceinline__ U32 packBox(S32 bx0, S32 by0, S32 w) {
+    const U32 m = (__byte_perm(0x3F557FFFu, 0x1F242A33u, (U32)(w - 1)) & 0xFFu) + 1u;
+    return (U32)bx0 | (U32)by0 << 4 | (U32)w << 8 | m << 12;
+}
+__device__ __forceinline__ void boxPixel(U32 box, S32 k, S32& px, S32& py) {
+    const S32 q = (S32)(((U32)k * (box >> 12)) >> 8);
+    px = (S32)(box & 0xFu) + k - q * (S32)((box >> 8) & 0xFu);
+    py = (S32)((box >> 4) & 0xFu) + q;
 }
 
 // Runs the fragment shader of triangle data td (16 words) at pixel (X, Y).
@@ -310,45 +401,70 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
         U32* gDepth = (U32*)__ldg((const unsigned long long*)&in->depth);
         const S64 tileOrigin = (S64)(ty * 8) * rowWords + (S64)tx * 8 * NS;
 
-        // Load or clear the tile (FineRaster.inl:562-580, 916-934), and its
-        // maximum depth for early Z.
-        U32 tileZMax = 0;
-        if constexpr (kVisibility) {
-            // Visibility keys start as depth << 32 (no fragment yet).
-            U32 z = 0;
-            if (clear) {
-                const U32 cc = __ldg(&in->clearColor), cd = __ldg(&in->clearDepth);
-                for (int w = lane; w < TW; w += 32) { sm.color[w] = cc; sm.key[w] = (U64)cd << 32; }
-                z = cd;
+        // The tile's words move two per lane and step, 64 words (8 / NS rows) a
+        // step, where the surfaces allow 8-byte accesses; one by one otherwise.
+        const bool wide = (((U64)gColor | (U64)gDepth) & 7u) == 0;
+        const S64 wideOrigin = tileOrigin + (S64)(lane / (4 * NS)) * rowWords + 2 * (lane % (4 * NS));
+        const S64 wideStep = (8 / NS) * rowWords;
+        if (count == 0) {
+            // A cleared tile that no triangle touches.
+            const U32 cc = __ldg(&in->clearColor), cd = __ldg(&in->clearDepth);
+            if (wide) {
+#pragma unroll
+                for (int i = 0; i < NS; i++) {
+                    *reinterpret_cast<uint2*>(&gColor[wideOrigin + i * wideStep]) = make_uint2(cc, cc);
+                    *reinterpret_cast<uint2*>(&gDepth[wideOrigin + i * wideStep]) = make_uint2(cd, cd);
+                }
             } else {
                 for (int w = lane; w < TW; w += 32) {
-                    S64 g = tileOrigin + (S64)(w / (8 * NS)) * rowWords + (w % (8 * NS));
+                    const S64 g = tileOrigin + (S64)(w / (8 * NS)) * rowWords + (w % (8 * NS));
+                    gColor[g] = cc;
+                    gDepth[g] = cd;
+                }
+            }
+            continue;
+        }
+
+        // Load or clear the tile (FineRaster.inl:562-580, 916-934), and its
+        // maximum depth for early Z. Visibility keys start as depth << 32 (no
+        // fragment yet).
+        U32 tileZMax = 0;
+        auto putDepth = [&](int w, U32 z) {
+            if constexpr (kVisibility) sm.key[w] = (U64)z << 32; else sm.depth[w] = z;
+        };
+        if (clear) {
+            const U32 cc = __ldg(&in->clearColor), cd = __ldg(&in->clearDepth);
+#pragma unroll
+            for (int w = lane; w < TW; w += 32) {
+                sm.color[w] = cc;
+                putDepth(w, cd);
+            }
+            tileZMax = cd;
+        } else {
+            U32 z = 0;
+            if (wide) {
+#pragma unroll
+                for (int i = 0; i < NS; i++) {
+                    const int w = 2 * lane + 64 * i;
+                    const uint2 c = *reinterpret_cast<const uint2*>(&gColor[wideOrigin + i * wideStep]);
+                    const uint2 dz = *reinterpret_cast<const uint2*>(&gDepth[wideOrigin + i * wideStep]);
+                    *reinterpret_cast<uint2*>(&sm.color[w]) = c;
+                    putDepth(w, dz.x);
+                    putDepth(w + 1, dz.y);
+                    z = max(z, max(dz.x, dz.y));
+                }
+            } else {
+                for (int w = lane; w < TW; w += 32) {
+                    const S64 g = tileOrigin + (S64)(w / (8 * NS)) * rowWords + (w % (8 * NS));
                     sm.color[w] = gColor[g];
                     const U32 dz = gDepth[g];
-                    sm.key[w] = (U64)dz << 32;
+                    putDepth(w, dz);
                     z = max(z, dz);
                 }
             }
-            tileZMax = __reduce_max_sync(0xFFFFFFFFu, z);
-            __syncwarp();
-        } else {
-            if (clear) {
-                const U32 cc = __ldg(&in->clearColor), cd = __ldg(&in->clearDepth);
-                for (int w = lane; w < TW; w += 32) { sm.color[w] = cc; sm.depth[w] = cd; }
-            } else {
-                for (int w = lane; w < TW; w += 32) {
-                    S64 g = tileOrigin + (S64)(w / (8 * NS)) * rowWords + (w % (8 * NS));
-                    sm.color[w] = gColor[g];
-                    sm.depth[w] = gDepth[g];
-                }
-            }
-            __syncwarp();
-            if (kDepth) {
-                U32 z = 0;
-                for (int w = lane; w < TW; w += 32) z = max(z, sm.depth[w]);
-                tileZMax = __reduce_max_sync(0xFFFFFFFFu, z);
-            }
+            if (kDepth) tileZMax = __reduce_max_sync(0xFFFFFFFFu, z);
         }
+        __syncwarp();
 
         // Pixel (0, 0) centre of the tile in the header frame.
         const S32 cx0 = ((tx * 8) << kSubpixelLog2) - ((width - 1) << (kSubpixelLog2 - 1));
@@ -379,11 +495,10 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                 // pixels per lane. Keys resolve by atomic minimum, so the
                 // order pairs are taken in does not change a bit.
                 S32 n = 0;
-                bool big = false;
+                bool big = false, far = false;
                 if (batch + lane < count) {
                     const U32 entry = __ldg(&d.tileList[start + batch + lane]);
-                    const U32 tri = entry >> 3, sub = entry & 7;
-                    const S64 slot = (sub == 7) ? (S64)tri : (S64)__ldg(&d.triHeader[tri].w) + sub;
+                    const S64 slot = entrySlotOf(d, entry);
                     const uint4 h = __ldg(&d.triHeader[slot]);
                     if ((h.w & 0xFFFFF000u) < tileZMax) {
                         const TileEdges te = tileEdges(h, cx0, cy0);
@@ -392,17 +507,10 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                             const uint4 q0 = __ldg(&d.triData[slot * 4]);
                             const S32 w = bx1 - bx0 + 1;
                             const S32 cnt = w * (by1 - by0 + 1);
-                            big = cnt > selfPixels;
-                            sm.order[lane] = entry - entryBase + 1u;
-                            sm.rec[lane].q[0] = make_uint4((U32)te.E[0], (U32)te.E[1], (U32)te.E[2], (U32)te.A[0]);
-                            sm.rec[lane].q[1] = make_uint4((U32)te.A[1], (U32)te.A[2], (U32)te.B[0], (U32)te.B[1]);
-                            sm.rec[lane].q[2] = make_uint4((U32)te.B[2], q0.x, q0.y, q0.z);
-                            if (!big) {
-                                n = cnt;
-                                // Row of box pixel k: (k * ceil(2^16 / w)) >> 16, exact for k < 64, w <= 8.
-                                sm.box[lane] = (U32)bx0 | (U32)by0 << 4 | (U32)w << 8 |
-                                               ((65536u + (U32)w - 1u) / (U32)w) << 12;
-                            }
+                            far = !packable(te);
+                            big = !far && cnt > selfPixels;
+                            if (!far && !big) n = cnt;
+                            sm.rec[lane] = packTri(te, q0, entry - entryBase + 1u, packBox(bx0, by0, w));
                         }
                     }
                 }
@@ -437,20 +545,16 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                     const S32 p = base + lane;
                     if (p >= P) continue;
                     const S32 k = p - first;
-                    const U32 bw = sm.box[j];
-                    const S32 w = (S32)((bw >> 8) & 0xFu);
-                    const S32 q = (S32)(((U32)k * (bw >> 12)) >> 16);
-                    const S32 px = (S32)(bw & 0xFu) + k - q * w, py = (S32)((bw >> 4) & 0xFu) + q;
-                    const uint4 r0 = sm.rec[j].q[0], r1 = sm.rec[j].q[1], r2 = sm.rec[j].q[2];
-                    const S32 E[3] = {(S32)r0.x, (S32)r0.y, (S32)r0.z};
-                    const S32 A[3] = {(S32)r0.w, (S32)r1.x, (S32)r1.y};
-                    const S32 B[3] = {(S32)r1.z, (S32)r1.w, (S32)r2.x};
-                    const U32 smask = sampleMaskOf<S>(E, A, B, px, py);
+                    S32 px, py;
+                    boxPixel(sm.rec[j].q[2].z, k, px, py);
+                    const uint4 r0 = sm.rec[j].q[0], r1 = sm.rec[j].q[1];
+                    const U32 smask = packedMask<S>(r0, r1.x, r1.y, packedPixel(px, py));
                     if (!smask) continue;
-                    const U32 order = sm.order[j];
+                    const uint2 r2 = *reinterpret_cast<const uint2*>(&sm.rec[j].q[2]);
+                    const U32 order = r2.y;
                     const U64 low = packed ? (order << NS | smask) : order;
                     const U32 X = (U32)(tx * 8 + px), Y = (U32)(ty * 8 + py);
-                    const U32 zx = r2.y, zy = r2.z, zb = r2.w;
+                    const U32 zx = r1.z, zy = r1.w, zb = r2.x;
 #pragma unroll
                     for (int i = 0; i < NS; i++) {
                         if (!(smask >> i & 1)) continue;
@@ -463,64 +567,67 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                 // Larger triangles: the whole warp, one at a time, in batch
                 // order (each lane owns its two pixels, so plain stores
                 // suffice). At one sample a lane keeps its two keys in
-                // registers over all of them: the row below is 4 pixels
-                // (64 subpixels) down, so its edge values are the first
-                // row's plus 64 B and its depth the first's plus 4 zy; a
-                // sample is covered iff no edge value is negative, i.e. iff
-                // their OR is not.
+                // registers over all of them; the row below is 4 pixels down.
                 const S32 px = lane & 7, py0 = lane >> 3, py1 = py0 + 4;
                 const U32 pX = (U32)(tx * 8 + px), pY0 = (U32)(ty * 8 + py0), pY1 = pY0 + 4;
+                const S32 pq0 = packedPixel(px, py0), pq1 = packedPixel(px, py1);
                 U32 bigMask = __ballot_sync(0xFFFFFFFFu, big);
                 if (S == 0 && bigMask) {
                     const int idx0 = py0 * 8 + px, idx1 = idx0 + 32;
                     U64 k0 = sm.key[idx0], k1 = sm.key[idx1];
-                    const S32 qx = px << kSubpixelLog2, qy = py0 << kSubpixelLog2;
                     for (; bigMask; bigMask &= bigMask - 1) {
                         const int j = __ffs(bigMask) - 1;
-                        const uint4 r0 = sm.rec[j].q[0], r1 = sm.rec[j].q[1], r2 = sm.rec[j].q[2];
-                        const S32 e00 = (S32)r0.x + (S32)r0.w * qx + (S32)r1.z * qy;
-                        const S32 e01 = (S32)r0.y + (S32)r1.x * qx + (S32)r1.w * qy;
-                        const S32 e02 = (S32)r0.z + (S32)r1.y * qx + (S32)r2.x * qy;
-                        const S32 e10 = e00 + ((S32)r1.z << (kSubpixelLog2 + 2));
-                        const S32 e11 = e01 + ((S32)r1.w << (kSubpixelLog2 + 2));
-                        const S32 e12 = e02 + ((S32)r2.x << (kSubpixelLog2 + 2));
-                        const U32 z0 = r2.y * pX + r2.z * pY0 + r2.w, z1 = z0 + (r2.z << 2);
-                        const U32 order = sm.order[j];
-                        const U64 key0 = ((U64)z0 << 32) | order, key1 = ((U64)z1 << 32) | order;
-                        if ((e00 | e01 | e02) >= 0 && key0 < k0) k0 = key0;
-                        if ((e10 | e11 | e12) >= 0 && key1 < k1) k1 = key1;
+                        const uint4 r0 = sm.rec[j].q[0], r1 = sm.rec[j].q[1];
+                        const uint2 r2 = *reinterpret_cast<const uint2*>(&sm.rec[j].q[2]);
+                        const U32 z0 = r1.z * pX + r1.w * pY0 + r2.x, z1 = z0 + (r1.w << 2);
+                        const U64 key0 = ((U64)z0 << 32) | r2.y, key1 = ((U64)z1 << 32) | r2.y;
+                        if (packedEdges(r0, r1.x, r1.y, pq0) >= 0 && key0 < k0) k0 = key0;
+                        if (packedEdges(r0, r1.x, r1.y, pq1) >= 0 && key1 < k1) k1 = key1;
                     }
                     sm.key[idx0] = k0;
                     sm.key[idx1] = k1;
                 }
+                auto lowerKeys = [&](U32 smask, S32 pyy, U32 Y, U32 zx, U32 zy, U32 zb, U32 order) {
+                    const U64 low = packed ? (order << NS | smask) : order;
+#pragma unroll
+                    for (int i = 0; i < NS; i++) {
+                        if (!(smask >> i & 1)) continue;
+                        const int idx = pyy * 8 * NS + i * 8 + px;
+                        const U64 key = ((U64)sampleDepth<S>(zx, zy, zb, pX, Y, i) << 32) | low;
+                        if (key < sm.key[idx]) sm.key[idx] = key;
+                    }
+                };
                 for (; bigMask; bigMask &= bigMask - 1) {
                     const int j = __ffs(bigMask) - 1;
-                    const uint4 r0 = sm.rec[j].q[0], r1 = sm.rec[j].q[1], r2 = sm.rec[j].q[2];
-                    const S32 E[3] = {(S32)r0.x, (S32)r0.y, (S32)r0.z};
-                    const S32 A[3] = {(S32)r0.w, (S32)r1.x, (S32)r1.y};
-                    const S32 B[3] = {(S32)r1.z, (S32)r1.w, (S32)r2.x};
-                    const U32 zx = r2.y, zy = r2.z, zb = r2.w;
-                    const U32 order = sm.order[j];
-#pragma unroll
+                    const uint4 r0 = sm.rec[j].q[0], r1 = sm.rec[j].q[1];
+                    const uint2 r2 = *reinterpret_cast<const uint2*>(&sm.rec[j].q[2]);
+#pragma unroll 1
+                    for (int half = 0; half < 2; half++)
+                        lowerKeys(packedMask<S>(r0, r1.x, r1.y, half ? pq1 : pq0), half ? py1 : py0, half ? pY1 : pY0, r1.z,
+                                  r1.w, r2.x, r2.y);
+                }
+                // Those whose steps a record cannot hold (over 2,048 pixels across).
+                for (U32 farMask = __ballot_sync(0xFFFFFFFFu, far); farMask; farMask &= farMask - 1) {
+                    const int j = __ffs(farMask) - 1;
+                    const TileEdges te = farEdges(d, start + batch + j, cx0, cy0);
+                    const uint4 r1 = sm.rec[j].q[1], r2 = sm.rec[j].q[2];
+#pragma unroll 1
                     for (int half = 0; half < 2; half++) {
-                        const S32 pyy = half ? py1 : py0;
-                        const U32 Y = half ? pY1 : pY0;
-                        const U32 smask = sampleMaskOf<S>(E, A, B, px, pyy);
-                        const U64 low = packed ? (order << NS | smask) : order;
-#pragma unroll
-                        for (int i = 0; i < NS; i++) {
-                            if (!(smask >> i & 1)) continue;
-                            const int idx = pyy * 8 * NS + i * 8 + px;
-                            const U64 key = ((U64)sampleDepth<S>(zx, zy, zb, pX, Y, i) << 32) | low;
-                            if (key < sm.key[idx]) sm.key[idx] = key;
-                        }
+                        const S32 py = half ? py1 : py0;
+                        lowerKeys(sampleMaskOf<S>(te.E, te.A, te.B, px, py), py, half ? pY1 : pY0, r1.z, r1.w, r2.x, r2.y);
                     }
                 }
                 __syncwarp();
                 // Exact current depth maximum for the next batch's early Z.
-                U32 z = 0;
-                for (int w = lane; w < TW; w += 32) z = max(z, (U32)(sm.key[w] >> 32));
-                tileZMax = __reduce_max_sync(0xFFFFFFFFu, z);
+                if (batch + 32 < count) {
+                    U32 z = 0;
+#pragma unroll
+                    for (int w = 2 * lane; w < TW; w += 64) {
+                        const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(&sm.key[w]);
+                        z = max(z, max((U32)(k.x >> 32), (U32)(k.y >> 32)));
+                    }
+                    tileZMax = __reduce_max_sync(0xFFFFFFFFu, z);
+                }
             } else {
                 // ---- 1. One triangle per lane: its words in shared memory, and
                 // the pixels of the small ones (box of at most selfPixels pixels)
@@ -529,10 +636,9 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                 // depend on the order the pairs are taken in).
                 bool valid = batch + lane < count;
                 bool self = false;     // small triangle: covered through the pairs
+                bool far = false;      // its steps do not fit a record
                 U32 myLo = 0, myHi = 0;
                 S32 n = 0;
-                U32* pairBox = sm.pairBox;
-                U32* pairMul = sm.pairMul;
                 sm.covLo[lane] = 0u;
                 sm.covHi[lane] = 0u;
                 // Batch filter (see step 2b): exact for single-sample depth-tested
@@ -544,8 +650,8 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                 }
                 if (valid) {
                     U32 entry = __ldg(&d.tileList[start + batch + lane]);
-                    U32 tri = entry >> 3, sub = entry & 7;
-                    S64 slot = (sub == 7) ? (S64)tri : (S64)__ldg(&d.triHeader[tri].w) + sub;
+                    const U32 tri = entry >> 3;
+                    const S64 slot = entrySlotOf(d, entry);
                     uint4 h = __ldg(&d.triHeader[slot]);
                     if (kDepth && (h.w & 0xFFFFF000u) >= tileZMax) valid = false;
                     if (valid) {
@@ -555,26 +661,12 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                         S32 bx0, bx1, by0, by1;
                         const bool inTile = pixelBox<S>(te, bx0, bx1, by0, by1);
                         const S32 w = bx1 - bx0 + 1;
-                        self = !inTile || w * (by1 - by0 + 1) <= selfPixels;
-#pragma unroll
-                        for (int k = 0; k < 3; k++) {
-                            sm.E[k][lane] = te.E[k];
-                            sm.A[k][lane] = te.A[k];
-                            sm.B[k][lane] = te.B[k];
-                        }
-                        sm.td[0][lane] = q0.x; sm.td[1][lane] = q0.y; sm.td[2][lane] = q0.z; sm.td[3][lane] = q0.w;
-                        uint4 q1 = __ldg(&tdp[1]), q2 = __ldg(&tdp[2]), q3 = __ldg(&tdp[3]);
-                        sm.td[4][lane] = q1.x; sm.td[5][lane] = q1.y; sm.td[6][lane] = q1.z; sm.td[7][lane] = q1.w;
-                        sm.td[8][lane] = q2.x; sm.td[9][lane] = q2.y; sm.td[10][lane] = q2.z; sm.td[11][lane] = q2.w;
-                        sm.td[12][lane] = q3.x; sm.td[13][lane] = q3.y; sm.td[14][lane] = q3.z; sm.td[15][lane] = q3.w;
-                        sm.tri[lane] = (S32)((S64)tri - triBase);
+                        far = inTile && !packable(te);
+                        self = !inTile || (!far && w * (by1 - by0 + 1) <= selfPixels);
+                        sm.rec[lane] = packTri(te, q0, (U32)((S64)tri - triBase), inTile ? packBox(bx0, by0, w) : 0u);
+                        sm.data[lane] = TriRec{__ldg(&tdp[1]), __ldg(&tdp[2]), __ldg(&tdp[3])};
                         // No pixel of the tile can be covered (!inTile): nothing to do.
-                        if (inTile && self) {
-                            n = w * (by1 - by0 + 1);
-                            pairBox[lane] = (U32)bx0 | (U32)by0 << 4 | (U32)w << 8;
-                            // Row of box pixel k: (k * ceil(2^16 / w)) >> 16, exact for k < 64, w <= 8.
-                            pairMul[lane] = (65536u + (U32)w - 1u) / (U32)w;
-                        }
+                        if (inTile && self) n = w * (by1 - by0 + 1);
                     }
                 }
                 S32 P = 0;
@@ -597,21 +689,15 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                     for (int s2 = 16; s2 > 0; s2 >>= 1)
                         if (sm.fragEnd[j + s2 - 1] <= p) j += s2;
                     const S32 k = p - (j ? sm.fragEnd[j - 1] : 0);
-                    const U32 bw = pairBox[j];
-                    const S32 w = (S32)(bw >> 8);
-                    const S32 q = (S32)(((U32)k * pairMul[j]) >> 16);
-                    const S32 px = (S32)(bw & 0xFu) + k - q * w, py = (S32)((bw >> 4) & 0xFu) + q;
-                    const S32 qx = px << kSubpixelLog2, qy = py << kSubpixelLog2;
-                    bool c = true;
-#pragma unroll
-                    for (int e = 0; e < 3; e++) {
-                        const S32 a = sm.A[e][j], b = sm.B[e][j];
-                        const S32 slack = (S == 0) ? 0 : (abs(a) + abs(b)) << (kSubpixelLog2 - 1);
-                        c = c && (sm.E[e][j] + a * qx + b * qy + slack >= 0);
-                    }
+                    S32 px, py;
+                    boxPixel(sm.rec[j].q[2].z, k, px, py);
+                    const uint4 r0 = sm.rec[j].q[0];
+                    const uint2 ab = *reinterpret_cast<const uint2*>(&sm.rec[j].q[1]);
+                    bool c = packedCover<S>(r0, ab.x, ab.y, packedPixel(px, py));
                     if (kDepth && S == 0 && !kQuads && c) {
                         const U32 X = (U32)(tx * 8 + px), Y = (U32)(ty * 8 + py);
-                        const U32 z = sm.td[0][j] * X + sm.td[1][j] * Y + sm.td[2][j];
+                        const uint2 zxy = *reinterpret_cast<const uint2*>(&sm.rec[j].q[1].z);
+                        const U32 z = zxy.x * X + zxy.y * Y + sm.rec[j].q[2].x;
                         c = z < sm.depth[py * 8 + px];
                         if constexpr (kFilter)
                             if (c) atomicMin((unsigned long long*)&sm.batchMin[py * 8 + px], ((unsigned long long)z << 32) | (U32)j);
@@ -633,6 +719,7 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                 }
                 __syncwarp();
                 const U32 coopMask = __ballot_sync(0xFFFFFFFFu, valid && !self);
+                const U32 farMask = __ballot_sync(0xFFFFFFFFu, valid && far);
 
                 // ---- 2. Large triangles, two pixels per lane.
                 const S32 px = lane & 7, py0 = lane >> 3, py1 = py0 + 4;
@@ -646,21 +733,10 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                         curZ0 = sm.depth[lane];
                         curZ1 = sm.depth[lane + 32];
                     }
-                    const S32 qx = px << kSubpixelLog2, qy0 = py0 << kSubpixelLog2, qy1 = py1 << kSubpixelLog2;
-                    for (U32 m = coopMask; m; m &= m - 1) {
-                        const int j = __ffs(m) - 1;
-                        bool c0 = true, c1 = true;
-#pragma unroll
-                        for (int k = 0; k < 3; k++) {
-                            S32 e = sm.E[k][j], a = sm.A[k][j], b = sm.B[k][j];
-                            S32 base = e + a * qx;
-                            S32 slack = (S == 0) ? 0 : (abs(a) + abs(b)) << (kSubpixelLog2 - 1);
-                            c0 = c0 && (base + b * qy0 + slack >= 0);
-                            c1 = c1 && (base + b * qy1 + slack >= 0);
-                        }
+                    const S32 pq0 = packedPixel(px, py0), pq1 = packedPixel(px, py1);
+                    auto setCoverage = [&](int j, bool c0, bool c1, U32 zx, U32 zy) {
                         if (kDepth && S == 0 && !kQuads) {
-                            const U32 zx = sm.td[0][j], zy = sm.td[1][j], zb = sm.td[2][j];
-                            const U32 z0 = zx * pX + zy * pY0 + zb, z1 = z0 + zy * 4u;
+                            const U32 z0 = zx * pX + zy * pY0 + sm.rec[j].q[2].x, z1 = z0 + zy * 4u;
                             c0 = c0 && (z0 < curZ0);
                             c1 = c1 && (z1 < curZ1);
                             if constexpr (kFilter) {
@@ -669,9 +745,20 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                                 if (c1 && k1 < min1) min1 = k1;
                             }
                         }
-                        U32 lo = __ballot_sync(0xFFFFFFFFu, c0);
-                        U32 hi = __ballot_sync(0xFFFFFFFFu, c1);
+                        const U32 lo = __ballot_sync(0xFFFFFFFFu, c0);
+                        const U32 hi = __ballot_sync(0xFFFFFFFFu, c1);
                         if (lane == j) { myLo = lo; myHi = hi; }
+                    };
+                    for (U32 m = coopMask & ~farMask; m; m &= m - 1) {
+                        const int j = __ffs(m) - 1;
+                        const uint4 r0 = sm.rec[j].q[0], r1 = sm.rec[j].q[1];
+                        setCoverage(j, packedCover<S>(r0, r1.x, r1.y, pq0), packedCover<S>(r0, r1.x, r1.y, pq1), r1.z, r1.w);
+                    }
+                    for (U32 m = farMask; m; m &= m - 1) {
+                        const int j = __ffs(m) - 1;
+                        const TileEdges te = farEdges(d, start + batch + j, cx0, cy0);
+                        const uint2 zxy = *reinterpret_cast<const uint2*>(&sm.rec[j].q[1].z);
+                        setCoverage(j, edgesMayCover<S>(te, px, py0), edgesMayCover<S>(te, px, py1), zxy.x, zxy.y);
                     }
                 }
                 if (kQuads) {
@@ -763,16 +850,20 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                         if (S == 0 && !kQuads) {
                             sampleMask = 1;  // single-sample masks are exact
                         } else {
-                            const S32 E[3] = {sm.E[0][j], sm.E[1][j], sm.E[2][j]};
-                            const S32 A[3] = {sm.A[0][j], sm.A[1][j], sm.A[2][j]};
-                            const S32 B[3] = {sm.B[0][j], sm.B[1][j], sm.B[2][j]};
-                            sampleMask = sampleMaskOf<S>(E, A, B, fx, fy);
+                            const uint4 r0 = sm.rec[j].q[0], r1 = sm.rec[j].q[1];
+                            if (farMask >> j & 1u) {
+                                const TileEdges te = farEdges(d, start + batch + j, cx0, cy0);
+                                sampleMask = sampleMaskOf<S>(te.E, te.A, te.B, fx, fy);
+                            } else {
+                                sampleMask = packedMask<S>(r0, r1.x, r1.y, packedPixel(fx, fy));
+                            }
                         }
                         covered = sampleMask != 0;
                         if (!kQuads && !covered) act = false;
                         const U32 X = (U32)(tx * 8 + fx), Y = (U32)(ty * 8 + fy);
                         if (kDepth) {
-                            const U32 zx = sm.td[0][j], zy = sm.td[1][j], zb = sm.td[2][j];
+                            const uint2 r1 = *reinterpret_cast<const uint2*>(&sm.rec[j].q[1].z);
+                            const U32 zx = r1.x, zy = r1.y, zb = sm.rec[j].q[2].x;
                             bool anyPass = false;
                             const int rowBase = fy * 8 * NS + fx;
 #pragma unroll
@@ -791,8 +882,11 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                     if (act) {
                         U32 td[16];
 #pragma unroll
-                        for (int q = 0; q < 16; q++) td[q] = sm.td[q][j];
-                        src = shadeFragment<FS, S, F>(td, sm.tri[j], tx * 8 + (pixel & 7), ty * 8 + (pixel >> 3), sampleMask,
+                        for (int q = 0; q < 3; q++) {
+                            const uint4 v = sm.data[j].q[q];
+                            td[4 + 4 * q] = v.x; td[5 + 4 * q] = v.y; td[6 + 4 * q] = v.z; td[7 + 4 * q] = v.w;
+                        }
+                        src = shadeFragment<FS, S, F>(td, (S32)sm.rec[j].q[2].y, tx * 8 + (pixel & 7), ty * 8 + (pixel >> 3), sampleMask,
                                                       verts, stride4, sm.shared, shadeMask, discard);
                     }
                     // ROP: same-pixel fragments of this pass applied in lane order.
@@ -816,7 +910,7 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                                         if (!(dz[i] < sm.depth[idx])) continue;
                                         sm.depth[idx] = dz[i];
                                     }
-                                    bs.m_triIdx = sm.tri[j];
+                                    bs.m_triIdx = (S32)sm.rec[j].q[2].y;
                                     bs.m_pixelPos = FW::Vec2i(tx * 8 + fx, ty * 8 + fy);
                                     bs.m_sampleIdx = i;
                                     bs.m_src = src;
@@ -831,7 +925,7 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                         }
                     }
                 }
-                if (kDepth) {
+                if (kDepth && batch + 32 < count) {
                     U32 z = 0;
                     for (int w = lane; w < TW; w += 32) z = max(z, sm.depth[w]);
                     tileZMax = __reduce_max_sync(0xFFFFFFFFu, z);
@@ -855,8 +949,6 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
             for (int hh = 0; hh < 2; hh++) {
                 const int p = lane + 32 * hh;
                 const int rowBase = (p >> 3) * 8 * NS + (p & 7);
-                U32 mine[NS];
-                int cnt = 0;
 #pragma unroll
                 for (int i0 = 0; i0 < NS; i0++) {
                     const U32 low = (U32)sm.key[rowBase + i0 * 8];
@@ -864,27 +956,16 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
 #pragma unroll
                     for (int i = 0; i < i0; i++)
                         if ((U32)sm.key[rowBase + i * 8] == low) first = false;
-                    U32 won = 0;
+                    const U32 firsts = __ballot_sync(0xFFFFFFFFu, first);
                     if (first) {
+                        U32 won = 0;
 #pragma unroll
                         for (int i = 0; i < NS; i++)
                             if ((U32)sm.key[rowBase + i * 8] == low) won |= 1u << i;
+                        winners[nw + __popc(firsts & ltMask)] = (U32)p | (U32)i0 << 6 | won << 9;
                     }
-                    mine[i0] = (U32)p | (U32)i0 << 6 | won << 9;
-                    cnt += first ? 1 : 0;
+                    nw += __popc(firsts);
                 }
-                S32 pos = cnt;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const S32 t = __shfl_up_sync(0xFFFFFFFFu, pos, o);
-                    if (lane >= o) pos += t;
-                }
-                const S32 total = __shfl_sync(0xFFFFFFFFu, pos, 31);
-                pos += nw - cnt;
-#pragma unroll
-                for (int i0 = 0; i0 < NS; i0++)
-                    if (mine[i0] >> 9) winners[pos++] = mine[i0];
-                nw += total;
             }
             __syncwarp();
             for (S32 w0 = 0; w0 < nw; w0 += 32) {
@@ -897,9 +978,8 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                 U32 low = (U32)sm.key[rowBase + i0 * 8];
                 U32 td[16];
                 const U32 entry = (packed ? low >> NS : low) - 1u + entryBase;
-                const U32 sub = entry & 7;
                 const U32 tri = entry >> 3;
-                const S64 slot = (sub == 7) ? (S64)tri : (S64)__ldg(&d.triHeader[tri].w) + sub;
+                const S64 slot = entrySlotOf(d, entry);
                 const uint4* tdp = &d.triData[slot * 4];
                 const uint4 q1 = __ldg(&tdp[1]), q2 = __ldg(&tdp[2]), q3 = __ldg(&tdp[3]);
                 td[4] = q1.x; td[5] = q1.y; td[6] = q1.z; td[7] = q1.w;
@@ -937,26 +1017,51 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
         }
 
         // Write the tile back (FineRaster.inl:736-746).
-        for (int w = lane; w < TW; w += 32) {
-            S64 g = tileOrigin + (S64)(w / (8 * NS)) * rowWords + (w % (8 * NS));
-            gColor[g] = sm.color[w];
-            if constexpr (kVisibility)
-                gDepth[g] = (U32)(sm.key[w] >> 32);
-            else
-                gDepth[g] = sm.depth[w];
+        if (wide) {
+#pragma unroll
+            for (int i = 0; i < NS; i++) {
+                const int w = 2 * lane + 64 * i;
+                uint2 z;
+                if constexpr (kVisibility) {
+                    const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(&sm.key[w]);
+                    z = make_uint2((U32)(k.x >> 32), (U32)(k.y >> 32));
+                } else {
+                    z = *reinterpret_cast<const uint2*>(&sm.depth[w]);
+                }
+                *reinterpret_cast<uint2*>(&gColor[wideOrigin + i * wideStep]) = *reinterpret_cast<const uint2*>(&sm.color[w]);
+                *reinterpret_cast<uint2*>(&gDepth[wideOrigin + i * wideStep]) = z;
+            }
+        } else {
+            for (int w = lane; w < TW; w += 32) {
+                const S64 g = tileOrigin + (S64)(w / (8 * NS)) * rowWords + (w % (8 * NS));
+                gColor[g] = sm.color[w];
+                if constexpr (kVisibility)
+                    gDepth[g] = (U32)(sm.key[w] >> 32);
+                else
+                    gDepth[g] = sm.depth[w];
+            }
         }
         __syncwarp();
     }
 }
 
-// The fine-stage kernel. At one sample the register budget is pinned to five
-// resident CTAs per SM (48 registers); with MSAA the compiler's own choice
-// measured faster than any pinned budget (4x MSAA: 63 registers, 0.58 ms on
-// the 4K grid, against 0.60 ms pinned to four CTAs, 0.64 ms to three and
-// 0.645 ms to five, where 48 registers fit without spills but with more
-// instructions).
+// The fine-stage kernel, with a register budget by kind (fine stage in us,
+// budget taken against the other):
+//   one sample: five resident CTAs per SM (48 registers); with quads four,
+//     since their shaders spill at 48 (textured quads 395 against 416).
+//   MSAA, ordered: four (textured 4x terrain 868 against 965 with the
+//     compiler's own 80 registers).
+//   MSAA, visibility: the compiler's own choice (4x heightfield at 4K 606
+//     with 64 registers, 610 pinned to four CTAs; 8x soup 457 with 112
+//     registers, 518 pinned).
 template <class V, class FS, class BS, int S, U32 F>
-__global__ void __launch_bounds__(kFineMaxThreads, 5) fineKernel1(DrawDev d, int group, S32 tileBegin, S32 tileEnd) {
+__global__ void __launch_bounds__(kFineMaxThreads, FineTraits<FS, BS, S, F>::kQuads ? 4 : 5)
+    fineKernel1(DrawDev d, int group, S32 tileBegin, S32 tileEnd) {
+    fineTiles<V, FS, BS, S, F>(d, group, tileBegin, tileEnd);
+}
+template <class V, class FS, class BS, int S, U32 F>
+__global__ void __launch_bounds__(kFineMaxThreads, 4)
+    fineKernelMsaaOrdered(DrawDev d, int group, S32 tileBegin, S32 tileEnd) {
     fineTiles<V, FS, BS, S, F>(d, group, tileBegin, tileEnd);
 }
 template <class V, class FS, class BS, int S, U32 F>
@@ -967,8 +1072,10 @@ template <class V, class FS, class BS, int S, U32 F>
 constexpr auto fineKernelFor() {
     if constexpr (S == 0)
         return &fineKernel1<V, FS, BS, S, F>;
-    else
+    else if constexpr (FineTraits<FS, BS, S, F>::kVisibility)
         return &fineKernelMsaa<V, FS, BS, S, F>;
+    else
+        return &fineKernelMsaaOrdered<V, FS, BS, S, F>;
 }
 
 }  // namespace cr
