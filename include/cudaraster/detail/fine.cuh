@@ -14,9 +14,9 @@
 // word, an edge value in one dp2a), tiles move 8 bytes a lane, and tiles that
 // no triangle touches are written without passing through shared memory. These
 // took the stage from 84 to 80 us on the 1M soup, 107 to 96 on 20,000
-// triangles of 60 pixels, 627 to 606 on the heightfield, 613 to 457 on 300k
-// triangles at 8x MSAA, 160 to 152 on 300k blended ones, 471 to 457 on the
-// textured terrain.
+// triangles of 60 pixels, 627 to 577 on the heightfield (with pixelBox's tight
+// boxes), 613 to 455 on 300k triangles at 8x MSAA, 160 to 152 on 300k blended
+// ones, 471 to 453 on the textured terrain.
 //
 // Both paths deal the (triangle, pixel) pairs of the batch's small triangles
 // (pixel box of at most fineSelfPixels pixels) over the lanes; larger
@@ -202,6 +202,9 @@ __device__ __forceinline__ bool edgesCover(const S32* E, const S32* A, const S32
     return ((E[0] + A[0] * qx + B[0] * qy) | (E[1] + A[1] * qx + B[1] * qy) | (E[2] + A[2] * qx + B[2] * qy)) >= 0;
 }
 
+// Largest distance of a sample from its pixel's centre on either axis, in subpixels.
+__host__ __device__ constexpr S32 sampleReach(int s) { return s == 0 ? 0 : (1 << (kSubpixelLog2 - 1)) - (1 << (kSubpixelLog2 - 1 - s)); }
+
 // Exact sample mask of pixel (px, py) of the tile.
 template <int S>
 __device__ __forceinline__ U32 sampleMaskOf(const S32* E, const S32* A, const S32* B, S32 px, S32 py) {
@@ -252,7 +255,7 @@ __device__ __forceinline__ bool packedCover(uint4 r0, U32 ab1, U32 ab2, S32 q) {
     S32 any = 0;
 #pragma unroll
     for (int k = 0; k < 3; k++)
-        any |= __dp2a_lo((S32)AB[k], q, (S32)E[k]) + ((abs(lo16(AB[k])) + abs(hi16(AB[k]))) << (kSubpixelLog2 - 1));
+        any |= __dp2a_lo((S32)AB[k], q, (S32)E[k]) + (abs(lo16(AB[k])) + abs(hi16(AB[k]))) * sampleReach(S);
     return any >= 0;
 }
 template <int S>
@@ -260,7 +263,7 @@ __device__ __forceinline__ bool edgesMayCover(const TileEdges& t, S32 px, S32 py
     S32 any = 0;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        const S32 slack = (S == 0) ? 0 : (abs(t.A[k]) + abs(t.B[k])) << (kSubpixelLog2 - 1);
+        const S32 slack = (abs(t.A[k]) + abs(t.B[k])) * sampleReach(S);
         any |= t.E[k] + t.A[k] * (px << kSubpixelLog2) + t.B[k] * (py << kSubpixelLog2) + slack;
     }
     return any >= 0;
@@ -283,10 +286,13 @@ __device__ __forceinline__ U32 sampleDepth(U32 zx, U32 zy, U32 zb, U32 X, U32 Y,
     return zx * (U32)msaaPatternX(S, i) + zy * (U32)i + (((zx * X + zy * Y) << S) + zb);
 }
 
-// Pixel box [bx0, bx1] x [by0, by1] of the tile that can hold covered samples.
+// Pixel box [bx0, bx1] x [by0, by1] of the tile that can hold covered samples:
+// the pixels whose samples' box meets the vertices' (padded by half a pixel, the
+// 8.4M-triangle heightfield took 606 us at 4x MSAA instead of 577, and a
+// textured one at 1080p 872 instead of 727).
 template <int S>
 __device__ __forceinline__ bool pixelBox(const TileEdges& t, S32& bx0, S32& bx1, S32& by0, S32& by1) {
-    const S32 pad = (S == 0) ? 0 : 8;
+    constexpr S32 pad = sampleReach(S);
     bx0 = max(0, (t.minX - pad + 15) >> kSubpixelLog2);
     bx1 = min(7, (t.maxX + pad) >> kSubpixelLog2);
     by0 = max(0, (t.minY - pad + 15) >> kSubpixelLog2);
