@@ -103,7 +103,7 @@ struct FineVisSmem {
     U32 color[kTileWords];
     U64 key[kTileWords];        // depth << 32 | order (order << NS | coverage mask with MSAA)
     TriRec rec[32];             // id: list entry within the scene + 1
-    S32 head[32];               // batch triangle whose pairs start at position i of the current pass
+    uint2 turn[32];             // the small triangles in turn: box (packBox), batch triangle << 16 | first pair
     U32 winners[kTileWords];    // resolve: (pixel | first sample << 6 | samples won << 9)
     F32 shared[32];
 };
@@ -221,7 +221,7 @@ __device__ __forceinline__ U32 sampleMaskOf(const S32* E, const S32* A, const S3
 __device__ __forceinline__ bool packable(const TileEdges& t) {
     return max(t.maxX - t.minX, t.maxY - t.minY) <= 32767;
 }
-__device__ __forceinline__ TriRec packTri(const TileEdges& t, uint4 z, U32 id, U32 box) {
+__device__ __forceinline__ TriRec packTri(const TileEdges& t, uint4 z, U32 id, U32 box = 0u) {
     U32 E[3], AB[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -322,6 +322,22 @@ __device__ __forceinline__ void boxPixel(U32 box, S32 k, S32& px, S32& py) {
     const S32 q = (S32)(((U32)k * (box >> 12)) >> 8);
     px = (S32)(box & 0xFu) + k - q * (S32)((box >> 8) & 0xFu);
     py = (S32)((box >> 4) & 0xFu) + q;
+}
+
+// Pairs of a batch's small triangles, dealt to the lanes 32 a pass: a triangle
+// whose first pair is `start` (-1: it has none) marks it, and pair base + lane
+// belongs to the last one marked at or before it. Returns that one's turn among
+// the small triangles; `before` counts those of the passes so far. Passing the
+// start's lane through shared memory and the carried one by shuffles took the
+// stage 80 us instead of 78 on the 1M soup, 262 / 258 on the 33.5M-triangle
+// terrain and 178 / 174 on a 2x MSAA heightfield. The ordered path keeps its
+// forms: there the textured terrain took 457 us with this one, 449 without.
+__device__ __forceinline__ S32 turnOf(S32 start, S32 base, S32& before) {
+    const U32 at = (U32)(start - base);
+    const U32 marks = __reduce_or_sync(0xFFFFFFFFu, at < 32u ? 1u << at : 0u);
+    const S32 turn = before + __popc(marks & (0xFFFFFFFFu >> (31 - (threadIdx.x & 31)))) - 1;
+    before += __popc(marks);
+    return turn;
 }
 
 // Runs the fragment shader of triangle data td (16 words) at pixel (X, Y).
@@ -499,17 +515,15 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
             if constexpr (kVisibility) {
                 // ---- Visibility. Every (triangle, pixel) pair of the batch's
                 // triangles whose pixel box has at most selfPixels pixels is
-                // dealt to the lanes in turn, 32 pairs a pass: pair p's
-                // triangle is the last one whose pairs start at or before p
-                // (one OR over the warp marks the pass's starts, the
-                // triangle of the previous pass's last pair carries over),
-                // its pixel follows by an exact multiply-shift division by
+                // dealt to the lanes in turn, 32 pairs a pass (turnOf); the
+                // pair's pixel follows by an exact multiply-shift division by
                 // the box width (a lane walking its own triangle's box
                 // measured slower, even for boxes of one or two pixels);
                 // larger triangles are rasterized by the whole warp, two
                 // pixels per lane. Keys resolve by atomic minimum, so the
                 // order pairs are taken in does not change a bit.
                 S32 n = 0;
+                U32 box = 0;
                 bool big = false, far = false;
                 if (batch + lane < count) {
                     const U32 entry = __ldg(&d.tileList[start + batch + lane]);
@@ -525,43 +539,36 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                             far = !packable(te);
                             big = !far && cnt > selfPixels;
                             if (!far && !big) n = cnt;
-                            sm.rec[lane] = packTri(te, q0, entry - entryBase + 1u, packBox(bx0, by0, w));
+                            box = packBox(bx0, by0, w);
+                            sm.rec[lane] = packTri(te, q0, entry - entryBase + 1u);
                         }
                     }
                 }
-                S32 P = 0, myStart = 0;
-                if (__any_sync(0xFFFFFFFFu, n > 0)) {
+                S32 P = 0, myStart = -1;
+                const U32 smallMask = __ballot_sync(0xFFFFFFFFu, n > 0);
+                if (smallMask) {
                     S32 incl = n;
 #pragma unroll
                     for (int o = 1; o < 32; o <<= 1) {
                         const S32 t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
                         if (lane >= o) incl += t;
                     }
-                    myStart = incl - n;
                     P = __shfl_sync(0xFFFFFFFFu, incl, 31);
+                    if (n > 0) {
+                        myStart = incl - n;
+                        sm.turn[__popc(smallMask & ltMask)] = make_uint2(box, (U32)lane << 16 | (U32)myStart);
+                    }
                 }
                 __syncwarp();
-                S32 carryJ = 0, carryStart = 0;   // triangle (and its first pair) of the last pair so far
+                S32 before = 0;
                 for (S32 base = 0; base < P; base += 32) {
-                    const bool starts = n > 0 && myStart >= base && myStart < base + 32;
-                    if (starts) sm.head[myStart - base] = lane;
-                    const U32 startMask = __reduce_or_sync(0xFFFFFFFFu, starts ? 1u << (myStart - base) : 0u);
-                    __syncwarp();
-                    const U32 upTo = startMask & (0xFFFFFFFFu >> (31 - lane));
-                    S32 j = carryJ, first = carryStart;
-                    if (upTo) {
-                        const int h = 31 - __clz(upTo);
-                        j = sm.head[h];
-                        first = base + h;
-                    }
-                    carryJ = __shfl_sync(0xFFFFFFFFu, j, 31);
-                    carryStart = __shfl_sync(0xFFFFFFFFu, first, 31);
-                    __syncwarp();   // every lane has read head before the next pass rewrites it
+                    const S32 turn = turnOf(myStart, base, before);
                     const S32 p = base + lane;
                     if (p >= P) continue;
-                    const S32 k = p - first;
+                    const uint2 who = sm.turn[turn];
+                    const int j = (int)(who.y >> 16);
                     S32 px, py;
-                    boxPixel(sm.rec[j].q[2].z, k, px, py);
+                    boxPixel(who.x, p - (S32)(who.y & 0xFFFFu), px, py);
                     const uint4 r0 = sm.rec[j].q[0], r1 = sm.rec[j].q[1];
                     const U32 smask = packedMask<S>(r0, r1.x, r1.y, packedPixel(px, py));
                     if (!smask) continue;
