@@ -93,7 +93,7 @@ constexpr size_t kStaticScratchBytes = alignUp(kOffItemBlockCount + 4 * kStaticM
 
 }  // namespace
 
-// The scratch array (about 25 MiB, held by every GPU that loads the library).
+// The scratch array (about 22 MiB, held by every GPU that loads the library).
 static __device__ __align__(256) unsigned char g_staticScratch[kStaticScratchBytes];
 
 namespace {
