@@ -288,6 +288,7 @@ __device__ __forceinline__ void flushMedium(const DrawDev& d, const U32* medium,
 // are written after the next one's counters have been issued.
 __global__ void __launch_bounds__(kListThreads) pairKernel(const __grid_constant__ DrawDev d) {
     pdlWait();
+    markStage(d.stageTiming, d.counters, 1);
     __shared__ PairSmem s_pair[kListWarps];
     __shared__ S32 s_bins[kSharedBins];
     if (__ldcg(&d.counters->overflow) & kOverflowSubtris) return;
@@ -592,6 +593,7 @@ constexpr int kScanTiles = kListThreads * 4;
 
 __global__ void __launch_bounds__(kListThreads) listScanKernel(const __grid_constant__ DrawDev d) {
     pdlWait();
+    markStage(d.stageTiming, d.counters, 2);
     __shared__ S32 s_warp[kListWarps];
     __shared__ S32 s_base;
     const bool failed = (__ldcg(&d.counters->overflow) & kOverflowSubtris) != 0;
@@ -950,9 +952,8 @@ __global__ void __launch_bounds__(kListThreads) listSortKernel(const __grid_cons
 
 // ------------------------------------------------------------ launchers
 
-// The list stages after setup; evCoarse (may be null) is recorded between the
-// bin (pairs, items) and coarse (list) stages.
-cudaError_t launchBinning(const DrawDev& d, int numSMs, cudaStream_t stream, cudaEvent_t evCoarse) {
+// The list stages after setup: bin (pairs, items) and coarse (scan, scatter).
+cudaError_t launchBinning(const DrawDev& d, int numSMs, cudaStream_t stream) {
     static IntsPerDevice<2> ctas;   // resident CTAs per SM of the pair and scatter kernels
     const int pairCtas = ctas.get(0, [](int) {
         int n = 0;
@@ -970,7 +971,6 @@ cudaError_t launchBinning(const DrawDev& d, int numSMs, cudaStream_t stream, cud
         e = launchKernel(pairKernel, pairGrid, kListThreads, 0, stream, true, d);
         if (e == cudaSuccess) e = launchKernel(itemKernel, numSMs * (kItemWarpsPerSM / kListWarps), kListThreads, 0, stream, true, d);
     }
-    if (e == cudaSuccess && evCoarse) e = cudaEventRecord(evCoarse, stream);
     // The scan also runs for a draw without triangles: it zeroes the counts.
     if (e == cudaSuccess)
         e = launchKernel(listScanKernel, (d.totalTiles + kScanTiles - 1) / kScanTiles, kListThreads, 0, stream, true, d);

@@ -25,7 +25,7 @@
 #include <vector>
 
 namespace cr {
-cudaError_t launchBinning(const DrawDev& d, int numSMs, cudaStream_t stream, cudaEvent_t evCoarse);
+cudaError_t launchBinning(const DrawDev& d, int numSMs, cudaStream_t stream);
 cudaError_t launchListSort(const DrawDev& d, int32_t tileBegin, int32_t tileEnd, int numSMs, cudaStream_t stream);
 }
 
@@ -143,9 +143,9 @@ struct cr_context {
     bool stageUsed[kStageSlots] = {};
     int stageNext = 0;
     Counters* hostCounters = nullptr;
-    cudaEvent_t ev[5] = {};
-    bool stageTiming = true;      // record the per-stage events of getStats
-    bool eventsRecorded = false;  // the last draw recorded them
+    cudaEvent_t ev[2] = {};       // before setup and after fine
+    bool stageTiming = true;      // time the stages for getStats
+    bool eventsRecorded = false;  // the last draw did
     bool drawn = false;           // a draw was enqueued (its counters are copied to hostCounters)
     int numSMs = 0;
     int device = 0;
@@ -258,7 +258,7 @@ cr_status cr_create(cr_context** out) {
         return CR_ERR_UNSUPPORTED;
     }
     ctx->numSMs = prop.multiProcessorCount;
-    for (int i = 0; i < 5; i++) {
+    for (int i = 0; i < 2; i++) {
         if (cudaEventCreate(&ctx->ev[i]) != cudaSuccess) { delete ctx; return CR_ERR_CUDA; }
     }
     if (cudaMallocHost(&ctx->hostCounters, sizeof(Counters)) != cudaSuccess) { delete ctx; return CR_ERR_CUDA; }
@@ -279,7 +279,7 @@ cr_status cr_destroy(cr_context* ctx) {
         if (ctx->stageDone[i]) cudaEventDestroy(ctx->stageDone[i]);
     }
     if (ctx->hostCounters) cudaFreeHost(ctx->hostCounters);
-    for (int i = 0; i < 5; i++)
+    for (int i = 0; i < 2; i++)
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
     delete ctx;
     return CR_OK;
@@ -700,6 +700,7 @@ DrawDev makeDrawDev(cr_context* ctx, const Plan& plan) {
     d.totalBins = plan.totalBins;
     d.totalTiles = plan.totalTiles;
     d.totalTris = plan.totalTris;
+    d.stageTiming = 0;
     d.model = plan.model;
     d.modelStride = plan.modelStride;
     d.modelVec4 = plan.model && plan.modelStride == 4 && ((uintptr_t)plan.model & 15) == 0;
@@ -778,11 +779,12 @@ bool capturing(cudaStream_t s) {
 // the descriptors (the copy node reads it when a captured graph replays;
 // with `writeKernel` a blocking draw's block goes as a kernel parameter) and
 // `hostCounters` (pinned) receives the device counters, written by the first
-// fine launch or copied after the draw; with `events` false no stage
-// events are recorded (graph capture).
+// fine launch or copied after the draw; with `events` false the
+// stages are not timed (graph capture).
 cr_status launchDrawWith(cr_context* ctx, const Plan& plan, cudaStream_t stream, void* stage, Counters* hostCounters,
                          bool events, bool writeKernel) {
     DrawDev d = makeDrawDev(ctx, plan);
+    d.stageTiming = events ? 1 : 0;
     // Stage the zeroed counters and the descriptors through pinned memory;
     // for a blocking draw a kernel parameter carries them to the device, else
     // (and for blocks above 8 KB) a copy; in a graph capture the copy node
@@ -809,12 +811,10 @@ cr_status launchDrawWith(cr_context* ctx, const Plan& plan, cudaStream_t stream,
     if (events) CR_CUDA(cudaEventRecord(ctx->ev[0], stream), "cudaEventRecord");
     for (const Plan::Group& g : plan.groups)
         CR_CUDA(g.pipe->launchSetup(d, g.instBegin, g.instEnd, g.triBegin, g.triEnd, stream), "setup launch");
-    if (events) CR_CUDA(cudaEventRecord(ctx->ev[1], stream), "cudaEventRecord");
-    CR_CUDA(launchBinning(d, ctx->numSMs, stream, events ? ctx->ev[2] : nullptr), "bin/coarse launch");
+    CR_CUDA(launchBinning(d, ctx->numSMs, stream), "bin/coarse launch");
     for (const Plan::Group& g : plan.groups)
         if (g.pipe->needsOrder)
             CR_CUDA(launchListSort(d, g.tileBegin, g.tileEnd, ctx->numSMs, stream), "list sort launch");
-    if (events) CR_CUDA(cudaEventRecord(ctx->ev[3], stream), "cudaEventRecord");
     // The first fine launch that has tiles writes the counters into the
     // pinned host buffer (its device address); without one, a copy follows.
     Counters* devHostCounters = nullptr;
@@ -834,7 +834,7 @@ cr_status launchDrawWith(cr_context* ctx, const Plan& plan, cudaStream_t stream,
         }
         CR_CUDA(g.pipe->launchFine(dg, (int)gi, g.tileBegin, g.tileEnd, warps, ctas, ctx->numSMs, stream), "fine launch");
     }
-    if (events) CR_CUDA(cudaEventRecord(ctx->ev[4], stream), "cudaEventRecord");
+    if (events) CR_CUDA(cudaEventRecord(ctx->ev[1], stream), "cudaEventRecord");
     ctx->eventsRecorded = events;
     if (!written)
         CR_CUDA(cudaMemcpyAsync(hostCounters, ctx->drawBlock.ptr, sizeof(Counters), cudaMemcpyDeviceToHost, stream),
@@ -1103,13 +1103,19 @@ cr_status cr_get_stats(cr_context* ctx, cr_stats* out) {
     if (!ctx || !out) return CR_ERR_INVALID_ARGUMENT;
     memset(out, 0, sizeof(*out));
     if (!ctx->eventsRecorded) return CR_OK;
-    CR_CUDA(cudaEventSynchronize(ctx->ev[4]), "cudaEventSynchronize");
-    float t[4] = {0, 0, 0, 0};
-    for (int i = 0; i < 4; i++) cudaEventElapsedTime(&t[i], ctx->ev[i], ctx->ev[i + 1]);
-    out->setup_time = t[0] * 1e-3f;
-    out->bin_time = t[1] * 1e-3f;
-    out->coarse_time = t[2] * 1e-3f;
-    out->fine_time = t[3] * 1e-3f;
+    CR_CUDA(cudaEventSynchronize(ctx->ev[1]), "cudaEventSynchronize");
+    float ms = 0.0f;
+    cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
+    // A stage without a launch (a draw without triangles) begins with the next.
+    uint64_t begin[4];
+    for (int i = 3; i >= 0; i--) {
+        begin[i] = ctx->hostCounters->stageBegin[i];
+        if (i < 3 && (begin[i] == 0 || begin[i] > begin[i + 1])) begin[i] = begin[i + 1];
+    }
+    out->setup_time = (float)(begin[1] - begin[0]) * 1e-9f;
+    out->bin_time = (float)(begin[2] - begin[1]) * 1e-9f;
+    out->coarse_time = (float)(begin[3] - begin[2]) * 1e-9f;
+    out->fine_time = std::max(ms * 1e-3f - (float)(begin[3] - begin[0]) * 1e-9f, 0.0f);
     return CR_OK;
 }
 

@@ -38,7 +38,7 @@
 #include <mutex>
 
 namespace cr {
-cudaError_t launchBinning(const DrawDev& d, int numSMs, cudaStream_t stream, cudaEvent_t evCoarse);
+cudaError_t launchBinning(const DrawDev& d, int numSMs, cudaStream_t stream);
 cudaError_t launchListSort(const DrawDev& d, int32_t tileBegin, int32_t tileEnd, int numSMs, cudaStream_t stream);
 }
 namespace cr {
@@ -258,7 +258,7 @@ extern "C" cr_status cr_draw_triangles_static(const char* pipe_name, void* color
     CR_STATIC_CUDA(cudaMemsetAsync(scratch + kOffCounters, 0, kOffInst - kOffCounters, s));
 
     CR_STATIC_CUDA(pipe->launchSetup(d, 0, 1, 0, num_tris, s));
-    CR_STATIC_CUDA(launchBinning(d, std::min(numSMs, kStaticSMs), s, nullptr));
+    CR_STATIC_CUDA(launchBinning(d, std::min(numSMs, kStaticSMs), s));
     if (pipe->needsOrder) CR_STATIC_CUDA(launchListSort(d, 0, numTiles, numSMs, s));
     const int warps = 8;
     CR_STATIC_CUDA(pipe->launchFine(d, 0, 0, numTiles, warps, pipe->fineOccupancy(warps), numSMs, s));

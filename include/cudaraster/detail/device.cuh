@@ -85,6 +85,7 @@ struct Counters {
     S32 chunkWork;            // pair-stage chunk counter (dynamic chunk assignment)
     S32 itemWarps;            // warps of the item kernel: blocks of item pair records that are theirs from the start
     S32 itemBlocks;           // blocks taken beyond those
+    U64 stageBegin[4];        // when setup, pairs, scan and fine began, in ns (draws with stage timing)
 };
 // Item pair records come in blocks of this many, each filled by one warp.
 constexpr int kItemBlock = 256;
@@ -174,6 +175,7 @@ struct DrawDev {
     // finished by then), in place of a device-to-host copy after the draw.
     // Null in every other launch.
     Counters* hostCounters;
+    S32 stageTiming;          // stages note when they begin
 };
 
 // ------------------------------------------------------ instance lookup
@@ -370,5 +372,20 @@ __device__ __forceinline__ U32 centroidCode(int s, U32 mask) {
 
 __host__ __device__ __forceinline__ S32 lo16(U32 v) { return (S32)(int16_t)(uint16_t)(v & 0xFFFF); }
 __host__ __device__ __forceinline__ S32 hi16(U32 v) { return (S32)(int16_t)(uint16_t)(v >> 16); }
+
+__device__ __forceinline__ U64 globalNanoseconds() {
+    U64 t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+// Notes when a stage begins; called after pdlWait(), so the stage before it
+// has ended. An event between two stages instead takes about 4 us of a small
+// draw and keeps the launches from overlapping (cube draw 80 us with an event
+// at every stage, 67 so; 5,000 blended triangles 93 / 81). The fine stage notes
+// its own with the counters it hands over.
+__device__ __forceinline__ void markStage(S32 timing, Counters* counters, int stage) {
+    if (timing && blockIdx.x == 0 && threadIdx.x == 0) counters->stageBegin[stage] = globalNanoseconds();
+}
+static_assert(sizeof(Counters) % 8 == 0 && sizeof(Counters) <= 128, "handed over by one warp, the last begin in its last two words");
 
 }  // namespace cr

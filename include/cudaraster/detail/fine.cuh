@@ -397,9 +397,15 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
     const U32 ltMask = (1u << lane) - 1u;
     pdlWait();
     pdlTrigger();
-    if (d.hostCounters != nullptr && blockIdx.x == 0 && threadIdx.x < (int)(sizeof(Counters) / 4))
-        reinterpret_cast<volatile U32*>(d.hostCounters)[threadIdx.x] =
-            reinterpret_cast<const volatile U32*>(d.counters)[threadIdx.x];
+    if (d.hostCounters != nullptr && blockIdx.x == 0 && threadIdx.x < (int)(sizeof(Counters) / 4)) {
+        U32 word = reinterpret_cast<const volatile U32*>(d.counters)[threadIdx.x];
+        // The last two words: when this stage began (see markStage).
+        if (d.stageTiming && threadIdx.x >= (int)(sizeof(Counters) / 4) - 2) {
+            const U64 t = globalNanoseconds();
+            word = threadIdx.x & 1 ? (U32)(t >> 32) : (U32)t;
+        }
+        reinterpret_cast<volatile U32*>(d.hostCounters)[threadIdx.x] = word;
+    }
     if (__ldg(&d.counters->overflow)) return;
     const S32 selfPixels = d.fineSelfPixels > 0 ? d.fineSelfPixels : fineSelfPixelsDefault(S, kVisibility);
 

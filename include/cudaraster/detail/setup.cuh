@@ -288,6 +288,7 @@ template <int S, U32 F>
 __global__ void __launch_bounds__(kSetupThreads, CR_SETUP_MIN_BLOCKS) setupKernel(DrawDev d, int instBegin, int instEnd, S64 triBegin, S64 triEnd) {
     pdlWait();
     pdlTrigger();
+    if (instBegin == 0) markStage(d.stageTiming, d.counters, 0);
     const S64 gt = triBegin + (S64)blockIdx.x * kSetupThreads + threadIdx.x;
     if (gt >= triEnd) return;
     const int ii = instBegin + findInstance64(d.triPrefix + instBegin, instEnd - instBegin, gt);
