@@ -35,8 +35,9 @@ struct PipeImpl {
         int64_t n = triEnd - triBegin;
         if (n <= 0) return cudaSuccess;
         unsigned grid = (unsigned)((n + kSetupThreads - 1) / kSetupThreads);
-        return launchKernel(setupKernel<S, F & (kRenderDepth | kRenderLerp)>, grid, kSetupThreads, 0, stream, true, d, instBegin,
-                            instEnd, (S64)triBegin, (S64)triEnd);
+        constexpr U32 kFlags = F & (kRenderDepth | kRenderLerp);
+        return launchKernel(d.stageTiming ? &setupKernel<S, kFlags, true> : &setupKernel<S, kFlags, false>, grid,
+                            kSetupThreads, 0, stream, true, d, instBegin, instEnd, (S64)triBegin, (S64)triEnd);
     }
     static size_t smemBytes(int warps) { return sizeof(typename FineTraits<FS, BS, S, F>::Smem) * (size_t)warps; }
     static cudaError_t launchFine(const DrawDev& d, int group, int32_t tileBegin, int32_t tileEnd, int warps,

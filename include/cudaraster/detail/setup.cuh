@@ -284,13 +284,15 @@ __device__ __forceinline__ bool cutByPlane(float4 v) {
 
 // triangleSetupImpl (TriangleSetup.inl:219-417), over the triangle range of
 // one pipe group [triBegin, triEnd) (global triangle slots).
-template <int S, U32 F>
+// kTimed: for draws with stage timing; in a test of the flag at run time the
+// 33.5M-triangle terrain's setup took 555 us instead of 550.
+template <int S, U32 F, bool kTimed>
 __global__ void __launch_bounds__(kSetupThreads, CR_SETUP_MIN_BLOCKS) setupKernel(DrawDev d, int instBegin, int instEnd, S64 triBegin, S64 triEnd) {
     pdlWait();
     pdlTrigger();
-    if (instBegin == 0) markStage(d.stageTiming, d.counters, 0);
     const S64 gt = triBegin + (S64)blockIdx.x * kSetupThreads + threadIdx.x;
     if (gt >= triEnd) return;
+    if (kTimed && gt == 0) markStage(1, d.counters, 0);
     const int ii = instBegin + findInstance64(d.triPrefix + instBegin, instEnd - instBegin, gt);
     const InstanceDev* in = &d.inst[ii];
     const S32 width = __ldg(&in->width), height = __ldg(&in->height);

@@ -42,3 +42,19 @@ def test_stage_times_add_up(cuda, pipe, tris):
     cr.drawTriangles()
     s = cr.getStats()
     assert [s.setupTime, s.binTime, s.coarseTime, s.fineTime] == [0.0] * 4
+
+
+def test_batch_whose_first_pipe_has_no_triangles(cuda):
+    """The first setup launch is the second pipe's: its time still counts as setup."""
+    p = pkg()
+    sc = pkg_mod("scenes").soup(200000, 640, 480, seed=4)
+    v, i = torch.from_numpy(np.ascontiguousarray(sc["vertices"][:, :8])).cuda(), torch.from_numpy(sc["indices"]).cuda()
+    insts = [{"pipe": pipe, "color": p.CudaSurface((640, 480), p.CudaSurface.FORMAT_RGBA8),
+              "depth": p.CudaSurface((640, 480), p.CudaSurface.FORMAT_DEPTH32), "vertices": v, "indices": i,
+              "numTris": n, "clear": (0.1, 0.2, 0.3, 1.0, 1.0)}
+             for pipe, n in (("PixelPipe_gouraud", 0), ("PixelPipe_gouraud_srcover", 200000))]
+    cr = p.CudaRaster()
+    cr.init()
+    cr.drawBatch(insts)
+    s = cr.getStats()
+    assert min(s.setupTime, s.binTime, s.coarseTime, s.fineTime) > 0.0
