@@ -443,7 +443,7 @@ def main():
     h2d = hv.numel() * 4 + hi.numel() * 4
     d2h = (hc[0].numel() + hd[0].numel()) * 4
 
-    # ---- roofline of the dominant stage (stage events bracket its kernels)
+    # ---- roofline of the dominant stage (stage timing brackets its kernels)
     peak, peak_kind = peaks()
     names = ["setup", "bin", "coarse", "fine"]
     dom = int(np.argmax(stage_ms))

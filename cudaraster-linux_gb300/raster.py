@@ -247,7 +247,7 @@ class CudaRaster:
         self._check(self._lib.cr_set_tuning(self._ctx, C.byref(t)))
 
     def setStageTiming(self, enabled: bool) -> None:
-        """Per-stage events for getStats (on by default); off lets the stages' launches overlap."""
+        """Stage times for getStats (on by default): two events a draw and the times the stages begin."""
         self._need_init()
         self._check(self._lib.cr_set_stage_timing(self._ctx, 1 if enabled else 0))
 

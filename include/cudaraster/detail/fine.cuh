@@ -9,14 +9,14 @@
 //
 // What bounds it: the shared-memory and L1 data pipe (70% of its wavefronts on
 // 1M small triangles, 72% on the 8.4M-triangle 4x MSAA heightfield) and
-// instruction issue (72%, 68%), at 30 to 38 resident warps. So triangles are
+// instruction issue (72%, 68%), at 30 to 38 resident warps (before). So triangles are
 // kept in packed records read by 128-bit loads (two 16-bit edge steps to a
 // word, an edge value in one dp2a), tiles move 8 bytes a lane, and tiles that
 // no triangle touches are written without passing through shared memory. These
-// took the stage from 84 to 80 us on the 1M soup, 107 to 96 on 20,000
-// triangles of 60 pixels, 627 to 577 on the heightfield (with pixelBox's tight
-// boxes), 613 to 455 on 300k triangles at 8x MSAA, 160 to 152 on 300k blended
-// ones, 471 to 453 on the textured terrain.
+// took the stage from 84 to 78 us on the 1M soup (with turnOf), 107 to 96 on
+// 20,000 triangles of 60 pixels, 627 to 573 on the heightfield (with pixelBox's
+// tight boxes), 613 to 455 on 300k triangles at 8x MSAA, 160 to 152 on 300k
+// blended ones, 471 to 449 on the textured terrain (with loadSlot32).
 //
 // Both paths deal the (triangle, pixel) pairs of the batch's small triangles
 // (pixel box of at most fineSelfPixels pixels) over the lanes; larger
