@@ -710,12 +710,23 @@ __global__ void __launch_bounds__(kListThreads) listScatterKernel(const __grid_c
         }
     }
     const S32 blocks = min(__ldcg(&d.counters->itemWarps) + __ldcg(&d.counters->itemBlocks), d.maxItemBlocks);
-    constexpr int kParts = kItemBlock / 32;
+    // The items' pairs, four per lane in flight too (one per lane: the stage 23.5 us
+    // instead of 22.1 on 20,000 triangles of 60 pixels, 49 / 46 on the water layer).
+    constexpr int kParts = kItemBlock / 128;
     for (S64 u = warpIdx; u < (S64)blocks * kParts; u += warps) {
-        const S32 block = (S32)(u / kParts), at = (S32)(u % kParts) * 32 + lane;
-        if (at >= __ldcg(&d.itemBlockCount[block])) continue;
-        const U64 rec = __ldcg(&d.itemPairs[(S64)block * kItemBlock + at]);
-        putEntry(d, atomicAdd(&d.tileCursor[(U32)rec], 1), (U32)(rec >> 32));
+        const S32 block = (S32)(u / kParts), at = (S32)(u % kParts) * 128 + lane;
+        const S32 count = __ldcg(&d.itemBlockCount[block]);
+        const U64* pairs = d.itemPairs + (S64)block * kItemBlock;
+        U64 rec[4];
+        S32 place[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) rec[k] = at + k * 32 < count ? __ldcg(&pairs[at + k * 32]) : 0ull;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (at + k * 32 < count) place[k] = atomicAdd(&d.tileCursor[(U32)rec[k]], 1);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (at + k * 32 < count) putEntry(d, place[k], (U32)(rec[k] >> 32));
     }
 }
 
