@@ -35,6 +35,7 @@
 // must hold the entry too.
 #include "cudaraster/detail/binning.cuh"
 #include "cudaraster/detail/launch.h"
+#include "cudaraster/detail/list_alloc.h"
 #include "cudaraster/detail/per_device.h"
 
 #include <algorithm>
@@ -45,11 +46,12 @@ constexpr int kListThreads = 256;
 constexpr int kListWarps = kListThreads / 32;
 
 // Warp-level inclusive scan.
-__device__ __forceinline__ S32 warpInclusiveScan(S32 v) {
+template <class T>
+__device__ __forceinline__ T warpInclusiveScan(T v) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        S32 t = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        T t = __shfl_up_sync(0xFFFFFFFFu, v, o);
         if (lane >= o) v += t;
     }
     return v;
@@ -510,7 +512,8 @@ __device__ __forceinline__ S32 stageItems(const DrawDev& d, S32 items, U32 entry
 // A warp's current block of item pair records: its own first, then from a
 // counter. A warp leaves at most one block partly filled, so a draw whose tile
 // entries fit has blocks for all; past the last one nothing is written (the
-// scan reports the overflow).
+// scan reports the overflow; the block numbers are compared unsigned, so a
+// counter past 2^31 writes nothing either).
 struct ItemBlock {
     S32 block, fill;
 };
@@ -529,7 +532,7 @@ __device__ __forceinline__ void recordItemPairs(const DrawDev& d, ItemBlock& blk
         S32 fresh = 0;
         if (lane == 0) {
             fresh = gridDim.x * kListWarps + atomicAdd(&d.counters->itemBlocks, 1);
-            if (block < d.maxItemBlocks) d.itemBlockCount[block] = kItemBlock;
+            if ((U32)block < (U32)d.maxItemBlocks) d.itemBlockCount[block] = kItemBlock;
         }
         fresh = __shfl_sync(0xFFFFFFFFu, fresh, 0);
         if (at >= kItemBlock) {
@@ -539,7 +542,7 @@ __device__ __forceinline__ void recordItemPairs(const DrawDev& d, ItemBlock& blk
         blk.fill -= kItemBlock;
         blk.block = fresh;
     }
-    if (hit && block < d.maxItemBlocks) d.itemPairs[(S64)block * kItemBlock + at] = (U64)entry << 32 | (U32)tile;
+    if (hit && (U32)block < (U32)d.maxItemBlocks) d.itemPairs[(S64)block * kItemBlock + at] = (U64)entry << 32 | (U32)tile;
 }
 
 // Records the pairs of the items and counts their tiles and bins. Persistent
@@ -580,26 +583,28 @@ __global__ void __launch_bounds__(kListThreads, kItemWarpsPerSM / kListWarps) it
         }
         __syncwarp();
     }
-    if (lane == 0 && blk.block < d.maxItemBlocks) d.itemBlockCount[blk.block] = blk.fill;
+    if (lane == 0 && (U32)blk.block < (U32)d.maxItemBlocks) d.itemBlockCount[blk.block] = blk.fill;
     if (blockIdx.x == 0 && threadIdx.x == 0) d.counters->itemWarps = warps;
 }
 
 // ------------------------------------------------------------------ scan
 
 // Four consecutive tiles per thread; a CTA's lists are one contiguous piece of
-// the list memory, allocated with one atomic. The first CTA also hands over
-// the bin counts. The work arrays end zeroed, for the next draw.
+// the list memory, allocated with one atomic on a 64-bit total (list_alloc.h):
+// a CTA whose lists do not fit flags the overflow, and no later stage reads a
+// start. The first CTA also hands over the bin counts. The work arrays end
+// zeroed, for the next draw.
 constexpr int kScanTiles = kListThreads * 4;
 
 __global__ void __launch_bounds__(kListThreads) listScanKernel(const __grid_constant__ DrawDev d) {
     pdlWait();
     markStage(d.stageTiming, d.counters, 2);
-    __shared__ S32 s_warp[kListWarps];
-    __shared__ S32 s_base;
+    __shared__ U64 s_warp[kListWarps];
+    __shared__ U64 s_base;
     const bool failed = (__ldcg(&d.counters->overflow) & kOverflowSubtris) != 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const S32 t0 = blockIdx.x * kScanTiles + threadIdx.x * 4;
-    S32 c[4], own[4];   // entries, and those recorded by setup
+    S32 c[4], own[4];   // entries, and those the pair stage recorded
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         c[k] = own[k] = 0;
@@ -623,22 +628,23 @@ __global__ void __launch_bounds__(kListThreads) listScanKernel(const __grid_cons
 #pragma unroll
     for (int k = 0; k < 4; k++)
         if (t0 + k < d.totalTiles) d.tileWork[(t0 + k) << d.tileWorkLog2] = 0;
-    const S32 sum = c[0] + c[1] + c[2] + c[3];
-    const S32 incl = warpInclusiveScan(sum);
+    const U64 sum = entriesOf4(c);
+    const U64 incl = warpInclusiveScan(sum);
     if (lane == 31) s_warp[warp] = incl;
     __syncthreads();
     if (warp == 0) {
-        const S32 v = lane < kListWarps ? s_warp[lane] : 0;
-        const S32 i = warpInclusiveScan(v);
+        const U64 v = lane < kListWarps ? s_warp[lane] : 0ull;
+        const U64 i = warpInclusiveScan(v);
         if (lane < kListWarps) s_warp[lane] = i - v;
         if (lane == kListWarps - 1 && !failed) {
-            const S32 base = atomicAdd(&d.counters->tileEntries, i);
-            if ((S64)base + i > d.maxTileEntries) atomicOr(&d.counters->overflow, kOverflowTile);
+            const U64 base = atomicAdd((unsigned long long*)&d.counters->tileTotal, (unsigned long long)i);
+            atomicMax(&d.counters->tileEntries, reportedEntries(base + i));
+            if (!listsFit(base + i, d.maxTileEntries)) atomicOr(&d.counters->overflow, kOverflowTile);
             s_base = base;
         }
     }
     __syncthreads();
-    S32 s = s_base + s_warp[warp] + incl - sum;
+    S32 s = (S32)(s_base + s_warp[warp] + incl - sum);
     if (!failed) {
         if (t0 + 3 < d.totalTiles) {
             const int4 v = make_int4(s, s + c[0], s + c[0] + c[1], s + c[0] + c[1] + c[2]);
@@ -656,22 +662,22 @@ __global__ void __launch_bounds__(kListThreads) listScanKernel(const __grid_cons
         }
     }
     if (blockIdx.x == 0) {
-        S32 mine = 0;
+        U64 mine = 0;
         for (S32 b = threadIdx.x; b < d.totalBins; b += kListThreads) {
             const S32 v = __ldcg(&d.binWork[b * kBinWorkStride]);
             d.binWork[b * kBinWorkStride] = 0;
             d.binCount[b] = v;
-            mine += v;
+            mine += (U32)v;
         }
-        mine = __reduce_add_sync(0xFFFFFFFFu, mine);
+        mine = warpInclusiveScan(mine);
         __syncthreads();
-        if (lane == 0) s_warp[warp] = mine;
+        if (lane == 31) s_warp[warp] = mine;
         __syncthreads();
         if (threadIdx.x == 0 && !failed) {
-            S64 total = 0;
+            U64 total = 0;
             for (int w = 0; w < kListWarps; w++) total += s_warp[w];
-            d.counters->binEntries = (S32)total;
-            if (total > d.maxBinEntries) atomicOr(&d.counters->overflow, kOverflowBin);
+            d.counters->binEntries = reportedEntries(total);
+            if (!listsFit(total, d.maxBinEntries)) atomicOr(&d.counters->overflow, kOverflowBin);
         }
     }
 }
@@ -679,7 +685,7 @@ __global__ void __launch_bounds__(kListThreads) listScanKernel(const __grid_cons
 // --------------------------------------------------------------- scatter
 
 __device__ __forceinline__ void putEntry(const DrawDev& d, S32 idx, U32 entry) {
-    if ((S64)idx < d.maxTileEntries) d.tileList[idx] = entry;
+    if (listHolds(idx, d.maxTileEntries)) d.tileList[idx] = entry;
 }
 
 // Persistent warps: the pair records, then those of the items.

@@ -11,6 +11,7 @@
 #include "cudaraster/detail/binning.cuh"
 #include "cudaraster/detail/device.cuh"
 #include "cudaraster/detail/launch.h"
+#include "cudaraster/detail/list_alloc.h"
 #include "cudaraster/detail/pipe_registry.h"
 
 #include <algorithm>
@@ -895,6 +896,9 @@ cr_status drawPlan(cr_context* ctx, const Plan& plan, cudaStream_t stream, bool 
         const Counters& c = *ctx->hostCounters;
         if (!c.overflow) return CR_OK;
         if (reruns >= 16) return fail(ctx, CR_ERR_CAPACITY, "CudaRaster: queues keep overflowing");
+        if (((c.overflow & kOverflowBin) && c.binEntries >= kMaxListEntries) ||
+            ((c.overflow & kOverflowTile) && c.tileEntries >= kMaxListEntries))
+            return fail(ctx, CR_ERR_CAPACITY, "CudaRaster: the draw's queues hold over 2^31 - 1 entries");
         int64_t subtris = plan.totalTris + c.extraSubtris;
         if (c.overflow & kOverflowSubtris) ctx->maxSubtris = std::max(ctx->maxSubtris, subtris + 4096);
         if (c.overflow & kOverflowBin) ctx->maxBinEntries = std::max<int64_t>(ctx->maxBinEntries, (int64_t)c.binEntries + 65536);

@@ -75,7 +75,7 @@ struct InstanceDev {
 
 struct Counters {
     S32 extraSubtris;         // subtriangle slots allocated past the triangle slots
-    S32 binEntries;           // total bin list entries
+    S32 binEntries;           // total bin list entries (saturated at 2^31 - 1, as tileEntries)
     S32 numUnits;             // coarse work units (slices of the large items)
     S32 tileEntries;          // total tile list entries
     S32 fineTile;             // fine-stage work counter
@@ -85,6 +85,7 @@ struct Counters {
     S32 chunkWork;            // pair-stage chunk counter (dynamic chunk assignment)
     S32 itemWarps;            // warps of the item kernel: blocks of item pair records that are theirs from the start
     S32 itemBlocks;           // blocks taken beyond those
+    U64 tileTotal;            // tile list entries allocated
     U64 stageBegin[4];        // when setup, pairs, scan and fine began, in ns (draws with stage timing)
 };
 // Item pair records come in blocks of this many, each filled by one warp.
