@@ -4,8 +4,8 @@
 // counter, as FineRaster.inl:534-552). The tile's colour and depth live in the
 // warp's shared memory for the whole tile. Its triangle list is consumed in
 // batches of 32; lane i fetches entry i (header, data slot, early-Z against
-// the tile's current maximum depth as FineRaster.inl:229-240, edge functions
-// at the tile origin). Then one of two algorithms runs, chosen at compile time:
+// the tile's current maximum depth as FineRaster.inl:229-240 or mayWin, edge
+// functions at the tile origin). Then one of two algorithms runs, chosen at compile time:
 //
 // What bounds it: the shared-memory and L1 data pipe (70% of its wavefronts on
 // 1M small triangles, 72% on the 8.4M-triangle 4x MSAA heightfield) and
@@ -41,7 +41,8 @@
 //   submission order on equal depth -- the same result as applying every
 //   fragment in order with a LESS test. Each sample keeps a 64-bit key
 //   (depth << 32 | list entry + 1) that fragments lower with atomicMin, so the
-//   tile's list may come in any order (entries grow in submission order);
+//   tile's list may come in any order (entries grow in submission order; early
+//   Z drops no triangle that could win, see mayWin);
 //   after the list, the tile's winners are listed and each is shaded once,
 //   32 at a time.
 //
@@ -267,6 +268,27 @@ __device__ __forceinline__ bool edgesMayCover(const TileEdges& t, S32 px, S32 py
         any |= t.E[k] + t.A[k] * (px << kSubpixelLog2) + t.B[k] * (py << kSubpixelLog2) + slack;
     }
     return any >= 0;
+}
+
+// Early Z of the visibility path. Lists come in no particular order there, so a
+// triangle may be dropped only if none of its samples can win, not even a tie:
+// if its lowest sample lies beyond the tile's maximum depth. The header's
+// minimum is lerpError(S) = 2200 << S below the lowest vertex. Up to 2,048
+// pixels across that covers the slopes' flooring to whole units per sample (at
+// most half the box on each axis from its centre, where the plane is anchored:
+// 2048 << S in all); the other errors stay within kZMargin: vertex depths cut
+// to 24 bits (256 units) and rounded (128), the area's reciprocal (512), and in
+// the anchor the cut of the gradients by 13 bits times at most 2^14 subpixels
+// on each axis (8192 for the smallest area). Larger triangles are never
+// dropped: their samples can lie thousands of units below the header's minimum.
+constexpr U32 kZMargin = 1u << 14;
+__device__ __forceinline__ U32 withZMargin(U32 z) { return z + min(kZMargin, ~z); }
+// zLimit: the tile's maximum depth with the margin.
+__device__ __forceinline__ bool mayWin(uint4 h, U32 zLimit) {
+    if ((h.w & 0xFFFFF000u) <= zLimit) return true;
+    const S32 w = max3i(lo16(h.x), lo16(h.y), lo16(h.z)) - min3i(lo16(h.x), lo16(h.y), lo16(h.z));
+    const S32 ht = max3i(hi16(h.x), hi16(h.y), hi16(h.z)) - min3i(hi16(h.x), hi16(h.y), hi16(h.z));
+    return max(w, ht) > 32767;
 }
 
 // Slot of a list entry's subtriangle, and the edges of a triangle that a record
@@ -531,11 +553,12 @@ __device__ __forceinline__ void fineTiles(const DrawDev& d, int group, S32 tileB
                 S32 n = 0;
                 U32 box = 0;
                 bool big = false, far = false;
+                const U32 zLimit = withZMargin(tileZMax);
                 if (batch + lane < count) {
                     const U32 entry = __ldg(&d.tileList[start + batch + lane]);
                     const S64 slot = entrySlotOf(d, entry);
                     const uint4 h = __ldg(&d.triHeader[slot]);
-                    if ((h.w & 0xFFFFF000u) < tileZMax) {
+                    if (mayWin(h, zLimit)) {
                         const TileEdges te = tileEdges(h, cx0, cy0);
                         S32 bx0, bx1, by0, by1;
                         if (pixelBox<S>(te, bx0, bx1, by0, by1)) {
