@@ -595,6 +595,7 @@ __global__ void __launch_bounds__(kListThreads, kItemWarpsPerSM / kListWarps) it
 // start. The first CTA also hands over the bin counts. The work arrays end
 // zeroed, for the next draw.
 constexpr int kScanTiles = kListThreads * 4;
+constexpr int kSortRun = 256;   // lists up to this length are sorted in a warp's registers
 
 __global__ void __launch_bounds__(kListThreads) listScanKernel(const __grid_constant__ DrawDev d) {
     pdlWait();
@@ -628,6 +629,8 @@ __global__ void __launch_bounds__(kListThreads) listScanKernel(const __grid_cons
 #pragma unroll
     for (int k = 0; k < 4; k++)
         if (t0 + k < d.totalTiles) d.tileWork[(t0 + k) << d.tileWorkLog2] = 0;
+    const S32 longest = __reduce_max_sync(0xFFFFFFFFu, max(max(c[0], c[1]), max(c[2], c[3])));
+    if (lane == 0 && longest > kSortRun) atomicMax(&d.counters->longestList, longest);
     const U64 sum = entriesOf4(c);
     const U64 incl = warpInclusiveScan(sum);
     if (lane == 31) s_warp[warp] = incl;
@@ -741,13 +744,14 @@ __global__ void __launch_bounds__(kListThreads) listScatterKernel(const __grid_c
 // A warp sorts the lists of four neighbouring tiles at a time where they have
 // at most 8 entries each, of two with at most 16, and single ones of up to 256
 // in registers; longer
-// ones are sorted by their CTA: runs of 256 by its warps, then merged pair by
+// ones are sorted by a CTA each: runs of 256 by its warps, then merged pair by
 // pair in shared memory (an entry's place in a merged run is its own index
 // plus its rank in the other run: the entries of a list are distinct), up to
-// kSortShared entries; lists beyond that are merged in place in global memory
-// with a bitonic network from runs of kSortShared.
+// kSortShared entries; lists beyond that by a radix sort through a copy in
+// global memory (mostly L2; 17,000 entries in each tile of a 64x64 viewport:
+// 1.15 ms a draw, 17.8 when such lists were merged in place with a bitonic
+// network and two CTAs had all of them).
 
-constexpr int kSortRun = 256;
 constexpr int kSortShared = 4096;
 constexpr int kSparseLists = 16;   // mean list length below which a warp takes four tiles at a time
 constexpr int kSortCtas = 6;   // resident CTAs per SM
@@ -858,42 +862,92 @@ __device__ __forceinline__ void ctaSort(U32* list, S32 n, U32* a, U32* b) {
     __syncthreads();
 }
 
-// One step of an ascending bitonic merge of v[0, n): compares i with its
-// partner at distance j, or (flip) with its mirror image in blocks of 2 j.
-// Partners at or beyond n count as larger than everything.
-__device__ __forceinline__ void mergeStep(U32* v, S32 n, S32 j, bool flip) {
-    for (S32 p = threadIdx.x; p < n; p += kListThreads) {
-        const S32 i = (p / j) * 2 * j + p % j;                          // the lower partner of pair p
-        const S32 o = flip ? (i | (2 * j - 1)) - (i & (2 * j - 1)) : i + j;
-        if (i < n && o < n) {
-            const U32 x = v[i], y = v[o];
-            if (x > y) {
-                v[i] = y;
-                v[o] = x;
+// One stable pass of a radix sort over bits [shift, shift + 8) of src[0, n) into
+// dst, by the whole CTA: a warp counts and then moves its own piece of the list
+// (at 32 entries a step, ranked among equal digits by ballots). hist holds
+// kListWarps x 256 words.
+__device__ __forceinline__ void radixPass(const U32* src, U32* dst, S32 n, int shift, S32* hist, S32* sums) {
+    static_assert(kListThreads == 256, "a thread per digit");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const U32 ltMask = (1u << lane) - 1u;
+    const S32 piece = (n + kListThreads - 1) / kListThreads * 32;
+    const S32 begin = min(warp * piece, n), end = min(begin + piece, n);
+    S32* mine = hist + warp * 256;
+    for (int i = threadIdx.x; i < kListWarps * 256; i += kListThreads) hist[i] = 0;
+    __syncthreads();
+    for (S32 i = begin + lane; i < end; i += 128) {
+        U32 v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] = i + k * 32 < end ? src[i + k * 32] : 0u;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (i + k * 32 < end) atomicAdd(&mine[v[k] >> shift & 255u], 1);
+    }
+    __syncthreads();
+    // The pieces' places among the entries of digit threadIdx.x, then the digits'.
+    S32 total = 0;
+    for (int w = 0; w < kListWarps; w++) {
+        const S32 c = hist[w * 256 + threadIdx.x];
+        hist[w * 256 + threadIdx.x] = total;
+        total += c;
+    }
+    const S32 incl = warpInclusiveScan(total);
+    if (lane == 31) sums[warp] = incl;
+    __syncthreads();
+    S32 base = incl - total;
+    for (int w = 0; w < warp; w++) base += sums[w];
+    for (int w = 0; w < kListWarps; w++) hist[w * 256 + threadIdx.x] += base;
+    __syncthreads();
+    for (S32 i0 = begin; i0 < end; i0 += 128) {
+        U32 v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] = i0 + k * 32 + lane < end ? src[i0 + k * 32 + lane] : 0u;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const bool on = i0 + k * 32 + lane < end;
+            const U32 digit = v[k] >> shift & 255u;
+            U32 peers = __ballot_sync(0xFFFFFFFFu, on);
+#pragma unroll
+            for (int b = 0; b < 8; b++) {
+                const bool bit = digit >> b & 1u;
+                const U32 set = __ballot_sync(0xFFFFFFFFu, bit);
+                peers &= bit ? set : ~set;
             }
+            const S32 at = on ? mine[digit] + __popc(peers & ltMask) : 0;
+            __syncwarp();
+            if (on && (peers & ltMask) == 0u) mine[digit] += __popc(peers);
+            __syncwarp();
+            if (on) dst[at] = v[k];
         }
     }
     __syncthreads();
 }
 
-__device__ __forceinline__ void ctaSortLong(U32* list, S32 n, U32* a, U32* b) {
-    for (S32 r = 0; r < n; r += kSortShared) ctaSort(list + r, min(n - r, kSortShared), a, b);
-    for (S64 run = kSortShared; run < n; run *= 2) {
-        mergeStep(list, n, (S32)run, true);
-        for (S32 j = (S32)(run / 2); j > 0; j >>= 1) mergeStep(list, n, j, false);
+// Sorts list[0, n) through tmp[0, n); entries are below 2^bits.
+__device__ __forceinline__ void ctaSortLong(U32* list, U32* tmp, S32 n, int bits, S32* hist, S32* sums) {
+    U32* src = list;
+    U32* dst = tmp;
+    for (int shift = 0; shift < bits; shift += 8) {
+        radixPass(src, dst, n, shift, hist, sums);
+        U32* t = src;
+        src = dst;
+        dst = t;
+    }
+    if (src != list) {
+        for (S32 i = threadIdx.x; i < n; i += kListThreads) list[i] = src[i];
+        __syncthreads();
     }
 }
 
-__global__ void __launch_bounds__(kListThreads) listSortKernel(const __grid_constant__ DrawDev d, S32 tileBegin,
+__global__ void __launch_bounds__(kListThreads, kSortCtas) listSortKernel(const __grid_constant__ DrawDev d, S32 tileBegin,
                                                                S32 tileEnd) {
     pdlWait();
     __shared__ U32 s_a[kSortShared], s_b[kSortShared];
-    __shared__ S32 s_long[kListThreads];
+    __shared__ S32 s_long[kListThreads], s_found;
     if (__ldcg(&d.counters->overflow)) return;
     const int lane = threadIdx.x & 31;
     const S32 warps = gridDim.x * kListWarps;
     const S32 quads = (tileEnd - tileBegin + 3) / 4;
-    bool anyLong = false;
     // A warp takes quads of tiles, every gridDim.x-th one per CTA. Neighbouring quads go to different CTAs: a crowded
     // viewport's long lists would otherwise pile up on a few.
     if (__ldcg(&d.counters->tileEntries) < kSparseLists * d.totalTiles) {
@@ -917,7 +971,6 @@ __global__ void __launch_bounds__(kListThreads) listSortKernel(const __grid_cons
                 if (most > 1) sortShort<8>(d.tileList, cnt, first);
                 continue;
             }
-            anyLong = anyLong || most > kSortRun;
 #pragma unroll 1
             for (int half = 0; half < 2; half++) {
                 const S32 c0 = __shfl_sync(0xFFFFFFFFu, cnt, half * 16), c1 = __shfl_sync(0xFFFFFFFFu, cnt, half * 16 + 8);
@@ -945,23 +998,25 @@ __global__ void __launch_bounds__(kListThreads) listSortKernel(const __grid_cons
                 start = __ldg(&d.tileStart[tileBegin + k]);
             }
             if (cnt > 1 && cnt <= kSortRun) warpSortAny(list, list, cnt);
-            anyLong = anyLong || cnt > kSortRun;
         }
     }
-    // The long lists among the CTA's tiles, by the whole CTA.
-    if (!__syncthreads_or(anyLong)) return;
-    for (S32 q0 = blockIdx.x; q0 < quads; q0 += (kListThreads / 4) * gridDim.x) {
-        // The CTA's quads are every gridDim.x-th one, in both cases.
-        const S32 t = tileBegin + (q0 + (threadIdx.x >> 2) * gridDim.x) * 4 + (threadIdx.x & 3);
+    // The long lists, each by a whole CTA; a CTA looks after every gridDim.x-th
+    // tile. (The warps above leave these lists alone.)
+    if (__ldcg(&d.counters->longestList) <= kSortRun) return;
+    const int bits = 64 - __clzll(d.totalTris * 8 - 1);
+    for (S32 t0 = tileBegin + (S32)blockIdx.x; t0 < tileEnd; t0 += kListThreads * gridDim.x) {
+        const S64 t = (S64)t0 + (S64)threadIdx.x * gridDim.x;
         const bool isLong = t < tileEnd && __ldg(&d.tileCount[t]) > kSortRun;
-        s_long[threadIdx.x] = isLong ? t : -1;
+        if (threadIdx.x == 0) s_found = 0;
         if (!__syncthreads_or(isLong)) continue;
-        for (int k = 0; k < kListThreads; k++) {
+        if (isLong) s_long[atomicAdd(&s_found, 1)] = (S32)t;
+        __syncthreads();
+        const int found = s_found;
+        for (int k = 0; k < found; k++) {
             const S32 lt = s_long[k];
-            if (lt < 0) continue;
-            const S32 ln = __ldg(&d.tileCount[lt]);
-            U32* l = d.tileList + __ldg(&d.tileStart[lt]);
-            if (ln <= kSortShared) ctaSort(l, ln, s_a, s_b); else ctaSortLong(l, ln, s_a, s_b);
+            const S32 ln = __ldg(&d.tileCount[lt]), start = __ldg(&d.tileStart[lt]);
+            if (ln <= kSortShared) ctaSort(d.tileList + start, ln, s_a, s_b);
+            else ctaSortLong(d.tileList + start, d.sortScratch + start, ln, bits, (S32*)s_a, (S32*)s_b);
         }
         __syncthreads();
     }
@@ -996,11 +1051,16 @@ cudaError_t launchBinning(const DrawDev& d, int numSMs, cudaStream_t stream) {
     return e;
 }
 
-// Sorts the lists of tiles [tileBegin, tileEnd) into submission order.
+// Sorts the lists of tiles [tileBegin, tileEnd) into submission order. A CTA to
+// 32 tiles, or to every tile where the draw has at least eight triangles a
+// tile and long lists are likely, which take a CTA each (20,000 blended
+// triangles of 60 pixels at 200x150 574 us a draw with the former, 259 with the
+// latter; 5,000 small ones at 641x479 80 and 83).
 cudaError_t launchListSort(const DrawDev& d, int32_t tileBegin, int32_t tileEnd, int numSMs, cudaStream_t stream) {
     if (d.totalTris <= 0 || tileEnd <= tileBegin) return cudaSuccess;
-    const int64_t need = ((int64_t)tileEnd - tileBegin + 4 * kListWarps - 1) / (4 * kListWarps);
-    return launchKernel(listSortKernel, (unsigned)std::min<int64_t>(need, (int64_t)numSMs * kSortCtas), kListThreads, 0, stream,
+    const int64_t tiles = (int64_t)tileEnd - tileBegin;
+    const int64_t want = d.totalTris >= 8 * (int64_t)d.totalTiles ? tiles : (tiles + 4 * kListWarps - 1) / (4 * kListWarps);
+    return launchKernel(listSortKernel, (unsigned)std::min<int64_t>(want, (int64_t)numSMs * kSortCtas), kListThreads, 0, stream,
                         true, d, tileBegin, tileEnd);
 }
 

@@ -730,6 +730,7 @@ DrawDev makeDrawDev(cr_context* ctx, const Plan& plan) {
     d.tileCount = ctx->tileCount.as<int32_t>();
     d.tileStart = ctx->tileStart.as<int32_t>();
     d.tileList = ctx->tileList.as<uint32_t>();
+    d.sortScratch = ctx->itemPairs.as<U32>();   // twice as large
     d.maxTileEntries = ctx->maxTileEntries;
     char* pref = ctx->drawBlock.as<char>() + cb + sizeof(InstanceDev) * plan.inst.size();
     size_t n1 = plan.inst.size() + 1;

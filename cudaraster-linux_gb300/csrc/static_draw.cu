@@ -238,6 +238,7 @@ extern "C" cr_status cr_draw_triangles_static(const char* pipe_name, void* color
     d.tileCount = (int32_t*)(scratch + kOffTileCount);
     d.tileStart = (int32_t*)(scratch + kOffTileStart);
     d.tileList = (uint32_t*)(scratch + kOffTileList);
+    d.sortScratch = (uint32_t*)(scratch + kOffItemPairs);   // twice as large
     d.maxTileEntries = kStaticMaxTileEntries;
     d.triPrefix = (const int64_t*)(scratch + kOffPrefix);
     d.tilePrefix = (const int32_t*)(scratch + kOffPrefix + offsetof(Prefixes, tile));

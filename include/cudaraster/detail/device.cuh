@@ -85,6 +85,8 @@ struct Counters {
     S32 chunkWork;            // pair-stage chunk counter (dynamic chunk assignment)
     S32 itemWarps;            // warps of the item kernel: blocks of item pair records that are theirs from the start
     S32 itemBlocks;           // blocks taken beyond those
+    S32 longestList;          // longest tile list, where one passes 256 entries
+    S32 pad;
     U64 tileTotal;            // tile list entries allocated
     U64 stageBegin[4];        // when setup, pairs, scan and fine began, in ns (draws with stage timing)
 };
@@ -165,6 +167,7 @@ struct DrawDev {
     S32* tileCount;           // [totalTiles]
     S32* tileStart;           // [totalTiles]
     U32* tileList;            // [maxTileEntries]
+    U32* sortScratch;         // [maxTileEntries] copies of long lists being sorted: memory that is free after the scatter
     S64 maxTileEntries;
     // instance lookup tables (prefix sums, numInstances + 1 entries)
     const S32* tilePrefix;    // tiles
