@@ -680,7 +680,7 @@ __global__ void __launch_bounds__(kListThreads) listScanKernel(const __grid_cons
             U64 total = 0;
             for (int w = 0; w < kListWarps; w++) total += s_warp[w];
             d.counters->binEntries = reportedEntries(total);
-            if (!listsFit(total, d.maxBinEntries)) atomicOr(&d.counters->overflow, kOverflowBin);
+            if (d.maxBinEntries >= 0 && !listsFit(total, d.maxBinEntries)) atomicOr(&d.counters->overflow, kOverflowBin);
         }
     }
 }

@@ -719,7 +719,7 @@ DrawDev makeDrawDev(cr_context* ctx, const Plan& plan) {
     d.fineSelfPixels = ctx->tuning.fine_self_pixels;
     d.binWork = ctx->binWork.as<int32_t>();
     d.binCount = ctx->binCount.as<int32_t>();
-    d.maxBinEntries = ctx->maxBinEntries;
+    d.maxBinEntries = ctx->userCapacity ? ctx->maxBinEntries : -1;
     d.tileWork = ctx->tileWork.as<int32_t>();
     d.tileWorkLog2 = tileWorkLog2(plan.totalTiles);
     d.tileItems = ctx->tileItems.as<int32_t>();

@@ -57,7 +57,6 @@ constexpr int kStaticMaxBins = (kStaticMaxViewport / 128) * (kStaticMaxViewport 
 constexpr int kStaticChunkTris = kMinChunkTris;
 constexpr int kStaticMaxChunks = kStaticMaxTris / kStaticChunkTris;
 constexpr int64_t kStaticMaxSubtris = kStaticMaxTris + 16384;
-constexpr int64_t kStaticMaxBinEntries = 4 * kStaticMaxTris;
 constexpr int64_t kStaticMaxTileEntries = 16 * kStaticMaxTris;
 // The list stages of a static draw run on at most this many SMs' worth of
 // CTAs: each warp of the item kernel may leave a block of records partly
@@ -227,7 +226,7 @@ extern "C" cr_status cr_draw_triangles_static(const char* pipe_name, void* color
     d.modelVec4 = 0;
     d.binWork = (int32_t*)(scratch + kOffBinWork);     // zero at load; each list scan clears it again
     d.binCount = (int32_t*)(scratch + kOffBinCount);
-    d.maxBinEntries = kStaticMaxBinEntries;
+    d.maxBinEntries = -1;
     d.tileWork = (int32_t*)(scratch + kOffTileWork);   // likewise
     d.tileWorkLog2 = tileWorkLog2(numTiles);
     d.tileItems = (int32_t*)(scratch + kOffTileItems);
@@ -270,8 +269,8 @@ extern "C" cr_status cr_draw_triangles_static(const char* pipe_name, void* color
     if (c.overflow)
         return report(error, error_size, CR_ERR_CAPACITY,
                       "cr_draw_triangles_static: the draw needs more than the static queues hold "
-                      "(%lld subtriangle slots, %lld bin entries, %lld tile entries); surfaces left untouched",
-                      (long long)kStaticMaxSubtris, (long long)kStaticMaxBinEntries, (long long)kStaticMaxTileEntries);
+                      "(%lld subtriangle slots, %lld tile entries); surfaces left untouched",
+                      (long long)kStaticMaxSubtris, (long long)kStaticMaxTileEntries);
 #undef CR_STATIC_CUDA
     return CR_OK;
 }

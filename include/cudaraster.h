@@ -209,7 +209,9 @@ cr_status cr_set_stage_timing(cr_context* ctx, int32_t enabled);
 /* Queue capacities (elements) for the next draws. All zero keeps the
  * reference-style estimates (CudaRaster.cpp:263-275); otherwise the given
  * sizes are used as they are (a predictor's sizing) and, when a draw
- * overflows them, grown by the rerun loop. Capacities never shrink. */
+ * overflows them, grown by the rerun loop. Capacities never shrink. Bin entries
+ * take no memory (the draw only counts them): a draw overflows by them only
+ * against a max_bin_entries given here, not against the estimate. */
 cr_status cr_set_capacity(cr_context* ctx, int64_t max_subtris, int64_t max_bin_entries,
                           int64_t max_tile_entries);
 

@@ -158,7 +158,7 @@ struct DrawDev {
     // bin
     S32* binWork;             // [totalBins * kBinWorkStride] entries counted so far; zero between draws (the list scan clears it)
     S32* binCount;            // [totalBins]
-    S64 maxBinEntries;
+    S64 maxBinEntries;        // a limit that the caller set (there are no bin lists to overflow); -1: none
     // tile lists
     S32* tileWork;            // [totalTiles << tileWorkLog2] pair records so far; zero between draws (the list scan clears it)
     S32 tileWorkLog2;         // spacing of the counters in words (log2)
