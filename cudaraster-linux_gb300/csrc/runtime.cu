@@ -96,6 +96,35 @@ struct DevBuf {
     template <class T> T* as() const { return (T*)ptr; }
 };
 
+// A piece of a DevBuf. It keeps the most it ever held, so that a draw none of
+// whose arrays needs more than an earlier one's never reallocates the buffer
+// (which a captured graph may point to).
+struct DevPart {
+    void* ptr = nullptr;
+    size_t bytes = 0;
+    template <class T> T* as() const { return (T*)ptr; }
+};
+// The pieces of a buffer, each at a multiple of 256 bytes: take() each one, then
+// place() them in the allocation.
+class Pieces {
+public:
+    void take(DevPart& part, size_t need) {
+        parts_[count_] = &part;
+        offsets_[count_++] = bytes_;
+        part.bytes = std::max(part.bytes, (need + 255) & ~(size_t)255);
+        bytes_ += part.bytes;
+    }
+    size_t bytes() const { return bytes_; }
+    void place(const DevBuf& buf) {
+        for (int i = 0; i < count_; i++) parts_[i]->ptr = buf.as<char>() + offsets_[i];
+    }
+
+private:
+    DevPart* parts_[16];
+    size_t offsets_[16], bytes_ = 0;
+    int count_ = 0;
+};
+
 struct HostInstance {
     const PipeDesc* pipe;
     InstanceDev dev;
@@ -127,8 +156,13 @@ struct cr_context {
     int64_t maxSubtris = 0, maxBinEntries = 0, maxTileEntries = 0;
     bool userCapacity = false;  // capacities set by cr_set_capacity replace the estimates
     // Device memory.
-    DevBuf triSubtris, triHeader, triData, pairs, pairCount, mediumItems, largeItems, binWork, binCount;
-    DevBuf itemPairs, itemBlockCount, tileWork, tileItems, tileCursor, tileCount, tileStart, tileList;
+    DevBuf triHeader, triData, pairs, itemPairs, tileList;
+    // The smaller arrays share two allocations: one of what is zero between
+    // draws (whatever the draws' sizes, so its pieces may move from draw to
+    // draw), one of the rest.
+    DevBuf zeroWork, listWork;
+    DevPart binWork, tileWork, tileItems;
+    DevPart triSubtris, pairCount, mediumItems, largeItems, itemBlockCount, binCount, tileCursor, tileCount, tileStart;
     // Per-draw block, written by one copy per draw: the zeroed Counters and one
     // fine-stage tile counter per pipe group, then the instance descriptors
     // and the prefix arrays.
@@ -271,9 +305,8 @@ cr_status cr_create(cr_context** out) {
 cr_status cr_destroy(cr_context* ctx) {
     if (!ctx) return CR_ERR_INVALID_ARGUMENT;
     cudaDeviceSynchronize();
-    DevBuf* bufs[] = {&ctx->triSubtris, &ctx->triHeader, &ctx->triData,    &ctx->pairs, &ctx->pairCount, &ctx->mediumItems, &ctx->itemPairs, &ctx->itemBlockCount,
-                      &ctx->largeItems, &ctx->binWork,   &ctx->binCount,   &ctx->tileWork,  &ctx->tileItems, &ctx->tileCursor,
-                      &ctx->tileCount,  &ctx->tileStart, &ctx->tileList,   &ctx->drawBlock};
+    DevBuf* bufs[] = {&ctx->triHeader, &ctx->triData,  &ctx->pairs,    &ctx->itemPairs,
+                      &ctx->tileList,  &ctx->zeroWork, &ctx->listWork, &ctx->drawBlock};
     for (DevBuf* b : bufs) b->release();
     for (int i = 0; i < cr_context::kStageSlots; i++) {
         if (ctx->hostStage[i]) cudaFreeHost(ctx->hostStage[i]);
@@ -654,23 +687,29 @@ cr_status ensureCapacity(cr_context* ctx, const Plan& plan) {
         ctx->maxBinEntries = std::max<int64_t>(ctx->maxBinEntries, 2 * T + 65536);
         ctx->maxTileEntries = std::max<int64_t>(ctx->maxTileEntries, 4 * T + 65536);
     }
-    CR_CUDA(ctx->triSubtris.ensure((size_t)T + 4), "cudaMalloc");
     CR_CUDA(ctx->triHeader.ensure((size_t)ctx->maxSubtris * 16), "cudaMalloc");
     CR_CUDA(ctx->triData.ensure((size_t)ctx->maxSubtris * 64), "cudaMalloc");
     CR_CUDA(ctx->pairs.ensure((size_t)std::max(plan.numChunks, 1) * 2 * plan.chunkTris * 8), "cudaMalloc");
-    CR_CUDA(ctx->pairCount.ensure((size_t)std::max(plan.numChunks, 1) * 4), "cudaMalloc");
-    CR_CUDA(ctx->mediumItems.ensure((size_t)std::max<int64_t>(T, 1) * 4), "cudaMalloc");
-    CR_CUDA(ctx->largeItems.ensure((size_t)ctx->maxSubtris * 4), "cudaMalloc");
-    CR_CUDA(ctx->binWork.ensureZeroed((size_t)plan.totalBins * kBinWorkStride * 4), "cudaMalloc");
-    CR_CUDA(ctx->binCount.ensure((size_t)plan.totalBins * 4), "cudaMalloc");
-    CR_CUDA(ctx->tileWork.ensureZeroed(((size_t)plan.totalTiles << tileWorkLog2(plan.totalTiles)) * 4), "cudaMalloc");
-    CR_CUDA(ctx->tileItems.ensureZeroed((size_t)plan.totalTiles * 4), "cudaMalloc");
-    CR_CUDA(ctx->tileCursor.ensure((size_t)plan.totalTiles * 4), "cudaMalloc");
     const int64_t blocks = itemBlocks(ctx, ctx->maxTileEntries);
     CR_CUDA(ctx->itemPairs.ensure((size_t)blocks * kItemBlock * 8), "cudaMalloc");
-    CR_CUDA(ctx->itemBlockCount.ensure((size_t)blocks * 4), "cudaMalloc");
-    CR_CUDA(ctx->tileCount.ensure((size_t)plan.totalTiles * 4), "cudaMalloc");
-    CR_CUDA(ctx->tileStart.ensure((size_t)plan.totalTiles * 4), "cudaMalloc");
+    Pieces zero;
+    zero.take(ctx->binWork, (size_t)plan.totalBins * kBinWorkStride * 4);
+    zero.take(ctx->tileWork, ((size_t)plan.totalTiles << tileWorkLog2(plan.totalTiles)) * 4);
+    zero.take(ctx->tileItems, (size_t)plan.totalTiles * 4);
+    CR_CUDA(ctx->zeroWork.ensureZeroed(zero.bytes()), "cudaMalloc");
+    zero.place(ctx->zeroWork);
+    Pieces work;
+    work.take(ctx->binCount, (size_t)plan.totalBins * 4);
+    work.take(ctx->tileCount, (size_t)plan.totalTiles * 4);
+    work.take(ctx->tileStart, (size_t)plan.totalTiles * 4);
+    work.take(ctx->tileCursor, (size_t)plan.totalTiles * 4);
+    work.take(ctx->pairCount, (size_t)plan.numChunks * 4);
+    work.take(ctx->itemBlockCount, (size_t)blocks * 4);
+    work.take(ctx->triSubtris, (size_t)T + 4);
+    work.take(ctx->mediumItems, (size_t)T * 4);
+    work.take(ctx->largeItems, (size_t)ctx->maxSubtris * 4);
+    CR_CUDA(ctx->listWork.ensure(work.bytes()), "cudaMalloc");
+    work.place(ctx->listWork);
     CR_CUDA(ctx->tileList.ensure((size_t)ctx->maxTileEntries * 4), "cudaMalloc");
     const size_t stage = drawBlockBytes(plan);
     CR_CUDA(ctx->drawBlock.ensure(stage), "cudaMalloc");
