@@ -286,9 +286,10 @@ __device__ __forceinline__ U32 withZMargin(U32 z) { return z + min(kZMargin, ~z)
 // zLimit: the tile's maximum depth with the margin.
 __device__ __forceinline__ bool mayWin(uint4 h, U32 zLimit) {
     if ((h.w & 0xFFFFF000u) <= zLimit) return true;
-    const S32 w = max3i(lo16(h.x), lo16(h.y), lo16(h.z)) - min3i(lo16(h.x), lo16(h.y), lo16(h.z));
-    const S32 ht = max3i(hi16(h.x), hi16(h.y), hi16(h.z)) - min3i(hi16(h.x), hi16(h.y), hi16(h.z));
-    return max(w, ht) > 32767;
+    // The extents of x and y as unsigned halves (biased, the subtraction borrows
+    // nothing between them): over 32,767 subpixels?
+    const U32 most = __vmaxs2(__vmaxs2(h.x, h.y), h.z) ^ 0x80008000u, least = __vmins2(__vmins2(h.x, h.y), h.z) ^ 0x80008000u;
+    return ((most - least) & 0x80008000u) != 0u;
 }
 
 // Slot of a list entry's subtriangle, and the edges of a triangle that a record
