@@ -13,6 +13,9 @@
 //   scan:    allocates each tile's list from the counts.
 //   scatter: writes the recorded pairs at their places, those of the items
 //            behind the others.
+//   rest:    expands the items whose pairs found no room again (in queued and
+//            captured draws that may have such; a blocking one makes room and
+//            reruns).
 //   sort:    puts the lists of order-dependent pipes in submission order.
 //
 // The counters' atomics give a list's entries in no particular order. Pipes
@@ -45,12 +48,12 @@ namespace cr {
 constexpr int kListThreads = 256;
 constexpr int kListWarps = kListThreads / 32;
 
-// Warp-level inclusive scan.
-template <class T>
+// Warp-level inclusive scan (of the first N lanes).
+template <class T, int N = 32>
 __device__ __forceinline__ T warpInclusiveScan(T v) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
+    for (int o = 1; o < N; o <<= 1) {
         T t = __shfl_up_sync(0xFFFFFFFFu, v, o);
         if (lane >= o) v += t;
     }
@@ -438,12 +441,11 @@ struct ItemUnits {
     S32 total;
 };
 
-// Splits the items over the launched warps: huge items in up to 64 slices that
+// Splits the items over `warps` warps: huge items in up to 64 slices that
 // give about eight units a warp, large ones in up to 2 and medium ones in
 // groups of 4 to 32 that give about one.
-__device__ __forceinline__ ItemUnits planItems(const DrawDev& d) {
+__device__ __forceinline__ ItemUnits planItems(const DrawDev& d, S32 warps) {
     ItemUnits u;
-    const S32 warps = (S32)gridDim.x * kListWarps;
     const S32 large = __ldcg(&d.counters->largeItems[0]), huge = __ldcg(&d.counters->largeItems[1]);
     u.medium = __ldcg(&d.counters->mediumItems);
     u.hugeSlices = min(max(8 * warps / max(huge, 1), 1), 64);
@@ -456,9 +458,10 @@ __device__ __forceinline__ ItemUnits planItems(const DrawDev& d) {
 }
 
 // Stages up to 32 items in shared memory: lane l < items has list entry
-// `entry`, of whose box it takes slice `slice` of `slices`; counts their bins
-// (a sliced item's with its first slice). Returns the number of (item, cell)
-// pairs.
+// `entry`, of whose box it takes slice `slice` of `slices`; with kBins counts
+// their bins (a sliced item's with its first slice). Returns the number of
+// (item, cell) pairs.
+template <bool kBins>
 __device__ __forceinline__ S32 stageItems(const DrawDev& d, S32 items, U32 entry, S32 slice, S32 slices, ItemSmem& sm) {
     const int lane = threadIdx.x & 31;
     S32 n = 0, bins = 0;
@@ -475,7 +478,7 @@ __device__ __forceinline__ S32 stageItems(const DrawDev& d, S32 items, U32 entry
             n = (S32)((U32)n * (U32)(slice + 1) / (U32)slices - c0);
         }
         stageItem(sm, lane, h, g, b, bb.small(), c0, ii, in);   // (an item without cells is never looked up)
-        if (slice == 0) {
+        if (kBins && slice == 0) {
             bins = bb.count();
             if (bins <= 4) {
                 const bool test = !bb.small();
@@ -491,7 +494,7 @@ __device__ __forceinline__ S32 stageItems(const DrawDev& d, S32 items, U32 entry
     sm.incl[lane] = incl;
     __syncwarp();
     // Boxes of more than four bins: the whole warp, one item at a time.
-    for (U32 m = __ballot_sync(0xFFFFFFFFu, bins > 4); m; m &= m - 1) {
+    for (U32 m = kBins ? __ballot_sync(0xFFFFFFFFu, bins > 4) : 0u; m; m &= m - 1) {
         const int j = __ffs(m) - 1;
         const InstanceDev* in = &d.inst[sm.inst[j]];
         const S32 width = __ldg(&in->width), height = __ldg(&in->height);
@@ -509,14 +512,43 @@ __device__ __forceinline__ S32 stageItems(const DrawDev& d, S32 items, U32 entry
     return __shfl_sync(0xFFFFFFFFu, incl, 31);
 }
 
+// A unit's items: how many, the list entry of lane l < items, and which slice
+// of how many of their boxes.
+__device__ __forceinline__ S32 unitItems(const DrawDev& d, const ItemUnits& iu, S32 u, U32& entry, S32& slice, S32& slices) {
+    const int lane = threadIdx.x & 31;
+    S32 items = 1;
+    slice = 0;
+    slices = 1;
+    entry = 0;
+    if (u < iu.hugeUnits + iu.largeUnits) {
+        const bool huge = u < iu.hugeUnits;
+        const S32 k = huge ? u : u - iu.hugeUnits;
+        slices = huge ? iu.hugeSlices : iu.largeSlices;
+        const S32 h = k / slices;
+        slice = k - h * slices;
+        entry = __ldcg(&d.largeItems[huge ? d.maxSubtris - 1 - h : (S64)h]);
+    } else {
+        const S32 first = (u - iu.hugeUnits - iu.largeUnits) * iu.group;
+        items = min(iu.group, iu.medium - first);
+        if (lane < items) entry = __ldcg(&d.mediumItems[first + lane]);
+    }
+    return items;
+}
+
 // A warp's current block of item pair records: its own first, then from a
-// counter. A warp leaves at most one block partly filled, so a draw whose tile
-// entries fit has blocks for all; past the last one nothing is written (the
-// scan reports the overflow; the block numbers are compared unsigned, so a
-// counter past 2^31 writes nothing either).
+// counter. A warp leaves at most one block partly filled. Past the last block
+// nothing is written: restKernel takes the warp's pairs beyond its full blocks.
+// (Block numbers are compared unsigned, so a counter past 2^31 gives none
+// either.)
 struct ItemBlock {
-    S32 block, fill;
+    S32 block, fill, full;
 };
+__device__ __forceinline__ bool isBlock(const DrawDev& d, S32 block) { return (U32)block < (U32)d.maxItemBlocks; }
+
+// Whether every item pair has a record.
+__device__ __forceinline__ bool itemsRecorded(const DrawDev& d) {
+    return (U32)__ldcg(&d.counters->itemWarps) + (U32)__ldcg(&d.counters->itemBlocks) <= (U32)d.maxItemBlocks;
+}
 
 // Records the pairs of the lanes with `hit` and counts their tiles.
 __device__ __forceinline__ void recordItemPairs(const DrawDev& d, ItemBlock& blk, bool hit, U32 entry, S32 tile) {
@@ -532,9 +564,10 @@ __device__ __forceinline__ void recordItemPairs(const DrawDev& d, ItemBlock& blk
         S32 fresh = 0;
         if (lane == 0) {
             fresh = gridDim.x * kListWarps + atomicAdd(&d.counters->itemBlocks, 1);
-            if ((U32)block < (U32)d.maxItemBlocks) d.itemBlockCount[block] = kItemBlock;
+            if (isBlock(d, block)) d.itemBlockCount[block] = kItemBlock;
         }
         fresh = __shfl_sync(0xFFFFFFFFu, fresh, 0);
+        if (isBlock(d, block)) blk.full++;
         if (at >= kItemBlock) {
             block = fresh;
             at -= kItemBlock;
@@ -542,37 +575,26 @@ __device__ __forceinline__ void recordItemPairs(const DrawDev& d, ItemBlock& blk
         blk.fill -= kItemBlock;
         blk.block = fresh;
     }
-    if (hit && (U32)block < (U32)d.maxItemBlocks) d.itemPairs[(S64)block * kItemBlock + at] = (U64)entry << 32 | (U32)tile;
+    if (hit && isBlock(d, block)) d.itemPairs[(S64)block * kItemBlock + at] = (U64)entry << 32 | (U32)tile;
 }
 
 // Records the pairs of the items and counts their tiles and bins. Persistent
-// warps over the units.
+// warps over the units. The launch has at most d.maxItemBlocks warps.
 __global__ void __launch_bounds__(kListThreads, kItemWarpsPerSM / kListWarps) itemKernel(const __grid_constant__ DrawDev d) {
     pdlWait();
     __shared__ ItemSmem s_items[kListWarps];
     if (__ldcg(&d.counters->overflow) & kOverflowSubtris) return;
     ItemSmem& sm = s_items[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    const ItemUnits iu = planItems(d);
-    if (blockIdx.x == 0 && threadIdx.x == 0) d.counters->numUnits = iu.total;
     const S32 warps = gridDim.x * kListWarps;
-    ItemBlock blk{(S32)(blockIdx.x * kListWarps + (threadIdx.x >> 5)), 0};
+    const ItemUnits iu = planItems(d, warps);
+    if (blockIdx.x == 0 && threadIdx.x == 0) d.counters->numUnits = iu.total;
+    ItemBlock blk{(S32)(blockIdx.x * kListWarps + (threadIdx.x >> 5)), 0, 0};
     for (S32 u = blockIdx.x * kListWarps + (threadIdx.x >> 5); u < iu.total; u += warps) {
-        S32 items = 1, slice = 0, slices = 1;
-        U32 entry = 0;
-        if (u < iu.hugeUnits + iu.largeUnits) {
-            const bool huge = u < iu.hugeUnits;
-            const S32 k = huge ? u : u - iu.hugeUnits;
-            slices = huge ? iu.hugeSlices : iu.largeSlices;
-            const S32 h = k / slices;
-            slice = k - h * slices;
-            entry = __ldcg(&d.largeItems[huge ? d.maxSubtris - 1 - h : (S64)h]);
-        } else {
-            const S32 first = (u - iu.hugeUnits - iu.largeUnits) * iu.group;
-            items = min(iu.group, iu.medium - first);
-            if (lane < items) entry = __ldcg(&d.mediumItems[first + lane]);
-        }
-        const S32 P = stageItems(d, items, entry, slice, slices, sm);
+        S32 slice, slices;
+        U32 entry;
+        const S32 items = unitItems(d, iu, u, entry, slice, slices);
+        const S32 P = stageItems<true>(d, items, entry, slice, slices, sm);
         for (S32 base = 0; base < P; base += 32) {
             const S32 p = base + lane;
             int j = 0;
@@ -583,7 +605,10 @@ __global__ void __launch_bounds__(kListThreads, kItemWarpsPerSM / kListWarps) it
         }
         __syncwarp();
     }
-    if (lane == 0 && (U32)blk.block < (U32)d.maxItemBlocks) d.itemBlockCount[blk.block] = blk.fill;
+    if (lane == 0) {
+        if (isBlock(d, blk.block)) d.itemBlockCount[blk.block] = blk.fill;
+        if (d.restItems) d.itemFull[blockIdx.x * kListWarps + (threadIdx.x >> 5)] = isBlock(d, blk.block) ? -1 : blk.full;
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) d.counters->itemWarps = warps;
 }
 
@@ -604,6 +629,8 @@ __global__ void __launch_bounds__(kListThreads) listScanKernel(const __grid_cons
     __shared__ U64 s_base;
     const bool failed = (__ldcg(&d.counters->overflow) & kOverflowSubtris) != 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (blockIdx.x == 0 && threadIdx.x == 32 && !d.restItems && !itemsRecorded(d))
+        atomicOr(&d.counters->overflow, kOverflowItems);
     const S32 t0 = blockIdx.x * kScanTiles + threadIdx.x * 4;
     S32 c[4], own[4];   // entries, and those the pair stage recorded
 #pragma unroll
@@ -631,13 +658,16 @@ __global__ void __launch_bounds__(kListThreads) listScanKernel(const __grid_cons
         if (t0 + k < d.totalTiles) d.tileWork[(t0 + k) << d.tileWorkLog2] = 0;
     const S32 longest = __reduce_max_sync(0xFFFFFFFFu, max(max(c[0], c[1]), max(c[2], c[3])));
     if (lane == 0 && longest > kSortRun) atomicMax(&d.counters->longestList, longest);
+    // Places modulo 2^32 (whole where the lists fit), the warp's total in two
+    // parts of at most 32 x 2^16.
     const U64 sum = entriesOf4(c);
-    const U64 incl = warpInclusiveScan(sum);
-    if (lane == 31) s_warp[warp] = incl;
+    const U32 incl = warpInclusiveScan((U32)sum);
+    const U32 low = __reduce_add_sync(0xFFFFFFFFu, (U32)sum & 0xFFFFu), high = __reduce_add_sync(0xFFFFFFFFu, (U32)(sum >> 16));
+    if (lane == 0) s_warp[warp] = ((U64)high << 16) + low;
     __syncthreads();
     if (warp == 0) {
         const U64 v = lane < kListWarps ? s_warp[lane] : 0ull;
-        const U64 i = warpInclusiveScan(v);
+        const U64 i = warpInclusiveScan<U64, kListWarps>(v);
         if (lane < kListWarps) s_warp[lane] = i - v;
         if (lane == kListWarps - 1 && !failed) {
             const U64 base = atomicAdd((unsigned long long*)&d.counters->tileTotal, (unsigned long long)i);
@@ -647,7 +677,7 @@ __global__ void __launch_bounds__(kListThreads) listScanKernel(const __grid_cons
         }
     }
     __syncthreads();
-    S32 s = (S32)(s_base + s_warp[warp] + incl - sum);
+    S32 s = (S32)((U32)s_base + (U32)s_warp[warp] + incl - (U32)sum);
     if (!failed) {
         if (t0 + 3 < d.totalTiles) {
             const int4 v = make_int4(s, s + c[0], s + c[0] + c[1], s + c[0] + c[1] + c[2]);
@@ -718,7 +748,7 @@ __global__ void __launch_bounds__(kListThreads) listScatterKernel(const __grid_c
                     putEntry(d, start[k] + (S32)(rec[k] >> 37), (t0 + ((U32)rec[k] & 1023u)) << 3 | 7u);
         }
     }
-    const S32 blocks = min(__ldcg(&d.counters->itemWarps) + __ldcg(&d.counters->itemBlocks), d.maxItemBlocks);
+    const S32 blocks = (S32)min((U32)__ldcg(&d.counters->itemWarps) + (U32)__ldcg(&d.counters->itemBlocks), (U32)d.maxItemBlocks);
     // The items' pairs, four per lane in flight too (one per lane: the stage 23.5 us
     // instead of 22.1 on 20,000 triangles of 60 pixels, 49 / 46 on the water layer).
     constexpr int kParts = kItemBlock / 128;
@@ -736,6 +766,41 @@ __global__ void __launch_bounds__(kListThreads) listScatterKernel(const __grid_c
 #pragma unroll
         for (int k = 0; k < 4; k++)
             if (at + k * 32 < count) putEntry(d, place[k], (U32)(rec[k] >> 32));
+    }
+}
+
+// The item pairs without a record, straight into the lists: the item kernel's
+// warps that ran out of blocks expand their units again and pass over the pairs
+// of their full blocks.
+__global__ void __launch_bounds__(kListThreads, kItemWarpsPerSM / kListWarps) restKernel(const __grid_constant__ DrawDev d) {
+    pdlWait();
+    __shared__ ItemSmem s_items[kListWarps];
+    if (__ldcg(&d.counters->overflow) || itemsRecorded(d)) return;
+    const S32 itemWarps = __ldcg(&d.counters->itemWarps);
+    ItemSmem& sm = s_items[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const ItemUnits iu = planItems(d, itemWarps);
+    for (S32 w = blockIdx.x * kListWarps + (threadIdx.x >> 5); w < itemWarps; w += gridDim.x * kListWarps) {
+        const S32 full = __ldcg(&d.itemFull[w]);
+        if (full < 0) continue;
+        S64 recorded = (S64)full * kItemBlock;   // still to pass over
+        for (S32 u = w; u < iu.total; u += itemWarps) {
+            S32 slice, slices;
+            U32 entry;
+            const S32 items = unitItems(d, iu, u, entry, slice, slices);
+            const S32 P = stageItems<false>(d, items, entry, slice, slices, sm);
+            for (S32 base = 0; base < P; base += 32) {
+                const S32 p = base + lane;
+                int j = 0;
+                S32 tile = 0;
+                const bool hit = p < P && pairTile(d, sm, items, p, j, tile);
+                const U32 e = __shfl_sync(0xFFFFFFFFu, entry, j);
+                const U32 mask = __ballot_sync(0xFFFFFFFFu, hit);
+                if (hit && __popc(mask & ((1u << lane) - 1u)) >= recorded) putEntry(d, atomicAdd(&d.tileCursor[tile], 1), e);
+                recorded = max(recorded - __popc(mask), (S64)0);
+            }
+            __syncwarp();
+        }
     }
 }
 
@@ -1037,17 +1102,20 @@ cudaError_t launchBinning(const DrawDev& d, int numSMs, cudaStream_t stream) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, listScatterKernel, kListThreads, 0);
         return n > 0 ? n : 1;
     });
+    const int itemGrid = numSMs * (kItemWarpsPerSM / kListWarps);
     cudaError_t e = cudaSuccess;
     if (d.totalTris > 0) {
         const int pairGrid = std::min(numSMs * pairCtas, (d.numChunks + kListWarps - 1) / kListWarps);
         e = launchKernel(pairKernel, pairGrid, kListThreads, 0, stream, true, d);
-        if (e == cudaSuccess) e = launchKernel(itemKernel, numSMs * (kItemWarpsPerSM / kListWarps), kListThreads, 0, stream, true, d);
+        if (e == cudaSuccess) e = launchKernel(itemKernel, itemGrid, kListThreads, 0, stream, true, d);
     }
     // The scan also runs for a draw without triangles: it zeroes the counts.
     if (e == cudaSuccess)
         e = launchKernel(listScanKernel, (d.totalTiles + kScanTiles - 1) / kScanTiles, kListThreads, 0, stream, true, d);
     if (e == cudaSuccess && d.totalTris > 0)
         e = launchKernel(listScatterKernel, numSMs * scatterCtas, kListThreads, 0, stream, true, d);
+    if (e == cudaSuccess && d.totalTris > 0 && d.restItems)
+        e = launchKernel(restKernel, numSMs, kListThreads, 0, stream, true, d);
     return e;
 }
 

@@ -20,6 +20,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -155,6 +156,10 @@ struct cr_context {
     // Capacities (elements), grown by the rerun loop and kept across draws.
     int64_t maxSubtris = 0, maxBinEntries = 0, maxTileEntries = 0;
     bool userCapacity = false;  // capacities set by cr_set_capacity replace the estimates
+    int64_t lastItemBlocks = 0; // blocks of item pair records that the last draw had
+    int64_t itemRecords = 0;    // item pair records that draws so far have had use for, where over kItemRecords
+    // Shared with the context's captured graphs: its use count tells whether any is alive.
+    std::shared_ptr<char> graphs = std::make_shared<char>();
     // Device memory.
     DevBuf triHeader, triData, pairs, itemPairs, tileList;
     // The smaller arrays share two allocations: one of what is zero between
@@ -162,7 +167,7 @@ struct cr_context {
     // draw), one of the rest.
     DevBuf zeroWork, listWork;
     DevPart binWork, tileWork, tileItems;
-    DevPart triSubtris, pairCount, mediumItems, largeItems, itemBlockCount, binCount, tileCursor, tileCount, tileStart;
+    DevPart triSubtris, pairCount, mediumItems, largeItems, itemBlockCount, itemFull, binCount, tileCursor, tileCount, tileStart;
     // Per-draw block, written by one copy per draw: the zeroed Counters and one
     // fine-stage tile counter per pipe group, then the instance descriptors
     // and the prefix arrays.
@@ -666,10 +671,20 @@ size_t drawBlockBytes(const Plan& plan) {
            kPrefixBytesPerInstance * (plan.inst.size() + 1) + 64;
 }
 
-// Blocks of item pair records: every tile entry may come from an item, and each
-// warp of the item kernel may leave one block partly filled.
-int64_t itemBlocks(const cr_context* ctx, int64_t maxTileEntries) {
-    return (maxTileEntries + kItemBlock - 1) / kItemBlock + (int64_t)ctx->numSMs * kItemWarpsPerSM;
+// Blocks of item pair records. Every tile entry may come from an item, but
+// mostly few do; each warp of the item kernel may leave one block partly filled.
+int64_t itemBlocks(const cr_context* ctx) {
+    const int64_t records = std::min(ctx->maxTileEntries, std::max<int64_t>(kItemRecords, ctx->itemRecords));
+    return (records + kItemBlock - 1) / kItemBlock + (int64_t)ctx->numSMs * kItemWarpsPerSM;
+}
+
+// Room for the records that the last draw lacked, unless a captured graph may
+// point to the present ones.
+void growItemRecords(cr_context* ctx) {
+    if (!ctx->drawn || ctx->graphs.use_count() > 1) return;
+    const volatile Counters* c = ctx->hostCounters;
+    const int64_t blocks = (int64_t)(uint32_t)c->itemWarps + (uint32_t)c->itemBlocks;
+    if (blocks > ctx->lastItemBlocks) ctx->itemRecords = std::max(ctx->itemRecords, blocks * kItemBlock);
 }
 
 cr_status ensureCapacity(cr_context* ctx, const Plan& plan) {
@@ -689,9 +704,14 @@ cr_status ensureCapacity(cr_context* ctx, const Plan& plan) {
     }
     CR_CUDA(ctx->triHeader.ensure((size_t)ctx->maxSubtris * 16), "cudaMalloc");
     CR_CUDA(ctx->triData.ensure((size_t)ctx->maxSubtris * 64), "cudaMalloc");
-    CR_CUDA(ctx->pairs.ensure((size_t)std::max(plan.numChunks, 1) * 2 * plan.chunkTris * 8), "cudaMalloc");
-    const int64_t blocks = itemBlocks(ctx, ctx->maxTileEntries);
+    growItemRecords(ctx);
+    const int64_t blocks = itemBlocks(ctx);
     CR_CUDA(ctx->itemPairs.ensure((size_t)blocks * kItemBlock * 8), "cudaMalloc");
+    // The larger of the two record buffers also serves as the sort's copy of
+    // the lists.
+    size_t pairBytes = (size_t)std::max(plan.numChunks, 1) * 2 * plan.chunkTris * 8;
+    if (ctx->itemPairs.bytes < (size_t)ctx->maxTileEntries * 4) pairBytes = std::max(pairBytes, (size_t)ctx->maxTileEntries * 4);
+    CR_CUDA(ctx->pairs.ensure(pairBytes), "cudaMalloc");
     Pieces zero;
     zero.take(ctx->binWork, (size_t)plan.totalBins * kBinWorkStride * 4);
     zero.take(ctx->tileWork, ((size_t)plan.totalTiles << tileWorkLog2(plan.totalTiles)) * 4);
@@ -705,6 +725,7 @@ cr_status ensureCapacity(cr_context* ctx, const Plan& plan) {
     work.take(ctx->tileCursor, (size_t)plan.totalTiles * 4);
     work.take(ctx->pairCount, (size_t)plan.numChunks * 4);
     work.take(ctx->itemBlockCount, (size_t)blocks * 4);
+    work.take(ctx->itemFull, (size_t)ctx->numSMs * kItemWarpsPerSM * 4);
     work.take(ctx->triSubtris, (size_t)T + 4);
     work.take(ctx->mediumItems, (size_t)T * 4);
     work.take(ctx->largeItems, (size_t)ctx->maxSubtris * 4);
@@ -765,11 +786,12 @@ DrawDev makeDrawDev(cr_context* ctx, const Plan& plan) {
     d.tileCursor = ctx->tileCursor.as<int32_t>();
     d.itemPairs = ctx->itemPairs.as<U64>();
     d.itemBlockCount = ctx->itemBlockCount.as<int32_t>();
-    d.maxItemBlocks = (int32_t)itemBlocks(ctx, ctx->maxTileEntries);
+    d.itemFull = ctx->itemFull.as<int32_t>();
+    d.maxItemBlocks = (int32_t)itemBlocks(ctx);
     d.tileCount = ctx->tileCount.as<int32_t>();
     d.tileStart = ctx->tileStart.as<int32_t>();
     d.tileList = ctx->tileList.as<uint32_t>();
-    d.sortScratch = ctx->itemPairs.as<U32>();   // twice as large
+    d.sortScratch = ctx->pairs.bytes > ctx->itemPairs.bytes ? ctx->pairs.as<U32>() : ctx->itemPairs.as<U32>();
     d.maxTileEntries = ctx->maxTileEntries;
     char* pref = ctx->drawBlock.as<char>() + cb + sizeof(InstanceDev) * plan.inst.size();
     size_t n1 = plan.inst.size() + 1;
@@ -825,6 +847,12 @@ bool capturing(cudaStream_t s) {
 cr_status launchDrawWith(cr_context* ctx, const Plan& plan, cudaStream_t stream, void* stage, Counters* hostCounters,
                          bool events, bool writeKernel) {
     DrawDev d = makeDrawDev(ctx, plan);
+    // Records for every tile entry never run out. With fewer, a blocking draw
+    // that lacks some is rerun with more (a launch less: 1.7 us), one that
+    // cannot be rerun, or must leave a captured graph's memory, finds the rest
+    // again.
+    const bool enough = ((int64_t)d.maxItemBlocks - (int64_t)ctx->numSMs * kItemWarpsPerSM) * kItemBlock >= ctx->maxTileEntries;
+    d.restItems = !enough && (!writeKernel || ctx->graphs.use_count() > 1);
     d.stageTiming = events ? 1 : 0;
     // Stage the zeroed counters and the descriptors through pinned memory;
     // for a blocking draw a kernel parameter carries them to the device, else
@@ -890,6 +918,7 @@ cr_status launchDraw(cr_context* ctx, const Plan& plan, cudaStream_t stream, boo
     cr_status st = launchDrawWith(ctx, plan, stream, ctx->hostStage[slot], ctx->hostCounters, ctx->stageTiming, sync);
     if (st != CR_OK) return st;
     ctx->drawn = true;
+    ctx->lastItemBlocks = itemBlocks(ctx);
     CR_CUDA(cudaEventRecord(ctx->stageDone[slot], stream), "cudaEventRecord");
     ctx->stageUsed[slot] = true;
     return CR_OK;
@@ -1048,6 +1077,7 @@ struct cr_batch_graph {
     cudaGraphExec_t exec = nullptr;
     void* stage = nullptr;
     Counters* counters = nullptr;
+    std::shared_ptr<char> alive;
 };
 
 extern "C" {
@@ -1064,6 +1094,7 @@ cr_status cr_batch_graph_create(cr_context* ctx, const cr_instance* instances, i
     if (v.empty()) return fail(ctx, CR_ERR_INVALID_ARGUMENT, "CudaRaster: empty batch");
     cr_batch_graph* g = new cr_batch_graph();
     g->ctx = ctx;
+    g->alive = ctx->graphs;
     st = buildPlan(ctx, v, g->plan);
     if (st == CR_OK) st = ensureCapacity(ctx, g->plan);
     if (st != CR_OK) { delete g; return st; }

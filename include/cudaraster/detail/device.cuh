@@ -42,6 +42,7 @@ enum : int {
     kOverflowSubtris = 1,
     kOverflowBin = 2,
     kOverflowTile = 4,
+    kOverflowItems = 8,   // item pairs lack records
 };
 
 // ---------------------------------------------------------------- layouts
@@ -93,6 +94,12 @@ struct Counters {
 // Item pair records come in blocks of this many, each filled by one warp.
 constexpr int kItemBlock = 256;
 constexpr int kItemWarpsPerSM = 40;   // resident warps of the item kernel (its grid)
+// A context keeps room for this many records (64 MB), or for as many as its tile
+// list has entries where that is less; more once a draw has had more (a record
+// for every possible tile entry took 1.07 of the 2.3 GB of list memory of a
+// 33.5M-triangle draw, which has 0.2M). Pairs without one are found again by
+// restKernel.
+constexpr S64 kItemRecords = 1 << 23;
 
 // Subtriangles by the size of their tile box, as the pair stage sorts them.
 // Those in at most 2x2 tiles become (tile, triangle) pair records at once. The
@@ -153,7 +160,9 @@ struct DrawDev {
     U32* mediumItems;         // [totalTris] list entries
     U64* itemPairs;           // [maxItemBlocks * kItemBlock] list entry << 32 | global tile
     S32* itemBlockCount;      // [maxItemBlocks]
+    S32* itemFull;            // [warps of the item kernel] blocks it filled before it got no more; -1: it did not run out
     S32 maxItemBlocks;
+    S32 restItems;            // pairs without a record go to restKernel (else, where there are any, the draw overflows)
     U32* largeItems;          // [maxSubtris] list entries: boxes of at most kHugeCells tiles from the front, larger from the back
     // bin
     S32* binWork;             // [totalBins * kBinWorkStride] entries counted so far; zero between draws (the list scan clears it)
