@@ -194,6 +194,7 @@ struct cr_context {
     cr_queue_layout lastLayout{};
     int lastWidth = 0, lastHeight = 0;   // viewport and samples of the last single draw
     int lastSamplesLog2 = 0;
+    bool lastOrdered = false;            // its tile lists were sorted
     int64_t lastTris = 0;
 };
 
@@ -488,11 +489,14 @@ cr_status cr_read_queue_output(cr_context* ctx, int32_t* bin_start, int32_t* bin
             CR_CUDA(cudaMemcpy(tile_list, ctx->tileList.ptr, (size_t)c.tile_entries * 4, cudaMemcpyDeviceToHost),
                     "cudaMemcpy");
             // Pipes that do not depend on the lists' order draw from unordered
-            // ones: the export gives them in submission order.
-            std::vector<int32_t> ts(nt), tc(nt);
-            CR_CUDA(cudaMemcpy(ts.data(), ctx->tileStart.ptr, nt * 4, cudaMemcpyDeviceToHost), "cudaMemcpy");
-            CR_CUDA(cudaMemcpy(tc.data(), ctx->tileCount.ptr, nt * 4, cudaMemcpyDeviceToHost), "cudaMemcpy");
-            for (size_t t = 0; t < nt; t++) std::sort(tile_list + ts[t], tile_list + ts[t] + tc[t]);
+            // ones, which are put in submission order here; the others' come
+            // as the draw sorted them.
+            if (!ctx->lastOrdered) {
+                std::vector<int32_t> ts(nt), tc(nt);
+                CR_CUDA(cudaMemcpy(ts.data(), ctx->tileStart.ptr, nt * 4, cudaMemcpyDeviceToHost), "cudaMemcpy");
+                CR_CUDA(cudaMemcpy(tc.data(), ctx->tileCount.ptr, nt * 4, cudaMemcpyDeviceToHost), "cudaMemcpy");
+                for (size_t t = 0; t < nt; t++) std::sort(tile_list + ts[t], tile_list + ts[t] + tc[t]);
+            }
         }
     } catch (const std::bad_alloc&) {
         return fail(ctx, CR_ERR_OUT_OF_MEMORY, "CudaRaster: out of host memory reading the queues back");
@@ -950,6 +954,7 @@ cr_status drawPlan(cr_context* ctx, const Plan& plan, cudaStream_t stream, bool 
     ctx->lastWidth = first.width;
     ctx->lastHeight = first.height;
     ctx->lastSamplesLog2 = first.samplesLog2;
+    ctx->lastOrdered = plan.inst[0].pipe->needsOrder != 0;
     ctx->lastTris = plan.totalTris;
     ctx->last.num_bins = plan.totalBins;
     ctx->last.num_tiles = plan.totalTiles;
