@@ -247,7 +247,7 @@ cr_status cr_batch_graph_destroy(cr_batch_graph* graph);
  * that owns a fixed memory budget, a real-time loop where cudaMalloc would
  * stall the frame, a plugin that only receives device pointers): no context,
  * no cudaMalloc/cudaFree, no pinned host buffers. The intermediate queues
- * live in one static array of about 22 MiB compiled into this library, held
+ * live in one static array of about 26 MiB compiled into this library, held
  * by every GPU that loads it until the process exits, and shared by every
  * call: calls that overlap on the GPU race, so order them on one stream.
  * Limits: num_tris <= 65536, width and height <= 1024, fixed queue sizes;
