@@ -1260,16 +1260,22 @@ cr_status cr_get_profiling_info(cr_context* ctx, char* buffer, int64_t size) {
     cr_counters c{};
     cr_get_counters(ctx, &c);
     // Format follows getProfilingInfo's default mode (CudaRaster.cpp:367-421):
-    // stage times, then the memory footprint of the intermediate queues.
-    double mb = 1.0 / (1024.0 * 1024.0);
+    // stage times, then the memory footprint: the triangle slots and the
+    // tile list entries in use, and what the context has allocated for the
+    // lists (with the records they are built from) and in all.
+    const double mb = 1.0 / (1024.0 * 1024.0);
+    const size_t lists = ctx->pairs.bytes + ctx->itemPairs.bytes + ctx->tileList.bytes + ctx->zeroWork.bytes + ctx->listWork.bytes;
+    const size_t all = lists + ctx->triHeader.bytes + ctx->triData.bytes + ctx->drawBlock.bytes;
     snprintf(buffer, (size_t)size,
              "Setup  %8.3f ms\nBin    %8.3f ms\nCoarse %8.3f ms\nFine   %8.3f ms\nTotal  %8.3f ms\n"
-             "Triangles     %lld\nSubtriangles  %lld (%.1f MB)\nBin entries   %lld (%.1f MB)\n"
-             "Tile entries  %lld (%.1f MB)\nCoarse units  %lld\nReruns        %d\n",
+             "Triangles     %lld\nSubtriangles  %lld (%.1f MB)\nBin entries   %lld\n"
+             "Tile entries  %lld (%.1f MB)\nCoarse units  %lld\nReruns        %d\n"
+             "List memory   %.1f MB\nScratch       %.1f MB\n",
              s.setup_time * 1e3, s.bin_time * 1e3, s.coarse_time * 1e3, s.fine_time * 1e3,
              (s.setup_time + s.bin_time + s.coarse_time + s.fine_time) * 1e3, (long long)c.num_tris,
-             (long long)c.num_subtris, c.num_subtris * 81.0 * mb, (long long)c.bin_entries, c.bin_entries * 4.0 * mb,
-             (long long)c.tile_entries, c.tile_entries * 4.0 * mb, (long long)c.coarse_units, c.reruns);
+             (long long)c.num_subtris, c.num_subtris * 81.0 * mb, (long long)c.bin_entries,
+             (long long)c.tile_entries, c.tile_entries * 4.0 * mb, (long long)c.coarse_units, c.reruns, lists * mb,
+             all * mb);
     return CR_OK;
 }
 

@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import importlib
 import json
+import re
 from pathlib import Path
 
 import numpy as np
@@ -260,8 +261,13 @@ def run_flythrough_plain(ft: FlyThrough, frames: range, tuning: dict | None = No
             sums.append(ft.checksum(f))
         if f in keep:
             kept[f] = ft.snapshot(f)
-    counters = [cr.getCounters() for cr in crs]
+    counters = [{**cr.getCounters(), "list_mb": list_memory_mb(cr)} for cr in crs]
     return wall, sums, kept, counters
+
+
+def list_memory_mb(cr) -> float:
+    """What a context has allocated for its tile lists and the records they are built from."""
+    return float(re.search(r"List memory\s+([0-9.]+) MB", cr.getProfilingInfo()).group(1))
 
 
 def run_flythrough_predicted(ft: FlyThrough, frames: int, train_frames: int = 50, tuning: dict | None = None,
@@ -407,7 +413,7 @@ def run_flythrough_predicted(ft: FlyThrough, frames: int, train_frames: int = 50
         pr.close()
     return {"wall_train": wall_train, "wall_pred": wall_pred, "wait": wait, "misses": misses, "records": rec,
             "checksums": [sums[f] for f in sorted(sums)], "kept": kept, "train_frames": train_frames,
-            "adam_steps": steps}
+            "adam_steps": steps, "list_mb": [list_memory_mb(cr) for cr in crs]}
 
 
 FLYTHROUGH_WORKLOAD = ("fly-through: 4096^2 heightfield (33.5M triangles, 6-octave value noise) + translucent water "
@@ -425,7 +431,7 @@ def measure_flythrough(n: int = 4096, width: int = 3840, height: int = 2160, fra
     run_flythrough_plain(ft, range(3), tuning)                                   # warm-up
     _, sums, kept, ctr = run_flythrough_plain(ft, range(frames), tuning, checksums=True, keep=keep)
     exact = run_flythrough_predicted(ft, frames, train_frames, tuning, checksums=True)
-    wall_plain, _, _, _ = run_flythrough_plain(ft, range(train_frames, frames), tuning)
+    wall_plain, _, _, plain_ctr = run_flythrough_plain(ft, range(train_frames, frames), tuning)
     res = run_flythrough_predicted(ft, frames, train_frames, tuning)
     n_pred = frames - train_frames
     plain_fps = n_pred / wall_plain
@@ -435,12 +441,14 @@ def measure_flythrough(n: int = 4096, width: int = 3840, height: int = 2160, fra
         r = sorted((x for x in res["records"] if x["layer"] == k), key=lambda x: x["frame"])
         T = layer["num_tris"]
         entry = {"layer": layer["name"], "triangles": T, "misses": res["misses"][k],
-                 "queue_mb_plain_estimate": round((2 * T + 65536 + 4 * T + 65536) * 4 / 2**20, 1),
-                 "queue_mb_predicted_mean": round(float(np.mean([x["cap_bin"] + x["cap_tile"] for x in r])) * 4 / 2**20,
-                                                  1),
-                 "queue_mb_predicted_max": round(float(np.max([x["cap_bin"] + x["cap_tile"] for x in r])) * 4 / 2**20,
-                                                 1),
-                 "queue_mb_used_max": round(float(np.max([x["bin"] + x["tile"] for x in r])) * 4 / 2**20, 1)}
+                 # Allocated for the lists by either path's contexts (the pair records and item
+                 # queues, 25 bytes a triangle, follow the triangle count in both), and of
+                 # that the tile list itself: as estimated, as predicted and as used.
+                 "list_memory_mb_plain": plain_ctr[k]["list_mb"], "list_memory_mb_predicted": res["list_mb"][k],
+                 "tile_list_mb_plain_estimate": round((4 * T + 65536) * 4 / 2**20, 1),
+                 "tile_list_mb_predicted_mean": round(float(np.mean([x["cap_tile"] for x in r])) * 4 / 2**20, 1),
+                 "tile_list_mb_predicted_max": round(float(np.max([x["cap_tile"] for x in r])) * 4 / 2**20, 1),
+                 "tile_list_mb_used_max": round(float(np.max([x["tile"] for x in r])) * 4 / 2**20, 1)}
         errs = {}
         for q in ("bin", "tile"):
             a = np.array([x[q] for x in r])
