@@ -443,7 +443,12 @@ struct ItemUnits {
 
 // Splits the items over `warps` warps: huge items in up to 64 slices that
 // give about eight units a warp, large ones in up to 2 and medium ones in
-// groups of 4 to 32 that give about one.
+// groups of 4 to 32 that give about one. In us of the bin stage, over 20,000
+// triangles of 60 pixels, 300k blended ones, 5,000 blended of 90 pixels, 5,000
+// of 6 and the 32-scene batch: 58.8, 29.2, 33.7, 17.8, 126; up to 16 slices:
+// 49.6, 28.5, 37.1, 17.8, 125; large ones whole: 57.9, 32.3, 35.6, 17.8, 124, in
+// up to 8: 58.5, 32.9, 36.9, 17.8, 126; groups from 1: 60.7, 29.1, 33.3, 16.8,
+// 126, from 16: 58.3, 27.5, 36.4, 20.1, 126, up to 8: 59.3, 29.0, 33.5, 17.8, 135.
 __device__ __forceinline__ ItemUnits planItems(const DrawDev& d, S32 warps) {
     ItemUnits u;
     const S32 large = __ldcg(&d.counters->largeItems[0]), huge = __ldcg(&d.counters->largeItems[1]);
@@ -727,15 +732,12 @@ __global__ void __launch_bounds__(kListThreads) listScatterKernel(const __grid_c
     if (__ldcg(&d.counters->overflow)) return;
     const int lane = threadIdx.x & 31;
     const S32 warps = gridDim.x * kListWarps, warpIdx = blockIdx.x * kListWarps + (threadIdx.x >> 5);
-    // A chunk's pairs by one warp, or by several where there are few chunks.
-    const S32 split = max(1, min(8, 2 * warps / max(d.numChunks, 1)));
-    for (S32 u = warpIdx; u < d.numChunks * split; u += warps) {
-        const S32 chunk = u / split, part = u - chunk * split;
+    for (S32 chunk = warpIdx; chunk < d.numChunks; chunk += warps) {
         const S32 count = __ldcg(&d.pairCount[chunk]);
         const U64* pairs = d.pairs + (S64)chunk * 2 * d.chunkTris;
         const U32 t0 = (U32)chunk * (U32)d.chunkTris;
         // Four pairs per lane in flight.
-        for (S32 p0 = part * 128 + lane; p0 < count; p0 += split * 128) {
+        for (S32 p0 = lane; p0 < count; p0 += 128) {
             U64 rec[4];
             S32 start[4];
 #pragma unroll
@@ -818,7 +820,10 @@ __global__ void __launch_bounds__(kListThreads, kItemWarpsPerSM / kListWarps) re
 // network and two CTAs had all of them).
 
 constexpr int kSortShared = 4096;
-constexpr int kSparseLists = 16;   // mean list length below which a warp takes four tiles at a time
+// Mean list length below which a warp takes four tiles at a time (coarse stage
+// of the textured terrain and of the 32-scene batch: 66 and 78 us; with 64: 79
+// and 78, with 4: 67 and 87).
+constexpr int kSparseLists = 16;
 constexpr int kSortCtas = 6;   // resident CTAs per SM
 
 // Sorts each W consecutive lanes' values (bitonic).
