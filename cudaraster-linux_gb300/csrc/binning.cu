@@ -60,6 +60,13 @@ __device__ __forceinline__ T warpInclusiveScan(T v) {
     return v;
 }
 
+// A warp's 64-bit total, in 16-bit digits (the warp-wide addition takes 32 bits).
+__device__ __forceinline__ U64 warpTotal(U64 v) {
+    const U32 lo = __reduce_add_sync(0xFFFFFFFFu, (U32)v & 0xFFFFu), mid = __reduce_add_sync(0xFFFFFFFFu, (U32)(v >> 16) & 0xFFFFu);
+    const U32 hi = __reduce_add_sync(0xFFFFFFFFu, (U32)(v >> 32));
+    return ((U64)hi << 32) + ((U64)mid << 16) + lo;
+}
+
 // Queues list entry `entry` as a large or huge item.
 __device__ __forceinline__ void queueLarge(const DrawDev& d, U32 entry, bool huge) {
     const S32 k = atomicAdd(&d.counters->largeItems[huge ? 1 : 0], 1);
@@ -550,9 +557,9 @@ struct ItemBlock {
 };
 __device__ __forceinline__ bool isBlock(const DrawDev& d, S32 block) { return (U32)block < (U32)d.maxItemBlocks; }
 
-// Whether every item pair has a record.
-__device__ __forceinline__ bool itemsRecorded(const DrawDev& d) {
-    return (U32)__ldcg(&d.counters->itemWarps) + (U32)__ldcg(&d.counters->itemBlocks) <= (U32)d.maxItemBlocks;
+// Whether every item pair has a record, by the draw's counters.
+__device__ __forceinline__ bool itemsRecorded(const DrawDev& d, S32 itemWarps, S32 itemBlocks) {
+    return (U32)itemWarps + (U32)itemBlocks <= (U32)d.maxItemBlocks;
 }
 
 // Records the pairs of the lanes with `hit` and counts their tiles.
@@ -634,8 +641,8 @@ __global__ void __launch_bounds__(kListThreads) listScanKernel(const __grid_cons
     __shared__ U64 s_base;
     const bool failed = (__ldcg(&d.counters->overflow) & kOverflowSubtris) != 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (blockIdx.x == 0 && threadIdx.x == 32 && !d.restItems && !itemsRecorded(d))
-        atomicOr(&d.counters->overflow, kOverflowItems);
+    // (Loaded now, looked at when the bins are handed over.)
+    const S32 itemWarps = __ldcg(&d.counters->itemWarps), itemBlocks = __ldcg(&d.counters->itemBlocks);
     const S32 t0 = blockIdx.x * kScanTiles + threadIdx.x * 4;
     S32 c[4], own[4];   // entries, and those the pair stage recorded
 #pragma unroll
@@ -663,12 +670,11 @@ __global__ void __launch_bounds__(kListThreads) listScanKernel(const __grid_cons
         if (t0 + k < d.totalTiles) d.tileWork[(t0 + k) << d.tileWorkLog2] = 0;
     const S32 longest = __reduce_max_sync(0xFFFFFFFFu, max(max(c[0], c[1]), max(c[2], c[3])));
     if (lane == 0 && longest > kSortRun) atomicMax(&d.counters->longestList, longest);
-    // Places modulo 2^32 (whole where the lists fit), the warp's total in two
-    // parts of at most 32 x 2^16.
+    // Places modulo 2^32 (whole where the lists fit) beside 64-bit totals.
     const U64 sum = entriesOf4(c);
     const U32 incl = warpInclusiveScan((U32)sum);
-    const U32 low = __reduce_add_sync(0xFFFFFFFFu, (U32)sum & 0xFFFFu), high = __reduce_add_sync(0xFFFFFFFFu, (U32)(sum >> 16));
-    if (lane == 0) s_warp[warp] = ((U64)high << 16) + low;
+    const U64 warpSum = warpTotal(sum);
+    if (lane == 0) s_warp[warp] = warpSum;
     __syncthreads();
     if (warp == 0) {
         const U64 v = lane < kListWarps ? s_warp[lane] : 0ull;
@@ -707,10 +713,12 @@ __global__ void __launch_bounds__(kListThreads) listScanKernel(const __grid_cons
             d.binCount[b] = v;
             mine += (U32)v;
         }
-        mine = warpInclusiveScan(mine);
+        mine = warpTotal(mine);
         __syncthreads();
-        if (lane == 31) s_warp[warp] = mine;
+        if (lane == 0) s_warp[warp] = mine;
         __syncthreads();
+        if (threadIdx.x == 0 && !d.restItems && !itemsRecorded(d, itemWarps, itemBlocks))
+            atomicOr(&d.counters->overflow, kOverflowItems);
         if (threadIdx.x == 0 && !failed) {
             U64 total = 0;
             for (int w = 0; w < kListWarps; w++) total += s_warp[w];
@@ -777,8 +785,8 @@ __global__ void __launch_bounds__(kListThreads) listScatterKernel(const __grid_c
 __global__ void __launch_bounds__(kListThreads, kItemWarpsPerSM / kListWarps) restKernel(const __grid_constant__ DrawDev d) {
     pdlWait();
     __shared__ ItemSmem s_items[kListWarps];
-    if (__ldcg(&d.counters->overflow) || itemsRecorded(d)) return;
     const S32 itemWarps = __ldcg(&d.counters->itemWarps);
+    if (__ldcg(&d.counters->overflow) || itemsRecorded(d, itemWarps, __ldcg(&d.counters->itemBlocks))) return;
     ItemSmem& sm = s_items[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const ItemUnits iu = planItems(d, itemWarps);
