@@ -685,7 +685,7 @@ int64_t itemBlocks(const cr_context* ctx) {
 // Room for the records that the last draw lacked, unless a captured graph may
 // point to the present ones.
 void growItemRecords(cr_context* ctx) {
-    if (!ctx->drawn || ctx->graphs.use_count() > 1) return;
+    if (!ctx->drawn || itemBlocks(ctx) * kItemBlock >= ctx->maxTileEntries || ctx->graphs.use_count() > 1) return;
     const volatile Counters* c = ctx->hostCounters;
     const int64_t blocks = (int64_t)(uint32_t)c->itemWarps + (uint32_t)c->itemBlocks;
     if (blocks > ctx->lastItemBlocks) ctx->itemRecords = std::max(ctx->itemRecords, blocks * kItemBlock);
