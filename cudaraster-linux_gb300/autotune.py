@@ -136,7 +136,7 @@ def main():
     ap.add_argument("--out", default=str(HERE / "tuning.json"))
     ap.add_argument("--quick", action="store_true")
     ap.add_argument("--grid", choices=["full", "medium"], default="full",
-                    help="medium: bins x warps x three unit sizes, for the large workloads")
+                    help="medium: bins x warps x two chunk sizes, for the large workloads")
     args = ap.parse_args()
     scenes = importlib.import_module(PKG + ".scenes")
     wl = importlib.import_module(PKG + ".workloads")
