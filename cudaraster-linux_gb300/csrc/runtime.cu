@@ -106,10 +106,12 @@ struct DevPart {
     template <class T> T* as() const { return (T*)ptr; }
 };
 // The pieces of a buffer, each at a multiple of 256 bytes: take() each one, then
-// place() them in the allocation.
+// place() them in the allocation (until then they point nowhere, also where it
+// fails).
 class Pieces {
 public:
     void take(DevPart& part, size_t need) {
+        part.ptr = nullptr;
         parts_[count_] = &part;
         offsets_[count_++] = bytes_;
         part.bytes = std::max(part.bytes, (need + 255) & ~(size_t)255);
