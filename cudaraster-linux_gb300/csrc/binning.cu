@@ -22,9 +22,9 @@
 // whose fine stage resolves visibility by keys (fine.cuh) do not depend on it;
 // for the others the lists are sorted. A count -> scan -> scatter pass per
 // level, bins then tiles, with every list in order (the design before) took
-// for its six kernels, against these, in us: 101 / 74 on 1M small triangles at
-// 1080p, 309 / 190 on an 8.4M-triangle 4x MSAA heightfield at 4K, 276 / 86 on
-// 20,000 triangles of 60 pixels, 85 / 63 with the sort (11) on 300k blended
+// for its six kernels, against these, in us: 101 / 67 on 1M small triangles at
+// 1080p, 309 / 180 on an 8.4M-triangle 4x MSAA heightfield at 4K, 276 / 81 on
+// 20,000 triangles of 60 pixels, 85 / 56 with the sort (11) on 300k blended
 // ones.
 //
 // None of these kernels lets its dependent launch early (launch.h): CTAs that

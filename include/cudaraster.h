@@ -85,7 +85,7 @@ typedef struct cr_counters {
     int64_t coarse_units;         /* coarse work units: groups or slices of the       */
                                   /* subtriangles that cover more than 2x2 tiles      */
     int64_t max_subtris;
-    int64_t max_bin_entries;
+    int64_t max_bin_entries;      /* as set; else an estimate that limits nothing     */
     int64_t max_tile_entries;
     int32_t reruns;               /* overflow-detect-and-rerun iterations of the draw */
     int32_t overflow;             /* nonzero if the last launch overflowed            */
