@@ -97,8 +97,9 @@ constexpr int kItemWarpsPerSM = 40;   // resident warps of the item kernel (its 
 // A context keeps room for this many records (64 MB), or for as many as its tile
 // list has entries where that is less; more once a draw has had more (a record
 // for every possible tile entry took 1.07 of the 2.3 GB of list memory of a
-// 33.5M-triangle draw, which has 0.2M). Pairs without one are found again by
-// restKernel.
+// 33.5M-triangle draw whose items make 1,516 units of work). A blocking draw
+// that lacks some makes room and reruns; in others restKernel finds the pairs
+// without one again.
 constexpr S64 kItemRecords = 1 << 23;
 
 // Subtriangles by the size of their tile box, as the pair stage sorts them.
